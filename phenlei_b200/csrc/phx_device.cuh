@@ -77,17 +77,180 @@ __device__ __forceinline__ T sutherland(T t, T s) { return t * sqrt(t) * (T(1) +
 
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+__device__ __forceinline__ uint32_t smem_u32(const void *p)
+{
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+__device__ __forceinline__ void mbar_init(uint64_t *mbar, uint32_t count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mbar)), "r"(count) : "memory");
+}
+
+// Bounded wait for the mbarrier phase with the given parity; false on timeout.
+__device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity)
+{
+    const uint32_t a = smem_u32(mbar);
+    for (long long i = 0; i < (1LL << 26); ++i) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(done)
+            : "r"(a), "r"(parity)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+__device__ __forceinline__ void mbar_expect(uint64_t *mbar, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes) : "memory");
+}
+
+// Bulk copy of global memory into shared memory (addresses and size multiples of
+// 16 bytes) of data read once: it leaves L2 first.
+__device__ __forceinline__ uint64_t evict_first_policy()
+{
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *mbar, uint64_t policy)
+{
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
+            smem_u32(dst)),
+        "l"(src), "r"(bytes), "r"(smem_u32(mbar)), "l"(policy)
+        : "memory");
+}
+
 // IEEE division on both paths, for the LU-SGS sweeps: the files holding the
 // face and SA passes are compiled with approximate FP32 division.
 __device__ __forceinline__ float idiv(float a, float b) { return __fdiv_rn(a, b); }
 __device__ __forceinline__ double idiv(double a, double b) { return a / b; }
 
-// Sweep geometry of the LU-SGS dataflow sweeps: a slot of kSweepLanes lanes
-// per schedule position, kSweepSlots slots per warp.  Every wait is bounded by
-// NsConst::spinLimit polls (phx_set_wait_limit).
-static constexpr int kSweepThreads = 256;
+// A row of the LU-SGS schedule is one warp: kSweepLanes lanes a cell.
 static_assert(kSweepLanes * kSweepSlots == 32, "one warp holds kSweepSlots slots");
-static_assert(kSweepMaxEntries == 2 * kSweepLanes, "a cell spans at most two adjacent slots");
+
+// The rows of one warp on their way through its shared memory: two rows of
+// kRow bytes a stage, `stages` stages, each filled by one bulk copy (a warp's
+// rows are contiguous) that lane 0 issues.  Gathered lane by lane instead, the
+// copies' address arithmetic took more instructions than the row's own work,
+// and one warp issues them one after the other.
+template <int kRow>
+struct RowPipe {
+    static constexpr int kStage = 2 * kRow;
+    unsigned char *buf;
+    uint64_t *full;
+    const unsigned char *src;         // the warp's next stage to be issued
+    int nrow, nstage, stages;         // rows, stages of rows, stages in flight
+    int slot, ahead;                  // slot of the current stage; stages issued
+    uint32_t parity;
+    uint64_t policy;
+
+    __device__ __forceinline__ unsigned char *at(int sl) const { return buf + sl * kStage; }
+    __device__ __forceinline__ void issue(int sl, int lane)
+    {
+        if (lane == 0) {
+            const uint32_t n = (uint32_t)min(2, nrow - 2 * ahead) * kRow;
+            mbar_expect(full + sl, n);
+            bulk_load(at(sl), src, n, full + sl, policy);
+        }
+        src += kStage;
+        ++ahead;
+    }
+    __device__ __forceinline__ void start(unsigned char *mem, uint64_t *bars, const unsigned char *rows, int row0, int n,
+                                          int st, int lane)
+    {
+        buf = mem;
+        full = bars;
+        src = rows + (size_t)row0 * kRow;
+        nrow = n;
+        nstage = (n + 1) / 2;
+        stages = st;
+        slot = ahead = 0;
+        parity = 0;
+        policy = evict_first_policy();
+        if (lane == 0) {
+            for (int i = 0; i < st; ++i) mbar_init(full + i, 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        for (int i = 0; i < st && i < nstage; ++i) issue(i, lane);
+        __syncwarp();
+    }
+    __device__ __forceinline__ bool wait() const { return mbar_wait(full + slot, parity); }
+    // after all lanes have read the current stage
+    __device__ __forceinline__ void advance(int lane)
+    {
+        if (ahead < nstage) issue(slot, lane);
+        if (++slot == stages) { slot = 0; parity ^= 1u; }
+    }
+    // before leaving early at stage k: the copies in flight
+    __device__ __forceinline__ void drain(int k) const
+    {
+        int sl = slot;
+        uint32_t p = parity;
+        for (; k < ahead; ++k) {
+            mbar_wait(full + sl, p);
+            if (++sl == stages) { sl = 0; p ^= 1u; }
+        }
+    }
+};
+
+// Factors of one face use in the sweeps: 16 values per lane of a row, in
+// 16-byte units rotated by the lane so that a warp reads them from shared
+// memory without bank conflicts.
+template <class T>
+__device__ __forceinline__ int use_unit(int k, int lane)
+{
+    return sizeof(T) == 4 ? (k + (lane >> 1)) & 3 : (k + lane) & 7;
+}
+__device__ __forceinline__ void put_use(float *use, int lane, const float *v)
+{
+    float4 *d = reinterpret_cast<float4 *>(use);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) d[use_unit<float>(k, lane)] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+}
+__device__ __forceinline__ void put_use(double *use, int lane, const double *v)
+{
+    double2 *d = reinterpret_cast<double2 *>(use);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) d[use_unit<double>(k, lane)] = make_double2(v[2 * k], v[2 * k + 1]);
+}
+__device__ __forceinline__ void get_use(const float *row, int lane, float *v)
+{
+    const float4 *d = reinterpret_cast<const float4 *>(row + lane * kUse);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float4 a = d[use_unit<float>(k, lane)];
+        v[4 * k] = a.x; v[4 * k + 1] = a.y; v[4 * k + 2] = a.z; v[4 * k + 3] = a.w;
+    }
+}
+__device__ __forceinline__ void get_use(const double *row, int lane, double *v)
+{
+    const double2 *d = reinterpret_cast<const double2 *>(row + lane * kUse);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const double2 a = d[use_unit<double>(k, lane)];
+        v[2 * k] = a.x; v[2 * k + 1] = a.y;
+    }
+}
+// 4 or 8 values of shared memory
+__device__ __forceinline__ void get4(const float *p, float *o)
+{
+    const float4 a = *reinterpret_cast<const float4 *>(p);
+    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
+}
+__device__ __forceinline__ void get4(const double *p, double *o)
+{
+    const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
+    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
+}
+template <class T>
+__device__ __forceinline__ void get8(const T *p, T *o) { get4(p, o); get4(p + 4, o + 4); }
 
 // Write-once sweep records.  Before a sweep every element of its output
 // records holds the sentinel, a NaN whose sign and payload no arithmetic
@@ -113,7 +276,8 @@ __device__ __forceinline__ bool is_sentinel(double v)
     return (unsigned long long)__double_as_longlong(v) == kSentinelD;
 }
 // a computed value as stored: the sentinel pattern becomes the canonical NaN
-__device__ __forceinline__ float unsentinel(float v) { return is_sentinel(v) ? __int_as_float(0x7fffffff) : v; }
+// (single-precision arithmetic gives no other NaN)
+__device__ __forceinline__ float unsentinel(float v) { return v; }
 __device__ __forceinline__ double unsentinel(double v)
 {
     return is_sentinel(v) ? __longlong_as_double(0x7fffffffffffffffLL) : v;
@@ -140,46 +304,53 @@ __device__ __forceinline__ void st_relaxed(double *p, double v)
     asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
 
-// Polls the first five elements of an 8-element record; true once none of
-// them is the sentinel (o then holds the final values).
-__device__ __forceinline__ bool poll5(const float *p, float *o)
+// Polls the first five elements of an 8-element record: the loads alone (the
+// values are looked at later), whether none of them is the sentinel (they are
+// then final), and both together.
+__device__ __forceinline__ void poll5_load(const float *p, float *o)
 {
-    asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3])
+    asm volatile(
+        "{\n\t.reg .f32 x, y, z;\n\t"
+        "ld.relaxed.gpu.global.v8.f32 {%0, %1, %2, %3, %4, x, y, z}, [%5];\n\t}\n"
+        : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4])
+        : "l"(p)
+        : "memory");
+}
+__device__ __forceinline__ void poll5_load(const double *p, double *o)
+{
+    asm volatile("ld.relaxed.gpu.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3])
                  : "l"(p)
                  : "memory");
     o[4] = ld_poll(p + 4);
+}
+template <class T>
+__device__ __forceinline__ bool poll5_done(const T *o)
+{
     return !(is_sentinel(o[0]) | is_sentinel(o[1]) | is_sentinel(o[2]) | is_sentinel(o[3]) | is_sentinel(o[4]));
 }
-__device__ __forceinline__ bool poll5(const double *p, double *o)
+template <class T>
+__device__ __forceinline__ bool poll5(const T *p, T *o)
 {
-    asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(o[0]), "=d"(o[1]) : "l"(p) : "memory");
-    asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(o[2]), "=d"(o[3]) : "l"(p + 2) : "memory");
-    o[4] = ld_poll(p + 4);
-    return !(is_sentinel(o[0]) | is_sentinel(o[1]) | is_sentinel(o[2]) | is_sentinel(o[3]) | is_sentinel(o[4]));
+    poll5_load(p, o);
+    return poll5_done(o);
 }
 
-// Publishes the five values of an 8-element record (slots 5-7 zero).
+// Publishes the five values of an 8-element record (the rest zero): whole
+// sectors, so that L2 need not fetch the sentinel's from DRAM to complete them.
 __device__ __forceinline__ void publish5(float *p, const float *v)
 {
-    asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(unsentinel(v[0])),
-                 "f"(unsentinel(v[1])), "f"(unsentinel(v[2])), "f"(unsentinel(v[3]))
-                 : "memory");
-    asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p + 4), "f"(unsentinel(v[4])),
-                 "f"(0.0f), "f"(0.0f), "f"(0.0f)
+    asm volatile("st.relaxed.gpu.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %6, %6};" ::"l"(p), "f"(unsentinel(v[0])),
+                 "f"(unsentinel(v[1])), "f"(unsentinel(v[2])), "f"(unsentinel(v[3])), "f"(unsentinel(v[4])), "f"(0.0f)
                  : "memory");
 }
 __device__ __forceinline__ void publish5(double *p, const double *v)
 {
-    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(unsentinel(v[0])),
-                 "d"(unsentinel(v[1]))
+    asm volatile("st.relaxed.gpu.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(unsentinel(v[0])),
+                 "d"(unsentinel(v[1])), "d"(unsentinel(v[2])), "d"(unsentinel(v[3]))
                  : "memory");
-    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p + 2), "d"(unsentinel(v[2])),
-                 "d"(unsentinel(v[3]))
+    asm volatile("st.relaxed.gpu.global.v4.f64 [%0], {%1, %2, %2, %2};" ::"l"(p + 4), "d"(unsentinel(v[4])), "d"(0.0)
                  : "memory");
-    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p + 4), "d"(unsentinel(v[4])), "d"(0.0)
-                 : "memory");
-    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p + 6), "d"(0.0), "d"(0.0) : "memory");
 }
 
 }  // namespace phx

@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kThreads) halo_pack_kernel(DevGrid g, int fiel
         o[15] = w.qrec[(size_t)c * kQ + 7];
     } else if (field == PHX_HALO_DQ) {
         T *o = reinterpret_cast<T *>(buf) + (size_t)i * kD;
-        const T *d = w.dqfwd + (size_t)c * kD;
+        const T *d = w.dqfwd + (size_t)g.lead[c] * kD;
 #pragma unroll
         for (int k = 0; k < kD; ++k) o[k] = d[k];
     } else if (field == PHX_HALO_TURB) {
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kThreads) halo_unpack_kernel(DevGrid g, NsCons
         w.qrec[(size_t)c * kQ + 7] = v[15];
     } else if (field == PHX_HALO_DQ) {
         const T *v = reinterpret_cast<const T *>(buf) + (size_t)i * kD;
-        T *d = w.dqfwd + (size_t)c * kD;
+        T *d = w.dqghost + (size_t)(c - g.nCell) * kD;
 #pragma unroll
         for (int k = 0; k < kD; ++k) d[k] = v[k];
     } else if (field == PHX_HALO_TURB) {

@@ -1,5 +1,5 @@
 // Host side of the phx library: context creation (grid metrics in FP64, the
-// cell-to-face lists, the LU-SGS level schedules, boundary classification),
+// cell-to-face lists, the LU-SGS schedules, boundary classification),
 // device memory, and the C ABI declared in include/phx.h.
 #include <cuda_runtime.h>
 
@@ -14,6 +14,7 @@
 
 #include "phx_internal.h"
 #include "phx_mlp.h"
+#include "phx_schedule.h"
 
 namespace phx {
 int mlp_loss_grad(const float *params, const float *x, const float *y, int B, float *grad, double &lossOut,
@@ -78,6 +79,7 @@ struct phx_ctx {
     int step = 0;
     bool haveResidual = false;
     std::vector<int> rankOf;              // storage index of each reference cell
+    std::vector<int> sweepRows[2];        // schedule rows of the LU-SGS sweeps, until the row arrays hold them
     // partitioned grids (interface faces): the topology and storage maps that
     // phx_swap_geometry needs to form the weights again, and the halo plan
     bool hasInterface = false;
@@ -685,6 +687,20 @@ int make_visc(phx_ctx *ctx, Work<T> &w)
     return PHX_OK;
 }
 
+// The rows of one LU-SGS sweep, `bytes` each: zeros (lanes without an entry and
+// the boundary part of cells without boundary faces stay so) and, at the end of
+// each, the schedule row.
+int make_rows(phx_ctx *ctx, unsigned char **rows, int which, size_t bytes)
+{
+    const std::vector<int> &src = ctx->sweepRows[which];
+    const size_t n = src.size() / kSweepRow, part = kSweepRow * sizeof(int);
+    const int r = dalloc(ctx, rows, n * bytes);
+    if (r) return r;
+    PHX_CUDA(ctx, cudaMemset(*rows, 0, n * bytes));
+    PHX_CUDA(ctx, cudaMemcpy2D(*rows + bytes - part, bytes, src.data(), part, part, n, cudaMemcpyHostToDevice));
+    return PHX_OK;
+}
+
 // Spalart-Allmaras arrays: nu~ of the free stream everywhere (TurbSolverUnstr::
 // InitFlowAsRestart, TurbSolverUnstr.cpp:910-930), eddy viscosity 0 and laminar
 // viscosity 1 until the first NS step forms it (NSSolverUnstruct.cpp:685-695).
@@ -698,10 +714,10 @@ int make_turb(phx_ctx *ctx, Work<T> &w, TurbWork<T> &t)
     r |= dalloc(ctx, &t.tgrad, nc * kTg);
     r |= dalloc(ctx, &t.tcrec, nc * kTc);
     r |= dalloc(ctx, &t.tface, nf * kTf);
-    r |= dalloc(ctx, &t.tcoef, 2 * nf);
-    r |= dalloc(ctx, &t.tdq, nc);
-    r |= dalloc(ctx, &t.tdqf, nc);
-    r |= dalloc(ctx, &t.tdfl, nc);
+    r |= make_rows(ctx, &t.trowf, 0, kRowSa<T>);
+    r |= make_rows(ctx, &t.trowb, 1, kRowSa<T>);
+    r |= dalloc(ctx, &t.tdq, (size_t)ctx->g.bwd.nRows * kSweepSlots);
+    r |= dalloc(ctx, &t.tdqf, (size_t)ctx->g.fwd.nRows * kSweepSlots);
     r |= dalloc(ctx, &t.tsrc, nc);
     if (ctx->prm.gradientName == 2) r |= dalloc(ctx, &t.qtnode, (size_t)ctx->nNode);
     r |= dalloc(ctx, &ctx->nmlp, 1);
@@ -721,7 +737,6 @@ int make_turb(phx_ctx *ctx, Work<T> &w, TurbWork<T> &t)
     }
     PHX_CUDA(ctx, cudaMemcpy(t.qt64, q.data(), sizeof(double) * nt, cudaMemcpyHostToDevice));
     PHX_CUDA(ctx, cudaMemcpy(w.trec, rec.data(), sizeof(T) * nt * kTr, cudaMemcpyHostToDevice));
-    PHX_CUDA(ctx, cudaMemset(t.tcoef, 0, sizeof(T) * 2 * nf));
     return PHX_OK;
 }
 
@@ -733,23 +748,26 @@ int make_work(phx_ctx *ctx, Work<T> &w, const std::vector<double> &limInit)
     r |= dalloc(ctx, &w.qrec, nt * kQ);
     r |= dalloc(ctx, &w.grec, nt * kG);
     r |= dalloc(ctx, &w.flux, nf * kFlux);
-    r |= dalloc(ctx, &w.coef, 2 * nf * kCoef);
+    r |= dalloc(ctx, &w.coef, (size_t)ctx->nBFace * kCoef);
+    r |= make_rows(ctx, &w.rowf, 0, kRowNs<T, true>);
+    r |= make_rows(ctx, &w.rowb, 1, kRowNs<T, false>);
     r |= dalloc(ctx, &w.crec, nc * kC);
     r |= dalloc(ctx, &w.dtraw, nc);
-    r |= dalloc(ctx, &w.dqrec, nt * kD);
-    r |= dalloc(ctx, &w.dqfwd, nt * kD);
-    r |= dalloc(ctx, &w.dflux, nc * kD);
+    const size_t nf8 = (size_t)ctx->g.fwd.nRows * kSweepSlots * kD, nb8 = (size_t)ctx->g.bwd.nRows * kSweepSlots * kD;
+    r |= dalloc(ctx, &w.dqrec, nb8);
+    r |= dalloc(ctx, &w.dqfwd, nf8);
+    r |= dalloc(ctx, &w.dqghost, (size_t)ctx->nBFace * kD);
     if (ctx->prm.gradientName == 2) r |= dalloc(ctx, &w.nrec, (size_t)ctx->nNode * kN);
     if (r) return r;
     if (w.nrec) PHX_CUDA(ctx, cudaMemset(w.nrec, 0, sizeof(T) * (size_t)ctx->nNode * kN));
     std::vector<T> q(nt * kQ, T(0));
     for (size_t i = 0; i < nt; ++i) q[i * kQ + 7] = (T)limInit[i];
     PHX_CUDA(ctx, cudaMemcpy(w.qrec, q.data(), sizeof(T) * q.size(), cudaMemcpyHostToDevice));
-    PHX_CUDA(ctx, cudaMemset(w.dqrec, 0, sizeof(T) * nt * kD));
-    PHX_CUDA(ctx, cudaMemset(w.dqfwd, 0, sizeof(T) * nt * kD));   // interface ghost rows until the first exchange
+    PHX_CUDA(ctx, cudaMemset(w.dqrec, 0, sizeof(T) * nb8));
+    PHX_CUDA(ctx, cudaMemset(w.dqfwd, 0, sizeof(T) * nf8));
+    PHX_CUDA(ctx, cudaMemset(w.dqghost, 0, sizeof(T) * (size_t)ctx->nBFace * kD));   // until the first exchange
     PHX_CUDA(ctx, cudaMemset(w.grec, 0, sizeof(T) * nt * kG));
     PHX_CUDA(ctx, cudaMemset(w.crec, 0, sizeof(T) * nc * kC));
-    PHX_CUDA(ctx, cudaMemset(w.coef, 0, sizeof(T) * 2 * nf * kCoef));
     return PHX_OK;
 }
 
@@ -891,7 +909,7 @@ int phx_ctx_create(const phx_grid_desc *gd, const phx_params *prm, phx_ctx **out
         for (int f = 0; f < nf; ++f) { c2f[fill[h.left[f]]++] = f; if (f >= nb) c2f[fill[h.right[f]]++] = f; }
     }
     for (int c = 0; c < nc; ++c)
-        if (c2f_off[c + 1] - c2f_off[c] > kSweepMaxEntries) { delete ctx; return PHX_ERR_ARG; }  // two sweep slots
+        if (c2f_off[c + 1] - c2f_off[c] > kMaxCellFaces) { delete ctx; return PHX_ERR_ARG; }
 
     // storage order
     // storage order: Morton (Z-curve) order of the cell centres, or, with
@@ -913,119 +931,84 @@ int phx_ctx_create(const phx_grid_desc *gd, const phx_params *prm, phx_ctx **out
     });
     std::vector<int> fpos(nf);
     for (int i = 0; i < nf; ++i) fpos[forder[i]] = i;
-    // storage index of any reference cell or ghost (ghost of reference boundary face f: nc + f)
-    auto sidx = [&](int c) { return c < nc ? rank[c] : nc + fpos[c - nc]; };
-
-    // LU-SGS level schedules from the reference's cell numbers, with each
-    // cell's entry count (neighbours on the sweep's side; the backward sweep
-    // also reads the ghosts of the cell's boundary faces)
-    std::vector<int> lev(nc, 0), cntF(nc, 0), cntB(nc, 0);
-    int nfl = 0;
-    for (int c = 0; c < nc; ++c) {
-        int l = 0;
-        for (int j = c2f_off[c]; j < c2f_off[c + 1]; ++j) {
-            const int f = c2f[j];
-            if (f < nb) { cntB[c]++; continue; }
-            const int o = h.left[f] == c ? h.right[f] : h.left[f];
-            if (o < c) { l = std::max(l, lev[o] + 1); cntF[c]++; }
-            else cntB[c]++;
-        }
-        lev[c] = l;
-        nfl = std::max(nfl, l + 1);
-    }
-    // Positions are slots of kSweepLanes lanes.  A cell with more entries
-    // than one slot holds takes two adjacent slots (the second continues its
-    // entries).  In each level the two-slot cells come first, so their slot
-    // pairs start at even slot numbers and never straddle a warp, and each
-    // level is padded with idle slots (-1) to a multiple of kSweepSlots, the
-    // slots of one warp, so that the slots one warp takes together always lie
-    // in one level and never depend on each other.
-    auto bucket = [&](int nlev, const std::vector<int> &cnt, std::vector<int> &cells, std::vector<uint8_t> &cont,
-                      bool ascending) {
-        std::vector<int> nbig(nlev, 0), nsmall(nlev, 0), off(nlev + 1, 0);
-        for (int c = 0; c < nc; ++c) (cnt[c] > kSweepLanes ? nbig : nsmall)[lev[c]]++;
-        for (int l = 0; l < nlev; ++l)
-            off[l + 1] = off[l] + (2 * nbig[l] + nsmall[l] + kSweepSlots - 1) / kSweepSlots * kSweepSlots;
-        cells.assign(off[nlev], -1);
-        cont.assign(off[nlev], 0);
-        std::vector<int> fbig(off.begin(), off.end() - 1), fsmall(nlev);
-        for (int l = 0; l < nlev; ++l) fsmall[l] = off[l] + 2 * nbig[l];
-        auto put = [&](int c) {
-            const int l = lev[c];
-            if (cnt[c] > kSweepLanes) {
-                cells[fbig[l]] = c;
-                cells[fbig[l] + 1] = c;
-                cont[fbig[l] + 1] = 1;
-                fbig[l] += 2;
-            } else {
-                cells[fsmall[l]++] = c;
+    // LU-SGS schedules from the reference's cell numbers, for the warps that are
+    // resident together
+    int maxWarps = ctx->mixed ? sweep_max_warps<float>(ctx->numSMs) : sweep_max_warps<double>(ctx->numSMs);
+    if (ctx->sa)
+        maxWarps = std::min(maxWarps, ctx->mixed ? sa_sweep_max_warps<float>(ctx->numSMs)
+                                                 : sa_sweep_max_warps<double>(ctx->numSMs));
+    cudaGetLastError();
+    struct Packed {
+        int nWarps = 0, nRows = 0;
+        // first, last: slot of each reference cell's first and last row; start: entries of the warps' first two rows
+        std::vector<int> rowOff, row, first, last, start;
+    } sweep[2];
+    std::vector<int2> use(nf, make_int2(-1, -1));
+    auto make_sweep = [&](int which) {
+        const bool forward = which == 0;
+        const SweepGraph graph{nc, nb, c2f_off.data(), c2f.data(), h.left.data(), h.right.data()};
+        SweepRows r = build_sweep(graph, forward, maxWarps);
+        Packed &p = sweep[which];
+        p.nWarps = r.nWarps;
+        p.nRows = r.rowOff[r.nWarps];
+        p.first.assign(nc, -1);
+        p.last.assign(nc, -1);
+        p.row.assign((size_t)p.nRows * kSweepRow, ~kSweepZero);
+        std::vector<int> lane((size_t)p.nRows * 32, ~kSweepZero);
+        std::vector<uint8_t> multi(p.nRows, 0);
+        for (size_t i = 0; i < r.cell.size(); ++i)
+            if (r.cell[i] >= 0 && (~r.flags[i] & (kSweepFirst | kSweepLast))) multi[i / kSweepSlots] = 1;
+        for (size_t i = 0; i < r.cell.size(); ++i) {
+            const int c = r.cell[i];
+            const size_t row = i / kSweepSlots;
+            int *info = &p.row[row * kSweepRow + 32 + i % kSweepSlots * 4];
+            info[0] = -1;
+            info[1] = r.store[row] * kSweepSlots + (int)(i % kSweepSlots) | (multi[row] ? kSweepMulti : 0);
+            info[2] = info[3] = 0;
+            if (c < 0) continue;
+            if (r.flags[i] & kSweepFirst) p.first[c] = (int)i;
+            else info[1] |= kSweepCarry;
+            if (r.flags[i] & kSweepLast) {
+                p.last[c] = (int)i;
+                info[0] = rank[c];
             }
-        };
-        if (ascending) for (int c = 0; c < nc; ++c) put(c);
-        else for (int c = nc - 1; c >= 0; --c) put(c);
-    };
-    std::vector<int> fwd_cells, bwd_cells;
-    std::vector<uint8_t> fwd_cont, bwd_cont;
-    bucket(nfl, cntF, fwd_cells, fwd_cont, true);
-    std::fill(lev.begin(), lev.end(), 0);
-    int nbl = 0;
-    for (int c = nc - 1; c >= 0; --c) {
-        int l = 0;
-        for (int j = c2f_off[c]; j < c2f_off[c + 1]; ++j) {
-            const int f = c2f[j];
-            if (f < nb) continue;
-            const int o = h.left[f] == c ? h.right[f] : h.left[f];
-            if (o > c) l = std::max(l, lev[o] + 1);
         }
-        lev[c] = l;
-        nbl = std::max(nbl, l + 1);
-    }
-    bucket(nbl, cntB, bwd_cells, bwd_cont, false);
-
-    // sweep entries (storage indices) of each cell in the cell's face order:
-    // {neighbour, face (sign bit set when the normal points into the cell),
-    // index of the face use's factors (2 f + side), 0}
-    auto cell_entries = [&](int c, bool forward, std::vector<int4> &e) {
-        e.clear();
-        for (int j = c2f_off[c]; j < c2f_off[c + 1]; ++j) {
-            const int f = c2f[j];
-            int nbr = -1;
-            bool isLeft = true;
-            if (f < nb) {
-                if (!forward) nbr = nc + f;
-            } else {
-                isLeft = h.left[f] == c;
-                const int o = isLeft ? h.right[f] : h.left[f];
-                if (forward ? (o < c) : (o > c)) nbr = o;
+        for (size_t e = 0; e < r.ent.size(); ++e) {
+            if (r.ent[e] < 0) continue;
+            const int c = r.cell[e / kSweepLanes], f = c2f[c2f_off[c] + r.ent[e]];
+            const bool isLeft = h.left[f] == c;
+            lane[e] = r.loc[e] >= 0 ? ~r.loc[e] : p.last[isLeft ? h.right[f] : h.left[f]];
+            (isLeft ? use[fpos[f]].x : use[fpos[f]].y) = forward ? (int)e : ~(int)e;
+        }
+        p.start.assign((size_t)p.nWarps * 64, ~kSweepZero);
+        for (int w = 0; w < p.nWarps; ++w)
+            for (int i = r.rowOff[w]; i < r.rowOff[w + 1]; ++i) {
+                const int k = i - r.rowOff[w];
+                int *to = k < 2 ? &p.start[(size_t)w * 64 + k * 32] : &p.row[(size_t)(i - 2) * kSweepRow];
+                std::copy(&lane[(size_t)i * 32], &lane[(size_t)i * 32] + 32, to);
             }
-            if (nbr < 0) continue;
-            e.push_back(make_int4(sidx(nbr), isLeft ? fpos[f] : (int)((unsigned)fpos[f] | 0x80000000u),
-                                  2 * fpos[f] + (isLeft ? 0 : 1), 0));
-        }
+        p.rowOff = std::move(r.rowOff);
     };
-    // per slot {storage cell, entry count} ({cell, -1} on the second slot of a
-    // two-slot cell) and kSweepLanes entries (neighbour -1 on unused lanes), so
-    // a lane reads its entry with one load and no offset lookup
-    auto pack = [&](const std::vector<int> &cells, const std::vector<uint8_t> &cont, bool forward,
-                    std::vector<int2> &pinfo, std::vector<int4> &ent) {
-        const size_t npos = cells.size();
-        pinfo.resize(npos);
-        ent.assign(npos * kSweepLanes, make_int4(-1, 0, 0, 0));
-        std::vector<int4> e;
-        for (size_t i = 0; i < npos; ++i) {
-            const int c = cells[i];
-            if (c < 0) { pinfo[i] = make_int2(-1, 0); continue; }
-            cell_entries(c, forward, e);
-            const int n = (int)e.size();
-            pinfo[i] = make_int2(rank[c], cont[i] ? -1 : n);
-            const int k0 = cont[i] ? kSweepLanes : 0;
-            for (int k = k0; k < std::min(n, k0 + kSweepLanes); ++k) ent[i * kSweepLanes + (k - k0)] = e[k];
-        }
-    };
-    std::vector<int2> fwd_pinfo, bwd_pinfo;
-    std::vector<int4> fwd_ent, bwd_ent;
-    pack(fwd_cells, fwd_cont, true, fwd_pinfo, fwd_ent);
-    pack(bwd_cells, bwd_cont, false, bwd_pinfo, bwd_ent);
+    make_sweep(0);
+    make_sweep(1);
+    if (std::max(sweep[0].nRows, sweep[1].nRows) > 0x7fffffff / 32) { delete ctx; return PHX_ERR_ARG; }
+    for (size_t i = 0; i < (size_t)sweep[0].nRows * kSweepSlots; ++i) {   // where the forward sweep leaves its sums
+        int *info = &sweep[0].row[i / kSweepSlots * kSweepRow + 32 + i % kSweepSlots * 4];
+        if (info[0] >= 0) info[2] = sweep[1].last[ord[info[0]]];
+    }
+    std::vector<int> lead(nc), last(nc);
+    for (int i = 0; i < nc; ++i) {
+        lead[i] = sweep[0].last[ord[i]];
+        last[i] = sweep[1].last[ord[i]];
+    }
+    // cells with boundary faces, in storage order
+    std::vector<int2> ghostCell;
+    {
+        std::vector<uint8_t> has(nc, 0);
+        for (int f = 0; f < nb; ++f) has[h.left[f]] = 1;
+        for (int i = 0; i < nc; ++i)
+            if (has[ord[i]]) ghostCell.push_back(make_int2(i, sweep[1].first[ord[i]]));
+    }
 
     // boundary classification (storage face order)
     std::vector<int32_t> bkind(nb), btype(nb);
@@ -1143,8 +1126,7 @@ int phx_ctx_create(const phx_grid_desc *gd, const phx_params *prm, phx_ctx **out
     DevGrid &g = ctx->g;
     g.nCell = nc; g.nBFace = nb; g.nFace = nf; g.nTotal = nt;
     g.avgVol = avgVol;
-    g.nFwdLevels = nfl; g.nBwdLevels = nbl;
-    g.nFwdPos = (int)fwd_cells.size(); g.nBwdPos = (int)bwd_cells.size();
+    g.nGhostCell = (int)ghostCell.size();
     g.walldist = nullptr;
     int rc = 0;
     if (ctx->sa) {
@@ -1182,10 +1164,18 @@ int phx_ctx_create(const phx_grid_desc *gd, const phx_params *prm, phx_ctx **out
             rc |= upload(ctx, &g.tn_pairs, ts.pairs);
         }
     }
-    rc |= upload(ctx, &g.fwd_pinfo, fwd_pinfo);
-    rc |= upload(ctx, &g.fwd_ent, fwd_ent);
-    rc |= upload(ctx, &g.bwd_pinfo, bwd_pinfo);
-    rc |= upload(ctx, &g.bwd_ent, bwd_ent);
+    for (int i = 0; i < 2; ++i) {
+        SweepDev &d = i == 0 ? g.fwd : g.bwd;
+        d.nWarps = sweep[i].nWarps;
+        d.nRows = sweep[i].nRows;
+        rc |= upload(ctx, &d.row_off, sweep[i].rowOff);
+        rc |= upload(ctx, &d.first, sweep[i].start);
+        ctx->sweepRows[i] = std::move(sweep[i].row);
+    }
+    rc |= upload(ctx, &g.use, use);
+    rc |= upload(ctx, &g.lead, lead);
+    rc |= upload(ctx, &g.last, last);
+    rc |= upload(ctx, &g.ghost_cell, ghostCell);
     rc |= dalloc(ctx, &ctx->q64[0], (size_t)5 * nt);
     rc |= dalloc(ctx, &ctx->q64[1], (size_t)5 * nt);
     rc |= dalloc(ctx, &ctx->tmp, (size_t)5 * nt);
@@ -1194,6 +1184,7 @@ int phx_ctx_create(const phx_grid_desc *gd, const phx_params *prm, phx_ctx **out
     if (!rc) rc = ctx->mixed ? make_work(ctx, ctx->w32, limInit) : make_work(ctx, ctx->w64, limInit);
     if (!rc && ctx->sa) rc = ctx->mixed ? make_turb(ctx, ctx->w32, ctx->t32) : make_turb(ctx, ctx->w64, ctx->t64);
     else if (!rc && prm->viscousType) rc = ctx->mixed ? make_visc(ctx, ctx->w32) : make_visc(ctx, ctx->w64);
+    for (auto &v : ctx->sweepRows) std::vector<int>().swap(v);
     if (!rc) rc = dalloc(ctx, &ctx->forces, 16);
     if (!rc && cudaMemset(ctx->red, 0, sizeof(Reduce)) != cudaSuccess) rc = PHX_ERR_CUDA;
     if (rc) {
@@ -1282,7 +1273,7 @@ int export_work(phx_ctx *ctx, const Work<T> &w, int which, int &rows, int &len)
     case PHX_GRADX: rows = 5; len = nt; launch_export<T>(g, w.grec, kG, 0, 5, 3, nc, ctx->tmp, nt, s); break;
     case PHX_GRADY: rows = 5; len = nt; launch_export<T>(g, w.grec, kG, 1, 5, 3, nc, ctx->tmp, nt, s); break;
     case PHX_GRADZ: rows = 5; len = nt; launch_export<T>(g, w.grec, kG, 2, 5, 3, nc, ctx->tmp, nt, s); break;
-    case PHX_DQ: rows = 5; len = nt; launch_export<T>(g, w.dqrec, kD, 0, 5, 1, nt, ctx->tmp, nt, s); break;
+    case PHX_DQ: rows = 5; len = nt; launch_export<T>(g, w.dqrec, kD, 0, 5, 1, nc, ctx->tmp, nt, s, g.last); break;
     case PHX_INVSPEC: rows = 1; len = nc; launch_export<T>(g, w.crec, kC, 6, 1, 1, nc, ctx->tmp, nc, s); break;
     case PHX_VISSPEC: rows = 1; len = nc; launch_export<T>(g, w.crec, kC, 7, 1, 1, nc, ctx->tmp, nc, s); break;
     case PHX_DT: rows = 1; len = nt; launch_export<T>(g, w.dtraw, 1, 0, 1, 1, nc, ctx->tmp, nt, s); break;
@@ -1490,7 +1481,7 @@ static int ns_lusgs(phx_ctx *ctx, int sweeps)
                       : launch_lusgs<double>(ctx->g, ctx->nc, ctx->w64, ctx->red, ctx->numSMs, ctx->stream, sweeps);
     if (e) return fail(ctx, PHX_ERR_CUDA, std::string("cooperative launch failed: ") + cudaGetErrorString((cudaError_t)e));
     ctx->nsForwardDone = sweeps == kSweepForward;
-    return check_launch(ctx, (sweeps & kSweepForward) ? 2 : 1);
+    return check_launch(ctx, sweeps == kSweepBoth ? 4 : 2);
 }
 
 static int refuse_zone(phx_ctx *ctx, const char *what)
@@ -1573,7 +1564,7 @@ static int sa_lusgs(phx_ctx *ctx, int sweeps)
                                                        ctx->stream, sweeps);
     if (e) return fail(ctx, PHX_ERR_CUDA, std::string("cooperative launch failed: ") + cudaGetErrorString((cudaError_t)e));
     ctx->saForwardDone = sweeps == kSweepForward;
-    return check_launch(ctx, (sweeps & kSweepForward) ? 2 : 1);
+    return check_launch(ctx, sweeps == kSweepBoth ? 3 : sweeps == kSweepForward ? 2 : 1);
 }
 
 int phx_sa_lusgs(phx_ctx *ctx)

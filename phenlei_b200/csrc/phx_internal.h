@@ -46,10 +46,34 @@ constexpr int kFlux = 16;  // face flux record: inviscid F0..4 (times area) | in
                            // spectral parts | pad | viscous F1..4 (times area; F0 is zero) | pad
 constexpr int kN = 8;      // nrec (GG-node): q node values (5), temperature node values of this
                            // iteration's state, those the gradient uses (the previous state's), pad
-constexpr int kCoef = 4;   // LU-SGS factors per face use: l1 x1 x2 | viscous spectral term
-constexpr int kSweepLanes = 4;   // LU-SGS lanes (neighbour entries) per schedule slot
-constexpr int kSweepSlots = 8;   // slots per warp: schedule levels are padded to this multiple
-constexpr int kSweepMaxEntries = 2 * kSweepLanes;   // entries of a cell: one slot, or two adjacent slots
+constexpr int kCoef = 4;   // LU-SGS factors of a boundary face: l1 x1 x2 | viscous spectral term
+// LU-SGS factors of an interior face use, as the sweeps read them: unit normal
+// from the cell to the neighbour, area | l1 x1 x2, viscous spectral term | the
+// neighbour's u v w c2 | total enthalpy, normal velocity, (gamma - 1) / 2 |u|^2, pad
+constexpr int kUse = 16;
+constexpr int kLeadF = 8;  // forward right-hand side of a cell: residual (5) | reciprocal diagonal | time step | pad
+constexpr int kLeadB = 16; // backward: residual less the forward sums (5), reciprocal diagonal, pad | boundary part (5), pad
+constexpr int kLeadT = 2;  // SA sweeps: right-hand side | reciprocal spectral radius
+constexpr int kSweepLanes = 4;   // LU-SGS lanes (neighbour entries) per slot of a schedule row
+constexpr int kSweepSlots = 8;   // slots (cells) of a row: one warp
+constexpr int kMaxCellFaces = 8; // faces of a cell
+constexpr int kSweepLocal = 4;   // shared-memory rows of a warp's own results
+constexpr int kSweepFirst = 8, kSweepLast = 16;   // flags of the host schedule: first, last row of a cell
+// A schedule row on the device (kSweepRow words): per lane the entry of the row
+// after next of its warp, the place of the neighbour's record (>= 0: it is
+// polled) or ~ the shared-memory slot of its result (kSweepZero: none, reads
+// zeros); then per slot {storage cell (-1: idle, or not the cell's last row),
+// shared-memory slot of the result | kSweepMulti (the row holds a cell of several
+// rows) | kSweepCarry (not the cell's first), forward: slot of the cell's last
+// backward row, 0}.
+constexpr int kSweepRow = 64, kSweepZero = kSweepLocal * kSweepSlots;
+constexpr int kSweepMulti = 256, kSweepCarry = 512;
+// Bytes of a row as the sweeps copy it: factors of the lanes' face uses, right-
+// hand sides of the cells, schedule row; NS (both sweeps) and SA.
+template <class T, bool kForward>
+constexpr int kRowNs = (32 * kUse + kSweepSlots * (kForward ? kLeadF : kLeadB)) * (int)sizeof(T) + kSweepRow * 4;
+template <class T>
+constexpr int kRowSa = (32 + kSweepSlots * kLeadT) * (int)sizeof(T) + kSweepRow * 4;
 constexpr long long kDefaultSpinLimit = 20000000LL;   // polls per dependency wait (~1-2 s)
 constexpr int kMaxDevices = 64;                       // per-device launch caches
 // Spalart-Allmaras records
@@ -58,6 +82,14 @@ constexpr int kTg = 4;     // tgrad: d nu~ / dx, dy, dz | pad
 constexpr int kTc = 4;     // tcrec: res_turb | spec_turb | pad
 constexpr int kTf = 8;     // tface: convective flux | diffusion flux1, flux2 | upwind Jacobians L, R |
                            // diffusion spectral term | pad
+
+// Schedule of one LU-SGS sweep (phx_schedule.cpp): warp w runs rows
+// [row_off[w], row_off[w + 1]).
+struct SweepDev {
+    int nWarps, nRows;
+    const int *row_off;
+    const int *first;    // [nWarps][2][32] entries of the warp's first two rows
+};
 
 // Read-only device grid (FP64 metrics, connectivity, schedules), storage order.
 struct DevGrid {
@@ -81,14 +113,13 @@ struct DevGrid {
     const int32_t *bkind;        // [nBFace] BcKind
     const int32_t *btype;        // [nBFace] bcType
     const uint8_t *farfield_adj; // [nCell] 1 if the cell touches a limiter-zeroing boundary
-    // LU-SGS schedules, slots in level order (levels padded with idle slots):
-    // pinfo = {storage cell or -1, entry count}, {cell, -1} on the second slot
-    // of a cell with more than kSweepLanes entries; ent = kSweepLanes entries
-    // per slot, the neighbours on the sweep's side in the cell's face order:
-    // {neighbour (-1: unused lane), face (sign bit set when the normal points
-    // into the cell), index of the face use's factors (2 f + side), 0}.
-    const int2 *fwd_pinfo, *bwd_pinfo;
-    const int4 *fwd_ent, *bwd_ent;
+    SweepDev fwd, bwd;           // LU-SGS schedules
+    const int2 *use;             // [nFace] lane (row * 32 + lane) of the left and of the right cell's use of the face;
+                                 // >= 0 in the forward sweep, ~ it in the backward sweep (interior faces)
+    const int *lead;             // [nCell] slot (row * kSweepSlots + slot) of the cell's last forward row
+    const int *last;             // [nCell] and of its last backward row
+    int nGhostCell;              // cells with boundary faces: {storage cell, slot of its first backward row}
+    const int2 *ghost_cell;
     // GG-node (gradientName 2): per storage node, its contributions {storage
     // cell, or storage boundary face with the sign bit set} with 1/distance
     // weights in the reference's order and their sum; per storage face, its
@@ -101,8 +132,6 @@ struct DevGrid {
     // pairs whose values it averages, in the reference's order
     const int *tn_off;
     const int2 *tn_pairs;
-    int nFwdLevels, nBwdLevels;
-    int nFwdPos, nBwdPos;        // schedule slots incl. idle padding (-1 cells)
     double avgVol;
 };
 
@@ -146,13 +175,15 @@ struct Work {
     T *qrec;        // [nTotal][kQ] working state, c2 = |gamma p / rho|, total enthalpy, limiter
     T *grec;        // [nTotal][kG] primitive gradients (ghost rows: interface ghosts only, from the halo exchange)
     T *flux;        // [nFace][kFlux] face flux times area and inviscid spectral radius term
-    T *coef;        // [2 nFace][kCoef] LU-SGS factors of each face use (side 0: the left cell's view)
+    T *coef;        // [nBFace][kCoef] LU-SGS factors of the boundary faces
+    unsigned char *rowf, *rowb;   // [rows][kRowNs] LU-SGS rows of the forward and the backward sweep
     T *crec;        // [nCell][kC] residual, diagonal, spectral radii
     T *dtraw;       // [nCell] CFL * vol / spectral radius, before the ktmax clamp
-    T *dqrec;       // [nTotal][kD] LU-SGS dq (backward sweep; write-once per sweep)
-    T *dqfwd;       // [nTotal][kD] forward-sweep dq (write-once per sweep; ghost rows: interface ghosts, from
-                    // the halo exchange between the sweeps)
-    T *dflux;       // [nCell][kD] delta flux carried from the forward to the backward sweep (write-once)
+    // LU-SGS dq, write-once per sweep, by the slot of the cell's last row (a
+    // row's eight records are written together, and mostly read together)
+    T *dqrec;       // [backward rows][kSweepSlots][kD] backward sweep
+    T *dqfwd;       // [forward rows][kSweepSlots][kD] forward sweep
+    T *dqghost;     // [nBFace][kD] forward dq behind interface faces, from the halo exchange between the sweeps
     T *trec;        // [nTotal][kTr] SA variable, eddy and laminar viscosity (SA runs; else null)
     T *nrec;        // [nNode][kN] GG-node node values (GG-node runs; else null)
 };
@@ -164,10 +195,9 @@ struct TurbWork {
     T *tgrad;       // [nCell][kTg] gradient of nu~
     T *tcrec;       // [nCell][kTc] residual, spectral radius, its reciprocal, pad
     T *tface;       // [nFace][kTf] face terms
-    T *tcoef;       // [2 nFace] LU-SGS matrix of each face use (side 0: left cell's view = mat_turbr)
-    T *tdq;         // [nCell] LU-SGS dq (backward sweep; write-once per sweep)
-    T *tdqf;        // [nCell] forward-sweep dq (write-once per sweep)
-    T *tdfl;        // [nCell] forward delta flux (write-once per sweep)
+    unsigned char *trowf, *trowb;   // [rows][kRowSa] LU-SGS rows
+    T *tdq;         // [backward rows][kSweepSlots] LU-SGS dq (write-once per sweep, by slot as the NS records)
+    T *tdqf;        // [forward rows][kSweepSlots] forward-sweep dq
     T *tsrc;        // [nCell] source computed by the learned-source kernel (sa_source != 0)
     T *qtnode;      // [nNode] GG-node node values of nu~ for the next SA gradient (GG-node runs; else null)
 };
@@ -186,6 +216,11 @@ template <class T>
 void launch_gradient_limiter(const DevGrid &g, const NsConst &c, const Work<T> &w, int nodePrev, cudaStream_t s);
 template <class T>
 void launch_residual(const DevGrid &g, const NsConst &c, const Work<T> &w, Reduce *red, double cfl, cudaStream_t s);
+// Resident warps of the sweeps (NS; SA's kernels hold at least as many).
+template <class T>
+int sweep_max_warps(int numSMs);
+template <class T>
+int sa_sweep_max_warps(int numSMs);
 // LU-SGS sweeps: bit 0 of `sweeps` runs the forward sweep (after resetting
 // the sweep records), bit 1 the backward sweep; 3 runs both in one launch.
 constexpr int kSweepForward = 1, kSweepBackward = 2, kSweepBoth = 3;
@@ -203,9 +238,10 @@ template <class T>
 void launch_sync_qrec(const DevGrid &g, const NsConst &c, const double *q64, const Work<T> &w, cudaStream_t s);
 // Export of record fields into reference-order SoA: out[k * outLen +
 // orig[i]] = rec[i * stride + first + k * step] for k < count, i < n.
+// `at` (if given): where record i lies.
 template <class T>
 void launch_export(const DevGrid &g, const T *rec, int stride, int first, int count, int step, int n, double *out,
-                   int outLen, cudaStream_t s);
+                   int outLen, cudaStream_t s, const int *at = nullptr);
 // q64[k][i] = in[k][orig[i]] and the inverse.
 void launch_import_q(const DevGrid &g, const double *in, double *q64, cudaStream_t s);
 void launch_export_q(const DevGrid &g, const double *q64, double *out, cudaStream_t s);

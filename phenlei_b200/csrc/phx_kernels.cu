@@ -390,7 +390,8 @@ void launch_gradient_limiter(const DevGrid &g, const NsConst &c, const Work<T> &
 // ---------------------------------------------------------------------------
 
 // dq-independent part of the neighbour's MXDQ_STD term for the use (cell ->
-// neighbour, normal pointing from cell to neighbour).
+// neighbour, normal pointing from cell to neighbour); o[3] is the normal
+// velocity of the neighbour.
 template <class T>
 __device__ __forceinline__ void lusgs_coef(const T *qc, const T *qn, T nx, T ny, T nz, T area, T gm, T *o)
 {
@@ -408,7 +409,37 @@ __device__ __forceinline__ void lusgs_coef(const T *qc, const T *qn, T nx, T ny,
     o[0] = a1;
     o[1] = (a1 + a1 - a2 - a3) / (c2 + c2);
     o[2] = (a2 - a3) / (cm + cm);
-    o[3] = T(0);
+    o[3] = cits;
+}
+
+// Where the sweeps' rows hold the factors of a face use (DevGrid::use), and a
+// cell's right-hand side (slot = row * kSweepSlots + slot).
+template <class T>
+__device__ __forceinline__ T *use_at(const Work<T> &w, int at)
+{
+    const int i = at < 0 ? ~at : at;
+    unsigned char *row = at < 0 ? w.rowb + (size_t)(i >> 5) * kRowNs<T, false> : w.rowf + (size_t)(i >> 5) * kRowNs<T, true>;
+    return reinterpret_cast<T *>(row) + (i & 31) * kUse;
+}
+template <class T, bool kForward>
+__device__ __forceinline__ T *lead_at(const Work<T> &w, int slot)
+{
+    unsigned char *row = (kForward ? w.rowf : w.rowb) + (size_t)(slot / kSweepSlots) * kRowNs<T, kForward>;
+    return reinterpret_cast<T *>(row) + 32 * kUse + (slot % kSweepSlots) * (kForward ? kLeadF : kLeadB);
+}
+
+// The factors of a face use (kUse) for the sweeps.
+template <class T>
+__device__ __forceinline__ void sweep_use(const T *qc, const T *qn, T nx, T ny, T nz, T area, T gm, T vspec, T *v)
+{
+    T cf[4];
+    lusgs_coef<T>(qc, qn, nx, ny, nz, area, gm, cf);
+    v[0] = nx; v[1] = ny; v[2] = nz; v[3] = area;
+    v[4] = cf[0]; v[5] = cf[1]; v[6] = cf[2]; v[7] = vspec;
+    v[8] = qn[1]; v[9] = qn[2]; v[10] = qn[3]; v[11] = qn[5];
+    v[12] = qn[6]; v[13] = cf[3];
+    v[14] = T(0.5) * (gm - T(1)) * (qn[1] * qn[1] + qn[2] * qn[2] + qn[3] * qn[3]);
+    v[15] = T(0);
 }
 
 // MUSCL state of one side (boundary ghosts carry a zero gradient, so their
@@ -653,15 +684,19 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1) face_flux_ke
     fl[6] = vspec;
     fl[7] = T(0);
     st8(w.flux + (size_t)f * kFlux, fl);
-    // LU-SGS factors: side 0 = the left cell's view, side 1 = the right cell's
-    T cf[4];
-    lusgs_coef<T>(qL, qR, xn, yn, zn, area, gm, cf);
-    cf[3] = vspec;
-    st4(w.coef + (size_t)(2 * f) * kCoef, cf);
-    if (f >= g.nBFace) {
-        lusgs_coef<T>(qR, qL, -xn, -yn, -zn, area, gm, cf);
+    // LU-SGS factors of the left cell's and the right cell's use
+    if (f < g.nBFace) {
+        T cf[4];
+        lusgs_coef<T>(qL, qR, xn, yn, zn, area, gm, cf);
         cf[3] = vspec;
-        st4(w.coef + (size_t)(2 * f + 1) * kCoef, cf);
+        st4(w.coef + (size_t)f * kCoef, cf);
+    } else {
+        const int2 at = ld(g.use + f);
+        T v[kUse];
+        sweep_use<T>(qL, qR, xn, yn, zn, area, gm, vspec, v);
+        put_use(use_at<T>(w, at.x), (at.x < 0 ? ~at.x : at.x) & 31, v);
+        sweep_use<T>(qR, qL, -xn, -yn, -zn, area, gm, vspec, v);
+        put_use(use_at<T>(w, at.y), (at.y < 0 ? ~at.y : at.y) & 31, v);
     }
 }
 
@@ -737,6 +772,9 @@ __global__ void __launch_bounds__(kThreads) cell_residual_kernel(DevGrid g, NsCo
         if (c.viscous) dd += vis;
         T out[8] = {res[0], res[1], res[2], res[3], res[4], idiv(T(1), dd), spec, vis};
         st8(w.crec + (size_t)cell * kC, out);
+        out[6] = dt;
+        out[7] = T(0);
+        st8(lead_at<T, true>(w, ld(g.lead + cell)), out);
     }
     // block minimum, then one atomic per block, skipped when it cannot lower
     // the running minimum (positive doubles order like their bit patterns)
@@ -774,56 +812,40 @@ void launch_residual(const DevGrid &g, const NsConst &c, const Work<T> &w, Reduc
 // LU-SGS (Controller::LUSGS, Controller.cpp:1878-1955) as a dataflow
 // computation.  The forward sweep of the reference visits cells in
 // increasing number and uses the just-updated dq of lower-numbered face
-// neighbours; the backward sweep the reverse.  Here the forward sweep writes
-// each cell's dq and delta flux into write-once records (dqfwd, dflux) and
-// the backward sweep writes the final dq into dqrec; all three are filled
-// with the sentinel before the sweep (sweep_reset_kernel), so a cell waits
-// only on the records of the neighbours it reads, polling the data itself,
-// and sees exactly the values the sequential sweep of the reference sees,
-// with no device-wide barrier and no completion flags.  Lane groups (one per
-// cell) take schedule positions in level order (forward positions, then
-// backward positions), the four groups of a warp four consecutive positions
-// of one level (levels are padded to multiples of four), so a warp only
-// waits on cells of earlier levels, held by other warps or by its own
-// earlier rounds.  All warps are co-resident (cooperative launch), so the
-// wait graph cannot cycle: the warp holding the lowest unfinished position
-// always has its inputs.  Every wait is bounded: a timeout sets
-// Reduce::error and the kernel gives up.  The dq-independent MXDQ_STD
-// factors were computed by the residual pass.
+// neighbours; the backward sweep the reverse.  Here each sweep is one launch of
+// one-warp blocks, each running its rows of the schedule (phx_schedule.cpp):
+// eight cells a row, four lanes a cell, a lane per neighbour.  A neighbour's
+// result is taken from the warp's shared memory where the schedule says that
+// this warp computed it and still holds it, and otherwise polled in its
+// write-once record (dqfwd, dqrec), filled with the sentinel before the sweep
+// (sweep_reset_kernel): the data is its own completion flag, and a cell sees
+// exactly the values the sequential sweep of the reference sees.  The records
+// of the row after next are polled while this row's sum is formed, so a warp that
+// runs behind the ones it reads from does not wait for L2 at all.  All warps
+// are co-resident (cooperative launch) and their rows ascend in level, so the
+// wait graph cannot cycle.  Every wait is bounded: a timeout sets
+// Reduce::error and the kernel gives up.  The dq-independent MXDQ_STD factors
+// were computed by the residual pass.
 // ---------------------------------------------------------------------------
 
 // Ghost-cell dq of a boundary face from the owner's forward dq dl
 // (SetGhostDQLUSGS, NSSolverUnstruct.cpp:14767-14810; SetSymmBCGhostDQLUSGS
-// :14812-14915; SetWallBCGhostDQLUSGS :14917-15006; far field 0).  The
-// dq-independent terms of the symmetry ghost (the owner's conservative state
-// Q, p_ghost / (gamma - 1), rho |u|^2 of the ghost) were formed before the
-// wait by ghost_static.
+// :14812-14915 with the owner's state ql and the ghost's qg;
+// SetWallBCGhostDQLUSGS :14917-15006; far field 0).
 template <class T>
-struct GhostStatic {
-    T Q[5];
-    T pmg, rmu2;
-};
-
-template <class T>
-__device__ __forceinline__ void ghost_static(const T *ql, const T *qg, T gm, GhostStatic<T> &s)
-{
-    const T r = ql[0], u = ql[1], v = ql[2], ww = ql[3], pp = ql[4];
-    const T em = idiv(idiv(pp, r), gm - T(1)) + T(0.5) * (u * u + v * v + ww * ww);
-    s.Q[0] = r; s.Q[1] = r * u; s.Q[2] = r * v; s.Q[3] = r * ww; s.Q[4] = r * em;
-    const T rm = qg[0], um = qg[1], vm = qg[2], wm = qg[3], pm = qg[4];
-    s.pmg = idiv(pm, gm - T(1));
-    s.rmu2 = rm * (um * um + vm * vm + wm * wm);
-}
-
-template <class T>
-__device__ __forceinline__ void ghost_dq(int kind, T xn, T yn, T zn, const GhostStatic<T> &s, const T *dl, T *o)
+__device__ __forceinline__ void ghost_dq(int kind, T xn, T yn, T zn, const T *ql, const T *qg, T gm, const T *dl, T *o)
 {
 #pragma unroll
     for (int k = 0; k < 5; ++k) o[k] = T(0);
     if (kind == BK_SYMMETRY) {
-        T Q[5];
+        const T r = ql[0], u = ql[1], v = ql[2], ww = ql[3], pp = ql[4];
+        const T em = idiv(idiv(pp, r), gm - T(1)) + T(0.5) * (u * u + v * v + ww * ww);
+        T Q[5] = {r, r * u, r * v, r * ww, r * em};
+        const T rm = qg[0], um = qg[1], vm = qg[2], wm = qg[3], pm = qg[4];
+        const T pmg = idiv(pm, gm - T(1));
+        const T rmu2 = rm * (um * um + vm * vm + wm * wm);
 #pragma unroll
-        for (int k = 0; k < 5; ++k) Q[k] = s.Q[k] + dl[k];
+        for (int k = 0; k < 5; ++k) Q[k] += dl[k];
         o[0] = dl[0];
         T rvn = T(2) * (xn * dl[1] + yn * dl[2] + zn * dl[3]);
         o[1] = dl[1] - xn * rvn;
@@ -831,332 +853,302 @@ __device__ __forceinline__ void ghost_dq(int kind, T xn, T yn, T zn, const Ghost
         o[3] = dl[3] - zn * rvn;
         rvn = T(2) * (xn * Q[1] + yn * Q[2] + zn * Q[3]);
         const T ru = Q[1] - xn * rvn, rv = Q[2] - yn * rvn, rw = Q[3] - zn * rvn;
-        const T rq0 = idiv(T(1), Q[0]);   // one division on the sweep's critical path, not two
+        const T rq0 = idiv(T(1), Q[0]);
         const T pnew = Q[4] - T(0.5) * (Q[1] * Q[1] + Q[2] * Q[2] + Q[3] * Q[3]) * rq0;
-        o[4] = pnew - s.pmg + T(0.5) * ((ru * ru + rv * rv + rw * rw) * rq0 - s.rmu2);
+        o[4] = pnew - pmg + T(0.5) * ((ru * ru + rv * rv + rw * rw) * rq0 - rmu2);
     } else if (kind == BK_WALL) {
         o[0] = dl[0]; o[1] = -dl[1]; o[2] = -dl[2]; o[3] = -dl[3]; o[4] = dl[4];
     }
 }
 
-// Static inputs of one schedule slot for one lane: the slot, this lane's
-// neighbour entry with its face, MXDQ factors and the neighbour's record,
-// and (lane 0 of the cell's first slot) the cell's residual record, time step
-// and volume.  Loaded into registers one round before the slot is processed,
-// so that only the neighbours' dq are waited for.
+// Delta flux of one neighbour (SolveLUSGSForward, NSSolverUnstruct.cpp:15118-15357):
+// MXDQ_STD with the use's factors u (kUse) and the neighbour's dq; the viscous
+// part for viscous runs.
 template <class T>
-struct SweepIn {
-    int cell, count;   // cell < 0: idle slot; count < 0: second slot of a two-slot cell
-    int nb, kind;      // neighbour storage index (-1: no entry); boundary kind of a ghost entry
-    T nx, ny, nz, area;
-    T cf[4];
-    T qn[8];
-    T ql[5];           // ghost entries: the owner cell's state
-    T cr[8];
-    T dt, vol;
-};
-
-template <class T, bool kForward>
-__device__ __forceinline__ void sweep_load(const DevGrid &g, const Work<T> &w, int2 info, int4 en, int lane,
-                                           SweepIn<T> &s)
+__device__ __forceinline__ void delta_flux(const T *u, T g1, int viscous, const T *dq, T *df)
 {
-    s.cell = info.x;
-    s.count = info.y;
-    s.nb = -1;
-    s.kind = -1;
-    const int nc = g.nCell;
-    if (info.x >= 0 && en.x >= 0) {
-        s.nb = en.x;
-        const int f = en.y & 0x7fffffff;
-        const T sgn = en.y < 0 ? T(-1) : T(1);
+    const T nx = u[0], ny = u[1], nz = u[2], area = u[3], um = u[8], vm = u[9], wm = u[10], cits = u[13];
+    const T dc = cits * dq[0] - nx * dq[1] - ny * dq[2] - nz * dq[3];
+    const T c2dc = u[11] * dc;
+    T dh = -g1 * (um * dq[1] + vm * dq[2] + wm * dq[3] - dq[4]);
+    dh += u[14] * dq[0];
+    const T a = dh * u[5] + dc * u[6];
+    const T b = c2dc * u[5] + dh * u[6];
+    df[0] = (u[4] * dq[0] - a) * area;
+    df[1] = (u[4] * dq[1] - um * a + nx * b) * area;
+    df[2] = (u[4] * dq[2] - vm * a + ny * b) * area;
+    df[3] = (u[4] * dq[3] - wm * a + nz * b) * area;
+    df[4] = (u[4] * dq[4] - u[12] * a + cits * b) * area;
+    if (viscous) {
+#pragma unroll
+        for (int m = 0; m < 5; ++m) df[m] -= u[7] * dq[m];
+    }
+}
+
+// Boundary part of the backward sweep: per cell with boundary faces the sum of
+// their ghosts' delta fluxes, in the cell's face order (the reference numbers
+// boundary faces first, so the backward sum starts with them).  An interface
+// ghost holds the neighbouring zone's forward dq, set by the halo exchange
+// between the sweeps (SetGhostDQLUSGS leaves it to CommunicationDQ,
+// Controller.cpp:1917-1924).  Everything here is known once the forward sweep
+// has ended; inside the sweep it sat on the critical path of the wall and
+// symmetry cells.
+template <class T>
+__global__ void __launch_bounds__(kThreads) sweep_ghost_kernel(DevGrid g, NsConst c, Work<T> w)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= g.nGhostCell) return;
+    const int2 gc = ld(g.ghost_cell + i);
+    const int cell = gc.x;
+    const T gm = (T)c.gama;
+    T ql[8], dl[8], sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    ld8(w.qrec + (size_t)cell * kQ, ql);
+    ld8(w.dqfwd + (size_t)ld(g.lead + cell) * kD, dl);
+    const int j1 = ld(g.c2f_off + cell + 1);
+    for (int j = ld(g.c2f_off + cell); j < j1; ++j) {
+        const int f = ld(g.c2f + j);
+        if (f >= g.nBFace) break;
+        const int kind = ld(g.bkind + f), ghost = g.nCell + f;
         double fr[4];
         ld4(g.frec + (size_t)f * kF, fr);
-        s.nx = sgn * (T)fr[0]; s.ny = sgn * (T)fr[1]; s.nz = sgn * (T)fr[2]; s.area = (T)fr[3];
-        ld4(w.coef + (size_t)en.z * kCoef, s.cf);
-        ld8(w.qrec + (size_t)en.x * kQ, s.qn);
-        if (!kForward && en.x >= nc) {
-            s.kind = ld(g.bkind + (en.x - nc));
-            T q8[8];
-            ld8(w.qrec + (size_t)info.x * kQ, q8);
+        const T nx = (T)fr[0], ny = (T)fr[1], nz = (T)fr[2], area = (T)fr[3];
+        T qg[8], cf[4], dq[8], df[5];
+        ld8(w.qrec + (size_t)ghost * kQ, qg);
+        ld4(w.coef + (size_t)f * kCoef, cf);
+        if (kind == BK_INTERFACE) ld8(w.dqghost + (size_t)f * kD, dq);
+        else ghost_dq<T>(kind, nx, ny, nz, ql, qg, gm, dl, dq);
+        const T v2 = qg[1] * qg[1] + qg[2] * qg[2] + qg[3] * qg[3];
+        const T u[kUse] = {nx, ny, nz, area, cf[0], cf[1], cf[2], cf[3], qg[1], qg[2], qg[3], qg[5], qg[6],
+                           nx * qg[1] + ny * qg[2] + nz * qg[3], T(0.5) * (gm - T(1)) * v2, T(0)};
+        delta_flux<T>(u, gm - T(1), c.viscous, dq, df);
 #pragma unroll
-            for (int k = 0; k < 5; ++k) s.ql[k] = q8[k];
-        }
+        for (int m = 0; m < 5; ++m) sum[m] += df[m];
     }
-    if (info.x >= 0 && info.y >= 0 && lane == 0) {
-        ld8(w.crec + (size_t)info.x * kC, s.cr);
-        s.dt = w.dtraw[info.x];
-        s.vol = (T)g.xrec[(size_t)info.x * kX + 3];
-    }
+    st8(lead_at<T, false>(w, gc.y) + 8, sum);
 }
 
-// One schedule slot of a sweep, processed by kSweepLanes lanes (one lane per
-// neighbour entry; a cell with more entries spans two adjacent slots, whose
-// first slot's lane 0 sums all of them).  The eight slots of a warp run in
-// lockstep: the warp polls until every lane's inputs are final, so no slot
-// ever spins while a sibling in the same warp is ready to work, and every
-// shuffle uses the full warp mask.  s.cell < 0 marks an idle slot (the
-// warp's trip count is uniform).
+// One sweep: a warp per block, so that the few warps of a small mesh spread over
+// the SMs.  What bounds it is the chain of dependent rows, about the sum of the
+// mesh's extents, times the time from a result to the next row's, and that is
+// the warp's instructions for a row one after the other (0.36 us forward, 0.29
+// us backward in single precision, 0.8 us where the records of a row are polled
+// when the row begins): whatever does not depend on dq is formed by the face and
+// cell passes or by the schedule, and a row arrives by one copy.
+// Both sweeps, mixed, against levels dealt out over all SMs with every result
+// through L2: 8k hexahedra 170 -> 107 us, 256x122x32 hexahedra 1001 -> 462 us,
+// the 1M-cell bump with prisms 970 -> 767 us.
+// Shared memory in front of the stages: the warp's results and a zero, barriers.
+template <class T>
+constexpr int kSweepHead = (kSweepZero + 1) * 8 * (int)sizeof(T) + (sizeof(T) == 4 ? 96 : 64);
+static_assert(kSweepHead<float> % 128 == 0 && kSweepHead<double> % 128 == 0, "aligned stages");
+
 template <class T, bool kForward>
-__device__ __forceinline__ bool sweep_position(const DevGrid &g, const NsConst &c, const Work<T> &w, Reduce *red,
-                                               double mindt, const SweepIn<T> &s, int lane, int base)
+__global__ void __launch_bounds__(32) lusgs_kernel(DevGrid g, NsConst c, Work<T> w, Reduce *red, int stages)
 {
-    const int nc = g.nCell;
-    const int cell = s.cell;
-    const bool live = cell >= 0;
-    const bool lead = live && s.count >= 0;   // the cell's first slot
-    const int e1 = lead ? s.count : 0;
-    const bool has = live && s.nb >= 0;
-    // wait for the inputs other positions write: the neighbour's dq (forward:
-    // its forward dq; backward: its final dq; a boundary ghost's comes from
-    // this cell's forward dq) and, backward, this cell's forward delta flux.
-    // An interface ghost holds the neighbouring zone's forward dq, set by the
-    // halo exchange between the sweeps (SetGhostDQLUSGS leaves it to
-    // CommunicationDQ, Controller.cpp:1917-1924).
-    const bool ghost = !kForward && has && s.nb >= nc;
-    const bool itfGhost = ghost && s.kind == BK_INTERFACE;
-    const T *src1 = !has ? nullptr
-                         : (ghost && !itfGhost) ? w.dqfwd + (size_t)cell * kD
-                                                : (kForward || itfGhost ? w.dqfwd : w.dqrec) + (size_t)s.nb * kD;
-    const T *src2 = (!kForward && lead && lane == 0) ? w.dflux + (size_t)cell * kD : nullptr;
-    T v1[5], fl[5];
-    bool r1 = !src1 || poll5(src1, v1);
-    bool r2 = !src2 || poll5(src2, fl);
-    const T gm = (T)c.gama;
-    // dq-independent terms, formed while the first poll is in flight:
-    // the reciprocal of the diagonal (NSSolverUnstruct.cpp:15867-15935),
-    // 1 / (dt' / vol) + spectral radii, dt' = min(dt, ktmax min dt)
-    // (ReduceMaxTimeStep, :5717-5745) -- formed by the residual pass for the
-    // raw dt, here only where the clamp applies -- and the symmetry ghost's
-    // static terms.  dq is then (res - flux) times the reciprocal: IEEE
-    // divisions after the wait held the publishing lanes for up to 2 us
-    // (per-cell timestamps), on the critical path of every level.
-    T rd = T(1);
-    if (lead && lane == 0) {
-        const T clamp = (T)(c.ktmax * mindt);
-        if (c.ktmax > 0 && s.dt > clamp) {
-            // the clamp applies: the residual pass's reciprocal is for the raw dt
-            const T dt = idiv(clamp, s.vol);
-            T d = idiv(T(1), dt);
-            d += s.cr[6];
-            if (c.viscous) d += s.cr[7];
-            rd = idiv(T(1), d);
-        } else {
-            rd = s.cr[5];
-        }
-    }
-    GhostStatic<T> gs;
-    if (ghost && s.kind == BK_SYMMETRY) ghost_static<T>(s.ql, s.qn, gm, gs);
-    // fault injection (phx_fault_hold_cell): the held cell's lead lane waits on
-    // nothing that is ever set, so its wait runs out
-    if (kForward && lead && lane == 0 && cell == c.holdCell) r2 = false;
-    long long spins = 0;
-    while (!__all_sync(0xffffffffu, r1 && r2)) {
-        ++spins;
-        if (spins > c.spinLimit) {
-            if ((threadIdx.x & 31) == 0) atomicExch(&red->error, PHX_ERR_TIMEOUT);
-            return false;
-        }
-        if ((spins & 1023) == 0 && __any_sync(0xffffffffu, ((volatile int *)&red->error)[0] != 0)) return false;
-        if (spins > 8) __nanosleep(20);
-        if (!r1) r1 = poll5(src1, v1);
-        if (!r2 && src2) r2 = poll5(src2, fl);
-    }
-    T df[5] = {0, 0, 0, 0, 0};
-    if (has) {
-        T dq[5];
-        if (ghost && !itfGhost) {
-            ghost_dq<T>(s.kind, s.nx, s.ny, s.nz, gs, v1, dq);
-        } else {
+    using Pipe = RowPipe<kRowNs<T, kForward>>;
+    constexpr int kLead = kForward ? kLeadF : kLeadB, kRow = kRowNs<T, kForward>;
+    constexpr int kLeadOff = 32 * kUse * (int)sizeof(T), kRowOff = kRow - kSweepRow * 4;
+    extern __shared__ __align__(128) unsigned char sm[];
+    T *loc = reinterpret_cast<T *>(sm);
+    const SweepDev &sw = kForward ? g.fwd : g.bwd;
+    const int t = threadIdx.x, slot = t / kSweepLanes, lane = t % kSweepLanes;
+    const int row0 = ld(sw.row_off + blockIdx.x), nrow = ld(sw.row_off + blockIdx.x + 1) - row0;
+    if (nrow <= 0) return;
+    if (t < 8) loc[kSweepZero * 8 + t] = T(0);
+    const double mindt = __longlong_as_double((long long)red->mindt_bits);
+    const T clamp = c.ktmax > 0 ? (T)(c.ktmax * mindt) : (T)kLarge;
+    const T g1 = (T)c.gama - T(1);
+    const int viscous = c.viscous, held = kForward && c.holdCell >= 0 ? c.holdCell : -2;
+    T *out = kForward ? w.dqfwd : w.dqrec;
+    T *mine = out + ((size_t)row0 * kSweepSlots + slot) * kD;   // record of this slot in the current row
+    Pipe pipe;
+    pipe.start(sm + kSweepHead<T>, reinterpret_cast<uint64_t *>(loc + (kSweepZero + 1) * 8), kForward ? w.rowf : w.rowb,
+               row0, nrow, stages, t);
+    // the entry of this lane in a row, and a first look at the record it polls
+    auto entry = [&](const int *p, int &en, T *v) {
+        en = p[t];
+        if (en >= 0) poll5_load(out + (size_t)en * kD, v);
+    };
+    T va[5], vb[5], rhs[5];
+    int ea, eb;
+    entry(sw.first + blockIdx.x * 64, ea, va);
+    entry(sw.first + blockIdx.x * 64 + 32, eb, vb);
+    bool ok = true;
+    auto step = [&](int i, int &en, T *v) -> bool {
+        const unsigned char *row = pipe.at(pipe.slot) + i * kRow;
+        const int4 info = reinterpret_cast<const int4 *>(row + kRowOff + 128)[slot];
+        const T *lead = reinterpret_cast<const T *>(row + kLeadOff) + slot * kLead;
+        T u[kUse];
+        get_use(reinterpret_cast<const T *>(row), t, u);
+        if (en < 0) {
+            const T *a = loc + ~en * 8;
+            T b[4];
+            get4(a, b);
 #pragma unroll
-            for (int k = 0; k < 5; ++k) dq[k] = v1[k];
+            for (int m = 0; m < 4; ++m) v[m] = b[m];
+            v[4] = a[4];
         }
-        const T nx = s.nx, ny = s.ny, nz = s.nz, area = s.area;
-        const T um = s.qn[1], vm = s.qn[2], wm = s.qn[3], c2 = s.qn[5], hm = s.qn[6];
-        const T *cf = s.cf;
-        const T cits = nx * um + ny * vm + nz * wm;
-        const T dc = cits * dq[0] - nx * dq[1] - ny * dq[2] - nz * dq[3];
-        const T c2dc = c2 * dc;
-        const T v2 = um * um + vm * vm + wm * wm;
-        const T g1 = gm - T(1);
-        T dh = -g1 * (um * dq[1] + vm * dq[2] + wm * dq[3] - dq[4]);
-        dh += T(0.5) * g1 * v2 * dq[0];
-        const T a = dh * cf[1] + dc * cf[2];
-        const T b = c2dc * cf[1] + dh * cf[2];
-        df[0] = (cf[0] * dq[0] - a) * area;
-        df[1] = (cf[0] * dq[1] - um * a + nx * b) * area;
-        df[2] = (cf[0] * dq[2] - vm * a + ny * b) * area;
-        df[3] = (cf[0] * dq[3] - wm * a + nz * b) * area;
-        df[4] = (cf[0] * dq[4] - hm * a + cits * b) * area;
-        if (c.viscous) {
-            // viscous part of the delta flux (SolveLUSGSForward, :15339-15357)
-#pragma unroll
-            for (int m = 0; m < 5; ++m) df[m] -= cf[3] * dq[m];
+        // fault injection (phx_fault_hold_cell): the held cell waits on
+        // nothing that is ever set, so its wait runs out
+        const bool hold = kForward && lane == 0 && info.x == held;
+        bool ready = (en < 0 || poll5_done(v)) && !hold;
+        if (!__all_sync(0xffffffffu, ready)) {
+            long long spins = 0;
+            do {
+                ++spins;
+                if (spins > c.spinLimit) {
+                    if (t == 0) atomicExch(&red->error, PHX_ERR_TIMEOUT);
+                    return false;
+                }
+                if ((spins & 1023) == 0 && __any_sync(0xffffffffu, ((volatile int *)&red->error)[0] != 0)) return false;
+                if (!ready && en >= 0) ready = poll5(out + (size_t)en * kD, v) && !hold;
+            } while (!__all_sync(0xffffffffu, ready));
         }
-    }
-    // in-order accumulation (entries are in the cell's face order; lanes
-    // past the cell's entry count are skipped); the second slot's lanes only
-    // when the warp holds a two-slot cell
-    T rhs0[5] = {0, 0, 0, 0, 0};
-#pragma unroll
-    for (int k = 0; k < kSweepLanes; ++k) {
-#pragma unroll
-        for (int m = 0; m < 5; ++m) {
-            const T v = __shfl_sync(0xffffffffu, df[m], base + k);
-            if (k < e1) rhs0[m] += v;
-        }
-    }
-    if (__any_sync(0xffffffffu, e1 > kSweepLanes)) {
-#pragma unroll
-        for (int k = kSweepLanes; k < kSweepMaxEntries; ++k) {
-#pragma unroll
-            for (int m = 0; m < 5; ++m) {
-                const T v = __shfl_sync(0xffffffffu, df[m], (base + k) & 31);
-                if (k < e1) rhs0[m] += v;
-            }
-        }
-    }
-    if (lead && lane == 0) {
-        T o[5];
+        T df[5];
+        delta_flux<T>(u, g1, viscous, v, df);
+        // the row after next, while this row's sum is formed
+        entry(reinterpret_cast<const int *>(row + kRowOff), en, v);
+        // sum in the cell's face order, on the cell's first lane; the backward
+        // sum starts with the boundary faces
+        T sum[5];
         if (kForward) {
+#pragma unroll
+            for (int m = 0; m < 5; ++m) sum[m] = df[m];
+        } else {
+            T b[4];
+            get4(lead + (kForward ? 0 : 8), b);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) sum[m] = b[m] + df[m];
+            sum[4] = lead[kForward ? 0 : 12] + df[4];
+        }
+        if ((info.y & kSweepMulti) && (info.y & kSweepCarry)) {
+#pragma unroll
+            for (int m = 0; m < 5; ++m) sum[m] = rhs[m] + df[m];
+        }
+#pragma unroll
+        for (int j = 1; j < kSweepLanes; ++j) {
+#pragma unroll
+            for (int m = 0; m < 5; ++m) sum[m] += __shfl_down_sync(0xffffffffu, df[m], j);
+        }
+        if (info.y & kSweepMulti) {
+#pragma unroll
+            for (int m = 0; m < 5; ++m) rhs[m] = sum[m];
+        }
+        __syncwarp();   // the row's reads of loc
+        if (lane == 0 && info.x >= 0) {
+            // reciprocal of the diagonal (NSSolverUnstruct.cpp:15867-15935),
+            // 1 / (dt' / vol) + spectral radii, dt' = min(dt, ktmax min dt)
+            // (ReduceMaxTimeStep, :5717-5745): formed by the residual pass for
+            // the raw dt, by the forward sweep where the clamp applies
+            T q[8], o[5];
+            get8(lead, q);
+            if (kForward && q[6] > clamp) {
+                const T *cr = w.crec + (size_t)info.x * kC;
+                T d = idiv(T(1), idiv(clamp, (T)ld(g.xrec + (size_t)info.x * kX + 3)));
+                d += ld(cr + 6);
+                if (viscous) d += ld(cr + 7);
+                q[5] = idiv(T(1), d);
+            }
             // dq = (res - Ux - L dq) / D, Ux = 0 for a single sweep
             // (LUSGSInitialization, Controller.cpp:1765-1777)
-            T fo[5];
 #pragma unroll
-            for (int k = 0; k < 5; ++k) { o[k] = (s.cr[k] - T(0) - rhs0[k]) * rd; fo[k] = T(0) + rhs0[k]; }
-            publish5(w.dflux + (size_t)cell * kD, fo);
-            publish5(w.dqfwd + (size_t)cell * kD, o);
-        } else {
-#pragma unroll
-            for (int k = 0; k < 5; ++k) o[k] = (s.cr[k] - fl[k] - rhs0[k]) * rd;
-            publish5(w.dqrec + (size_t)cell * kD, o);
+            for (int m = 0; m < 5; ++m) { q[m] -= sum[m]; o[m] = q[m] * q[5]; }
+            T *own = loc + (info.y & 255) * 8;
+            st4(own, o);
+            own[4] = o[4];
+            publish5(mine, o);
+            if (kForward) st8(lead_at<T, false>(w, info.z), q);
         }
-    }
-    return true;
-}
-
-// One sweep over the schedule: rounds of ngroups positions.  The entries
-// ({cell, count} and this lane's neighbour entry) are loaded two rounds
-// ahead and the records they point to one round ahead (into registers, and
-// into L2 a round before that), so a position starts by polling.
-template <class T, bool kForward>
-__device__ __forceinline__ bool sweep_all(const DevGrid &g, const NsConst &c, const Work<T> &w, Reduce *red,
-                                          double mindt, int group, int wgroup0, int ngroups, int lane, int base)
-{
-    const int npos = kForward ? g.nFwdPos : g.nBwdPos;
-    const int2 *pinfo = kForward ? g.fwd_pinfo : g.bwd_pinfo;
-    const int4 *ent = kForward ? g.fwd_ent : g.bwd_ent;
-    auto entry = [&](int p, int2 &info, int4 &en) {
-        info = make_int2(-1, 0);
-        en = make_int4(-1, 0, 0, 0);
-        if (p < npos) { info = __ldg(pinfo + p); en = __ldg(ent + (size_t)p * kSweepLanes + lane); }
+        mine += kSweepSlots * kD;
+        __syncwarp();
+        return true;
     };
-    int p = group;
-    int2 info;
-    int4 en;
-    entry(p, info, en);
-    SweepIn<T> cur;
-    sweep_load<T, kForward>(g, w, info, en, lane, cur);
-    entry(p + ngroups, info, en);   // entries of the next round
-    for (int p0 = wgroup0; p0 < npos; p0 += ngroups) {
-        SweepIn<T> nxt;
-        sweep_load<T, kForward>(g, w, info, en, lane, nxt);
-        entry(p + 2 * ngroups, info, en);
-        if (!sweep_position<T, kForward>(g, c, w, red, mindt, cur, lane, base)) return false;
-        // the records of the round after next into L2 (its entries have arrived)
-        if (en.x >= 0) {
-            prefetch_l2(g.frec + (size_t)(en.y & 0x7fffffff) * kF);
-            prefetch_l2(w.coef + (size_t)en.z * kCoef);
-            prefetch_l2(w.qrec + (size_t)en.x * kQ);
-        }
-        if (lane == 0 && info.x >= 0 && info.y >= 0) {
-            prefetch_l2(w.crec + (size_t)info.x * kC);
-            prefetch_l2(w.dtraw + info.x);
-        }
-        cur = nxt;
-        p += ngroups;
+    int k = 0;
+    while (ok && k < pipe.nstage) {
+        ok = pipe.wait() && step(0, ea, va) && (2 * k + 1 >= nrow || step(1, eb, vb));
+        if (!ok) break;
+        pipe.advance(t);
+        ++k;
     }
-    return true;
+    if (!ok) {
+        if (t == 0 && ((volatile int *)&red->error)[0] == 0) atomicExch(&red->error, PHX_ERR_TIMEOUT);
+        __syncwarp();
+        pipe.drain(k);
+    }
 }
 
+// Fills the sweeps' polled records (forward dq, final dq) with the sentinel.
 template <class T>
-__global__ void __launch_bounds__(kSweepThreads) lusgs_kernel(DevGrid g, NsConst c, Work<T> w, Reduce *red,
-                                                              int sweeps)
+__global__ void __launch_bounds__(kThreads) sweep_reset_kernel(int rowsF, int rowsB, T *f, T *b)
 {
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int group = tid / kSweepLanes, lane = tid % kSweepLanes;   // slot lane group
-    const int ngroups = (gridDim.x * blockDim.x) / kSweepLanes;
-    const int wgroup0 = group & ~(kSweepSlots - 1);   // first group of this warp
-    const int base = (threadIdx.x & 31) & ~(kSweepLanes - 1);
-    const double mindt = __longlong_as_double((long long)red->mindt_bits);
-    if ((sweeps & kSweepForward) && !sweep_all<T, true>(g, c, w, red, mindt, group, wgroup0, ngroups, lane, base))
-        return;
-    if (sweeps & kSweepBackward) sweep_all<T, false>(g, c, w, red, mindt, group, wgroup0, ngroups, lane, base);
+    constexpr int kQuads = kSweepSlots * kD / 4;
+    const T s = sweep_sentinel<T>(), v[4] = {s, s, s, s};
+    const long long nf = (long long)rowsF * kQuads, nb = (long long)rowsB * kQuads, n = max(nf, nb);
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        if (i < nf) st4(f + i * 4, v);
+        if (i < nb) st4(b + i * 4, v);
+    }
 }
 
-// Fills the sweep's output records (forward dq, forward delta flux, final dq)
-// with the sentinel: 8-element records, 16-byte stores.
+// Shared memory of a sweep's warp with the given number of stages.
+template <class T, bool kForward>
+static int sweep_smem(int stages) { return kSweepHead<T> + stages * RowPipe<kRowNs<T, kForward>>::kStage; }
+
+// Warps of the sweeps that are resident together with two stages each: the
+// schedule is made for at most this many.  PHX_LUSGS_MAX_BLOCKS caps them
+// (tuning; tests of many rows per warp).
 template <class T>
-__global__ void __launch_bounds__(kThreads) sweep_reset_kernel(int n, T *a, T *b, T *c)
+int sweep_max_warps(int numSMs)
 {
-    const T s = sweep_sentinel<T>();
-    const long long tot = (long long)n * kD;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i * 4 < tot;
-         i += (long long)gridDim.x * blockDim.x) {
-        const T v[4] = {s, s, s, s};
-        st4(a + i * 4, v);
-        st4(b + i * 4, v);
-        st4(c + i * 4, v);
-    }
-}
-
-// Grid of the sweeps: every resident lane group (cooperative launch), at most
-// one group per schedule position.
-template <class K>
-static int sweep_blocks(K kernel, int &perSM, const DevGrid &g, int numSMs)
-{
-    if (perSM < 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kernel, kSweepThreads, 0);
-        if (perSM < 1) perSM = 1;
-    }
-    int blocks = numSMs * perSM;
-    const int npos = g.nFwdPos > g.nBwdPos ? g.nFwdPos : g.nBwdPos;
-    const int need = (int)(((long long)npos * kSweepLanes + kSweepThreads - 1) / kSweepThreads);
-    if (blocks > need) blocks = need;
-    // PHX_LUSGS_MAX_BLOCKS caps the grid (tuning; tests of many positions per group)
+    cudaFuncSetAttribute(lusgs_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sweep_smem<T, true>(4));
+    cudaFuncSetAttribute(lusgs_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sweep_smem<T, false>(4));
+    int f = 0, b = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, lusgs_kernel<T, true>, 32, sweep_smem<T, true>(2));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, lusgs_kernel<T, false>, 32, sweep_smem<T, false>(2));
+    int n = std::max(1, std::min(std::min(f, b), 16)) * numSMs;
     if (const char *cap = getenv("PHX_LUSGS_MAX_BLOCKS")) {
         const int v = atoi(cap);
-        if (v > 0 && blocks > v) blocks = v;
+        if (v > 0 && n > v) n = v;
     }
-    return blocks < 1 ? 1 : blocks;
+    return n;
+}
+template int sweep_max_warps<double>(int);
+template int sweep_max_warps<float>(int);
+
+template <class T, bool kForward>
+static cudaError_t launch_sweep(const DevGrid &g, const NsConst &c, const Work<T> &w, Reduce *red, int numSMs, cudaStream_t s)
+{
+    const int warps = (kForward ? g.fwd : g.bwd).nWarps;
+    // more stages where the warps leave shared memory to spare (224 KB of an SM,
+    // 1 KB of each block the system's)
+    int stages = 2;
+    const int perSM = (warps + numSMs - 1) / numSMs;
+    while (stages < 4 && perSM * (sweep_smem<T, kForward>(stages + 1) + 1024) <= 224 * 1024) ++stages;
+    DevGrid gg = g;
+    NsConst cc = c;
+    Work<T> ww = w;
+    Reduce *rr = red;
+    void *args[] = {&gg, &cc, &ww, &rr, &stages};
+    return cudaLaunchCooperativeKernel((void *)lusgs_kernel<T, kForward>, dim3(warps), dim3(32), args,
+                                       sweep_smem<T, kForward>(stages), s);
 }
 
 template <class T>
 int launch_lusgs(const DevGrid &g, const NsConst &c, const Work<T> &w, Reduce *red, int numSMs, cudaStream_t s,
                  int sweeps)
 {
-    // residency of the cooperative launch, per device (a process may drive several)
-    static int perSMcache[kMaxDevices][2];
-    static bool init = false;
-    if (!init) {
-        for (auto &d : perSMcache) d[0] = d[1] = -1;
-        init = true;
+    cudaError_t e = cudaSuccess;
+    if (sweeps & kSweepForward) {
+        const long long n = (long long)std::max(g.fwd.nRows, g.bwd.nRows) * kSweepSlots * kD / 4;
+        const int rb = (int)std::min<long long>((n + kThreads - 1) / kThreads, (long long)numSMs * 16);
+        sweep_reset_kernel<T><<<rb, kThreads, 0, s>>>(g.fwd.nRows, g.bwd.nRows, w.dqfwd, w.dqrec);
+        e = launch_sweep<T, true>(g, c, w, red, numSMs, s);
     }
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= kMaxDevices) return (int)cudaErrorInvalidDevice;
-    const int blocks = sweep_blocks(lusgs_kernel<T>, perSMcache[dev][sizeof(T) == 8 ? 0 : 1], g, numSMs);
-    const long long quads = (long long)g.nCell * kD / 4;
-    const int rb = (int)std::min<long long>((quads + kThreads - 1) / kThreads, (long long)numSMs * 16);
-    if (sweeps & kSweepForward)
-        sweep_reset_kernel<T><<<rb > 0 ? rb : 1, kThreads, 0, s>>>(g.nCell, w.dqfwd, w.dflux, w.dqrec);
-    DevGrid gg = g;
-    NsConst cc = c;
-    Work<T> ww = w;
-    Reduce *rr = red;
-    int sw = sweeps;
-    void *args[] = {&gg, &cc, &ww, &rr, &sw};
-    const cudaError_t e =
-        cudaLaunchCooperativeKernel((void *)lusgs_kernel<T>, dim3(blocks), dim3(kSweepThreads), args, 0, s);
+    if (e == cudaSuccess && (sweeps & kSweepBackward)) {
+        if (g.nGhostCell > 0)
+            sweep_ghost_kernel<T><<<(g.nGhostCell + kThreads - 1) / kThreads, kThreads, 0, s>>>(g, c, w);
+        e = launch_sweep<T, false>(g, c, w, red, numSMs, s);
+    }
     return e == cudaSuccess ? 0 : (int)e;
 }
 
@@ -1189,7 +1181,7 @@ __global__ void __launch_bounds__(kThreads) update_kernel(DevGrid g, NsConst c, 
             const double em = (p / r) / (gm - 1.0) + 0.5 * (u * u + v * v + ww * ww);
             double Q[5] = {r, r * u, r * v, r * ww, r * em};
             T dq[8];
-            ld8(w.dqrec + (size_t)cell * kD, dq);
+            ld8(w.dqrec + (size_t)ld(g.last + cell) * kD, dq);
 #pragma unroll
             for (int k = 0; k < 5; ++k) Q[k] += (double)dq[k];
             double prim[5];
@@ -1333,20 +1325,20 @@ void launch_solution_fix(const DevGrid &g, const NsConst &c, const Work<T> &w, c
 // ---------------------------------------------------------------------------
 template <class T>
 __global__ void export_kernel(DevGrid g, const T *rec, int stride, int first, int count, int step, int n, double *out,
-                              int outLen)
+                              int outLen, const int *at)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int o = g.orig[i];
-    for (int k = 0; k < count; ++k) out[(size_t)k * outLen + o] = (double)rec[(size_t)i * stride + first + k * step];
+    const int o = g.orig[i], r = at ? at[i] : i;
+    for (int k = 0; k < count; ++k) out[(size_t)k * outLen + o] = (double)rec[(size_t)r * stride + first + k * step];
 }
 
 template <class T>
 void launch_export(const DevGrid &g, const T *rec, int stride, int first, int count, int step, int n, double *out,
-                   int outLen, cudaStream_t s)
+                   int outLen, cudaStream_t s, const int *at)
 {
     export_kernel<T><<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(g, rec, stride, first, count, step, n, out,
-                                                                       outLen);
+                                                                       outLen, at);
 }
 
 __global__ void import_q_kernel(DevGrid g, const double *in, double *q)
@@ -1450,7 +1442,8 @@ void launch_finish_step(Reduce *r, double *hist, int i, double ncell, cudaStream
                                          double *, Reduce *, int *, cudaStream_t);                                  \
     template void launch_sync_qrec<T>(const DevGrid &, const NsConst &, const double *, const Work<T> &,            \
                                       cudaStream_t);                                                                \
-    template void launch_export<T>(const DevGrid &, const T *, int, int, int, int, int, double *, int, cudaStream_t);
+    template void launch_export<T>(const DevGrid &, const T *, int, int, int, int, int, double *, int, cudaStream_t, \
+                                   const int *);
 PHX_INSTANTIATE(double)
 PHX_INSTANTIATE(float)
 

@@ -29,11 +29,6 @@ namespace phx {
 // ---------------------------------------------------------------------------
 // tcgen05 / TMEM / mbarrier helpers (inline PTX, sm_100a)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void *p)
-{
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
 // Shared-memory matrix descriptor: canonical K-major layout without swizzle,
 // core matrices of 8 rows x 16 bytes; lbo = byte distance between the two
 // 8-element K chunks of one MMA, sbo = byte distance between 8-row groups;
@@ -69,29 +64,6 @@ __device__ __forceinline__ void umma_commit(uint64_t *mbar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(mbar))
                  : "memory");
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t *mbar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mbar)), "r"(count) : "memory");
-}
-
-// Bounded wait for the mbarrier phase with the given parity; false on timeout.
-__device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity)
-{
-    const uint32_t a = smem_u32(mbar);
-    for (long long i = 0; i < (1LL << 26); ++i) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(done)
-            : "r"(a), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
 }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }

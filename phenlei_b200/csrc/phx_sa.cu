@@ -188,6 +188,20 @@ __global__ void __launch_bounds__(kThreads) sa_visc_grad_kernel(DevGrid g, NsCon
     st4(t.tgrad + (size_t)cell * kTg, o);
 }
 
+// Where the SA sweeps' rows hold the matrix of a face use (DevGrid::use), and a
+// cell's right-hand side (slot = row * kSweepSlots + slot).
+template <class T>
+__device__ __forceinline__ T *sa_use_at(const TurbWork<T> &t, int at)
+{
+    const int i = at < 0 ? ~at : at;
+    return reinterpret_cast<T *>((at < 0 ? t.trowb : t.trowf) + (size_t)(i >> 5) * kRowSa<T>) + (i & 31);
+}
+template <class T>
+__device__ __forceinline__ T *sa_lead_at(unsigned char *rows, int slot)
+{
+    return reinterpret_cast<T *>(rows + (size_t)(slot / kSweepSlots) * kRowSa<T>) + 32 + (slot % kSweepSlots) * kLeadT;
+}
+
 // ---------------------------------------------------------------------------
 // SA face pass (one thread per face):
 //  * convection: GetQlQrTurbulence / GetQlQrNS (TurbSolverUnstr.cpp:4978-5140;
@@ -307,8 +321,11 @@ __global__ void __launch_bounds__(kThreads) sa_face_kernel(DevGrid g, NsConst c,
         matR += oRe * ovol * ns2 * cr;
     }
     st8(t.tface + (size_t)f * kTf, out);
-    t.tcoef[2 * (size_t)f] = matR;
-    if (!bnd) t.tcoef[2 * (size_t)f + 1] = matL;
+    if (f >= g.nBFace) {
+        const int2 at = ld(g.use + f);
+        *sa_use_at<T>(t, at.x) = matR;
+        *sa_use_at<T>(t, at.y) = matL;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -387,6 +404,9 @@ __global__ void __launch_bounds__(kThreads) sa_cell_kernel(DevGrid g, NsConst c,
     }
     T o[4] = {res, spec, idiv(T(1), spec), T(0)};   // the sweep multiplies by the reciprocal
     st4(t.tcrec + (size_t)cell * kTc, o);
+    T *lead = sa_lead_at<T>(t.trowf, ld(g.lead + cell));
+    lead[0] = o[0];
+    lead[1] = o[2];
 }
 
 template <class T>
@@ -413,204 +433,141 @@ void launch_sa_residual(const DevGrid &g, const NsConst &c, const double *q64, c
 // TurbSolverUnstr.cpp:1400-1638): dq = (res - L/U dq - rhs0) / spec_turb with
 // the face matrices of each face use.  Same dataflow schedule, write-once
 // records and bounded waits as the NS sweep (phx_kernels.cu): tdqf (forward
-// dq), tdfl (forward delta flux) and tdq (final dq) hold the sentinel until
-// written.  dq of the ghosts is the ghost residual, which is zero, so ghost
-// entries of the backward sweep add nothing and are skipped; an interface
-// ghost's too, as the reference exchanges no SA dq between the sweeps
-// (Controller::CommunicationDQ, CFD/Solver/src/Controller.cpp:2874-2880).
+// dq) and tdq (final dq) hold the sentinel until written.  dq of the ghosts is
+// the ghost residual, which is zero, so boundary faces add nothing; an
+// interface ghost's neither, as the reference exchanges no SA dq between the
+// sweeps (Controller::CommunicationDQ, CFD/Solver/src/Controller.cpp:2874-2880).
 // ---------------------------------------------------------------------------
-// Static inputs of one slot for one lane (loaded a round ahead): neighbour
-// (-1: none or a ghost), its face matrix, and (lane 0 of the cell's first
-// slot) the cell's residual and the reciprocal of its spectral radius.
-template <class T>
-struct SaSweepIn {
-    int cell, count, nb;
-    T mat, res, rspec;
-};
-
-template <class T>
-__device__ __forceinline__ void sa_sweep_load(const DevGrid &g, const TurbWork<T> &t, int2 info, int4 en, int lane,
-                                              SaSweepIn<T> &s)
-{
-    s.cell = info.x;
-    s.count = info.y;
-    s.nb = -1;
-    if (info.x >= 0 && en.x >= 0 && en.x < g.nCell) {
-        s.nb = en.x;
-        s.mat = t.tcoef[en.z];
-    }
-    if (info.x >= 0 && info.y >= 0 && lane == 0) {
-        T cr[4];
-        ld4(t.tcrec + (size_t)info.x * kTc, cr);
-        s.res = cr[0];
-        s.rspec = cr[2];
-    }
-}
+// Bound by the chain of rows as the NS sweep (0.23 us a row); a row is small, so
+// 16 of them are in flight.  Both sweeps, mixed: 256x122x32 hexahedra 767 -> 351
+// us, the 1M-cell bump with prisms 771 -> 533 us.
+static constexpr int kSaStages = 8;
 
 template <class T, bool kForward>
-__device__ __forceinline__ bool sa_sweep_position(const TurbWork<T> &t, Reduce *red, const SaSweepIn<T> &s, int lane,
-                                                  int base, long long spinLimit)
+__global__ void __launch_bounds__(32) sa_lusgs_kernel(DevGrid g, TurbWork<T> t, Reduce *red, long long spinLimit)
 {
-    const int cell = s.cell;
-    const bool live = cell >= 0;
-    const bool lead = live && s.count >= 0;   // the cell's first slot
-    const int e1 = lead ? s.count : 0;
-    const bool has = live && s.nb >= 0;
-    // the neighbour's dq (forward: its forward dq; backward: its final dq)
-    // and, backward, this cell's forward delta flux
-    const T *src1 = has ? (kForward ? t.tdqf : t.tdq) + s.nb : nullptr;
-    const T *src2 = (!kForward && lead && lane == 0) ? t.tdfl + cell : nullptr;
-    T v1 = T(0), fl = T(0);
-    bool r1 = true, r2 = true;
-    if (src1) { v1 = ld_poll(src1); r1 = !is_sentinel(v1); }
-    if (src2) { fl = ld_poll(src2); r2 = !is_sentinel(fl); }
-    // the SA cell pass formed the reciprocal of the spectral radius (a division
-    // on the sweep's critical path costs up to microseconds; see the NS sweep)
-    const T rspec = s.rspec;
-    long long spins = 0;
-    while (!__all_sync(0xffffffffu, r1 && r2)) {
-        ++spins;
-        if (spins > spinLimit) {
-            if ((threadIdx.x & 31) == 0) atomicExch(&red->error, PHX_ERR_TIMEOUT);
-            return false;
-        }
-        if ((spins & 1023) == 0 && __any_sync(0xffffffffu, ((volatile int *)&red->error)[0] != 0)) return false;
-        if (spins > 8) __nanosleep(20);
-        if (!r1) { v1 = ld_poll(src1); r1 = !is_sentinel(v1); }
-        if (!r2) { fl = ld_poll(src2); r2 = !is_sentinel(fl); }
-    }
-    const T df = has ? s.mat * v1 : T(0);
-    T rhs0 = T(0);
-#pragma unroll
-    for (int k = 0; k < kSweepLanes; ++k) {
-        const T v = __shfl_sync(0xffffffffu, df, base + k);
-        if (k < e1) rhs0 += v;
-    }
-    if (__any_sync(0xffffffffu, e1 > kSweepLanes)) {
-#pragma unroll
-        for (int k = kSweepLanes; k < kSweepMaxEntries; ++k) {
-            const T v = __shfl_sync(0xffffffffu, df, (base + k) & 31);
-            if (k < e1) rhs0 += v;
-        }
-    }
-    if (lead && lane == 0) {
-        if (kForward) {
-            st_relaxed(t.tdfl + cell, unsentinel(T(0) + rhs0));
-            st_relaxed(t.tdqf + cell, unsentinel((s.res - T(0) - rhs0) * rspec));
-        } else {
-            st_relaxed(t.tdq + cell, unsentinel((s.res - fl - rhs0) * rspec));
-        }
-    }
-    return true;
-}
-
-// Rounds of ngroups positions; entries loaded two rounds ahead, the face
-// matrices and residual records one round ahead.
-template <class T, bool kForward>
-__device__ __forceinline__ bool sa_sweep_all(const DevGrid &g, const TurbWork<T> &t, Reduce *red, int group,
-                                             int wgroup0, int ngroups, int lane, int base, long long spinLimit)
-{
-    const int npos = kForward ? g.nFwdPos : g.nBwdPos;
-    const int2 *pinfo = kForward ? g.fwd_pinfo : g.bwd_pinfo;
-    const int4 *ent = kForward ? g.fwd_ent : g.bwd_ent;
-    auto entry = [&](int p, int2 &info, int4 &en) {
-        info = make_int2(-1, 0);
-        en = make_int4(-1, 0, 0, 0);
-        if (p < npos) { info = __ldg(pinfo + p); en = __ldg(ent + (size_t)p * kSweepLanes + lane); }
+    constexpr int kRow = kRowSa<T>, kRowOff = kRow - kSweepRow * 4;
+    using Pipe = RowPipe<kRow>;
+    __shared__ __align__(128) unsigned char buf[kSaStages * Pipe::kStage];
+    __shared__ T loc[kSweepZero + 1];
+    __shared__ uint64_t bars[kSaStages];
+    const SweepDev &sw = kForward ? g.fwd : g.bwd;
+    const int th = threadIdx.x, slot = th / kSweepLanes, lane = th % kSweepLanes;
+    const int row0 = ld(sw.row_off + blockIdx.x), nrow = ld(sw.row_off + blockIdx.x + 1) - row0;
+    if (nrow <= 0) return;
+    if (th == 0) loc[kSweepZero] = T(0);
+    T *out = kForward ? t.tdqf : t.tdq;
+    T *mine = out + (size_t)row0 * kSweepSlots + slot;   // record of this slot in the current row
+    Pipe pipe;
+    pipe.start(buf, bars, kForward ? t.trowf : t.trowb, row0, nrow, kSaStages, th);
+    // the entry of this lane in a row, and a first look at the record it polls
+    auto entry = [&](const int *p, int &en, T &v) {
+        en = p[th];
+        if (en >= 0) v = ld_poll(out + en);
     };
-    int p = group;
-    int2 info;
-    int4 en;
-    entry(p, info, en);
-    SaSweepIn<T> cur;
-    sa_sweep_load<T>(g, t, info, en, lane, cur);
-    entry(p + ngroups, info, en);
-    for (int p0 = wgroup0; p0 < npos; p0 += ngroups) {
-        SaSweepIn<T> nxt;
-        sa_sweep_load<T>(g, t, info, en, lane, nxt);
-        entry(p + 2 * ngroups, info, en);
-        if (!sa_sweep_position<T, kForward>(t, red, cur, lane, base, spinLimit)) return false;
-        if (en.x >= 0 && en.x < g.nCell) prefetch_l2(t.tcoef + en.z);
-        if (lane == 0 && info.x >= 0 && info.y >= 0) prefetch_l2(t.tcrec + (size_t)info.x * kTc);
-        cur = nxt;
-        p += ngroups;
+    T va = T(0), vb = T(0), rhs = T(0);
+    int ea, eb;
+    entry(sw.first + blockIdx.x * 64, ea, va);
+    entry(sw.first + blockIdx.x * 64 + 32, eb, vb);
+    bool ok = true;
+    auto step = [&](int i, int &en, T &v) -> bool {
+        const unsigned char *row = pipe.at(pipe.slot) + i * kRow;
+        const int4 info = reinterpret_cast<const int4 *>(row + kRowOff + 128)[slot];
+        const T mat = reinterpret_cast<const T *>(row)[th];
+        const T *lead = reinterpret_cast<const T *>(row) + 32 + slot * kLeadT;
+        const T r0 = lead[0], rspec = lead[1];
+        if (en < 0) v = loc[~en];
+        bool ready = en < 0 || !is_sentinel(v);
+        if (!__all_sync(0xffffffffu, ready)) {
+            long long spins = 0;
+            do {
+                ++spins;
+                if (spins > spinLimit) {
+                    if (th == 0) atomicExch(&red->error, PHX_ERR_TIMEOUT);
+                    return false;
+                }
+                if ((spins & 1023) == 0 && __any_sync(0xffffffffu, ((volatile int *)&red->error)[0] != 0)) return false;
+                if (!ready) { v = ld_poll(out + en); ready = !is_sentinel(v); }
+            } while (!__all_sync(0xffffffffu, ready));
+        }
+        const T df = mat * v;
+        // the row after next, while this row's sum is formed
+        entry(reinterpret_cast<const int *>(row + kRowOff), en, v);
+        T sum = (info.y & kSweepMulti) && (info.y & kSweepCarry) ? rhs + df : df;
+#pragma unroll
+        for (int j = 1; j < kSweepLanes; ++j) sum += __shfl_down_sync(0xffffffffu, df, j);
+        if (info.y & kSweepMulti) rhs = sum;
+        __syncwarp();   // the row's reads of loc
+        if (lane == 0 && info.x >= 0) {
+            // the SA cell pass formed the reciprocal of the spectral radius
+            const T q = r0 - sum, o = q * rspec;
+            loc[info.y & 255] = o;
+            st_relaxed(mine, unsentinel(o));
+            if (kForward) {
+                T *nxt = sa_lead_at<T>(t.trowb, info.z);
+                nxt[0] = q;
+                nxt[1] = rspec;
+            }
+        }
+        mine += kSweepSlots;
+        __syncwarp();
+        return true;
+    };
+    int k = 0;
+    while (ok && k < pipe.nstage) {
+        ok = pipe.wait() && step(0, ea, va) && (2 * k + 1 >= nrow || step(1, eb, vb));
+        if (!ok) break;
+        pipe.advance(th);
+        ++k;
     }
-    return true;
+    if (!ok) {
+        if (th == 0 && ((volatile int *)&red->error)[0] == 0) atomicExch(&red->error, PHX_ERR_TIMEOUT);
+        __syncwarp();
+        pipe.drain(k);
+    }
 }
 
+// Fills the SA sweeps' polled records with the sentinel.
 template <class T>
-__global__ void __launch_bounds__(kSweepThreads) sa_lusgs_kernel(DevGrid g, TurbWork<T> t, Reduce *red,
-                                                                 long long spinLimit, int sweeps)
-{
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int group = tid / kSweepLanes, lane = tid % kSweepLanes;
-    const int ngroups = (gridDim.x * blockDim.x) / kSweepLanes;
-    const int wgroup0 = group & ~(kSweepSlots - 1);
-    const int base = (threadIdx.x & 31) & ~(kSweepLanes - 1);
-    if ((sweeps & kSweepForward) && !sa_sweep_all<T, true>(g, t, red, group, wgroup0, ngroups, lane, base, spinLimit))
-        return;
-    if (sweeps & kSweepBackward) sa_sweep_all<T, false>(g, t, red, group, wgroup0, ngroups, lane, base, spinLimit);
-}
-
-// Fills the SA sweep's output records with the sentinel.
-template <class T>
-__global__ void __launch_bounds__(kThreads) sa_sweep_reset_kernel(int n, T *a, T *b, T *c)
+__global__ void __launch_bounds__(kThreads) sa_sweep_reset_kernel(int nf, int nb, T *f, T *b)
 {
     const T s = sweep_sentinel<T>();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        a[i] = s;
-        b[i] = s;
-        c[i] = s;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < max(nf, nb); i += gridDim.x * blockDim.x) {
+        if (i < nf) f[i] = s;
+        if (i < nb) b[i] = s;
     }
 }
+
+template <class T>
+int sa_sweep_max_warps(int numSMs)
+{
+    int f = 0, b = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, sa_lusgs_kernel<T, true>, 32, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, sa_lusgs_kernel<T, false>, 32, 0);
+    return std::max(1, std::min(f, b)) * numSMs;
+}
+template int sa_sweep_max_warps<double>(int);
+template int sa_sweep_max_warps<float>(int);
 
 template <class T>
 int launch_sa_lusgs(const DevGrid &g, const NsConst &c, const Work<T> &w, const TurbWork<T> &t, Reduce *red,
                     int numSMs, cudaStream_t s, int sweeps)
 {
     (void)w;
-    // residency of the cooperative launch, per device (a process may drive several)
-    static int perSMcache[kMaxDevices][2];
-    static bool init = false;
-    if (!init) {
-        for (auto &d : perSMcache) d[0] = d[1] = -1;
-        init = true;
-    }
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= kMaxDevices) return (int)cudaErrorInvalidDevice;
-    int &resident = perSMcache[dev][sizeof(T) == 8 ? 0 : 1];
-    if (resident < 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, sa_lusgs_kernel<T>, kSweepThreads, 0);
-        if (resident < 1) resident = 1;
-    }
-    // at most two blocks per SM: the scalar sweep does little work per poll,
-    // and more polling slots only load L2 (16M cells: 4.1 ms at two blocks per
-    // SM against 4.5 ms at six); PHX_SA_SWEEP_BLOCKS_PER_SM changes the cap
-    // (tuning)
-    int cap = 2;
-    if (const char *e = getenv("PHX_SA_SWEEP_BLOCKS_PER_SM")) cap = atoi(e) > 0 ? atoi(e) : cap;
-    const int perSM = resident < cap ? resident : cap;
-    int blocks = numSMs * perSM;
-    const int npos = g.nFwdPos > g.nBwdPos ? g.nFwdPos : g.nBwdPos;
-    const int need = (int)(((long long)npos * kSweepLanes + kSweepThreads - 1) / kSweepThreads);
-    if (blocks > need) blocks = need;
-    if (const char *cap = getenv("PHX_LUSGS_MAX_BLOCKS")) {
-        const int v = atoi(cap);
-        if (v > 0 && blocks > v) blocks = v;
-    }
-    if (blocks < 1) blocks = 1;
-    const int rb = std::min((g.nCell + kThreads - 1) / kThreads, numSMs * 16);
-    if (sweeps & kSweepForward)
-        sa_sweep_reset_kernel<T><<<rb > 0 ? rb : 1, kThreads, 0, s>>>(g.nCell, t.tdqf, t.tdfl, t.tdq);
     DevGrid gg = g;
     TurbWork<T> tt = t;
     Reduce *rr = red;
     long long lim = c.spinLimit;
-    int sw = sweeps;
-    void *args[] = {&gg, &tt, &rr, &lim, &sw};
-    const cudaError_t e =
-        cudaLaunchCooperativeKernel((void *)sa_lusgs_kernel<T>, dim3(blocks), dim3(kSweepThreads), args, 0, s);
+    void *args[] = {&gg, &tt, &rr, &lim};
+    cudaError_t e = cudaSuccess;
+    if (sweeps & kSweepForward) {
+        const int nf = g.fwd.nRows * kSweepSlots, nb = g.bwd.nRows * kSweepSlots;
+        const int rb = std::min((std::max(nf, nb) + kThreads - 1) / kThreads, numSMs * 16);
+        sa_sweep_reset_kernel<T><<<rb, kThreads, 0, s>>>(nf, nb, t.tdqf, t.tdq);
+        e = cudaLaunchCooperativeKernel((void *)sa_lusgs_kernel<T, true>, dim3(g.fwd.nWarps), dim3(32), args, 0, s);
+    }
+    if (e == cudaSuccess && (sweeps & kSweepBackward))
+        e = cudaLaunchCooperativeKernel((void *)sa_lusgs_kernel<T, false>, dim3(g.bwd.nWarps), dim3(32), args, 0, s);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
@@ -621,7 +578,7 @@ __global__ void __launch_bounds__(kThreads) sa_update_kernel(DevGrid g, Work<T> 
 {
     const int cell = blockIdx.x * blockDim.x + threadIdx.x;
     if (cell >= g.nCell) return;
-    const double v = t.qt64[cell] + (double)t.tdq[cell];
+    const double v = t.qt64[cell] + (double)t.tdq[ld(g.last + cell)];
     t.qt64[cell] = v;
     w.trec[(size_t)cell * kTr] = (T)v;
 }
