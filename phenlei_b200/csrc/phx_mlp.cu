@@ -8,7 +8,7 @@
 // swizzle), FP32 accumulators in tensor memory (TMEM), tcgen05.mma issued by
 // one thread and completed through an mbarrier, results read back with
 // tcgen05.ld.  The last layer (64 -> 1) is a dot product on the CUDA cores.
-// Training uses hand-written FP32 forward / backward / Adam kernels.
+// Training uses one FP32 kernel for forward and backward, and one for Adam.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -429,115 +429,252 @@ void launch_mlp_capture(const DevGrid &g, const NsConst &c, const Work<T> &w, co
 }
 
 // ---------------------------------------------------------------------------
-// Training (FP32, CUDA cores): C[M x N] (+)= op(A) op(B) with element strides
-// A(i, k) = A[i * as0 + k * as1], B(k, j) = B[k * bs0 + j * bs1]; 16 x 16 tiles.
+// Training (FP32, CUDA cores).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) mlp_gemm_kernel(int M, int N, int K, const float *A, long long as0,
-                                                       long long as1, const float *B, long long bs0, long long bs1,
-                                                       float *C, int ldc, const float *bias, int accumulate)
+// flat parameter vector: w1 b1 w2 b2 w3 b3 w4 b4 (weights row-major [out][in])
+constexpr int kNW1 = kMlpH * kMlpIn, kNW2 = kMlpH * kMlpH, kNW3 = kMlpH * kMlpH;
+constexpr int kOffW1 = 0, kOffB1 = kOffW1 + kNW1, kOffW2 = kOffB1 + kMlpH, kOffB2 = kOffW2 + kNW2;
+constexpr int kOffW3 = kOffB2 + kMlpH, kOffB3 = kOffW3 + kNW3, kOffW4 = kOffB3 + kMlpH, kOffB4 = kOffW4 + kMlpH;
+constexpr int kNParam = kOffB4 + 1;
+
+// Samples of one batch: row b is sample perm[b] (or b), its features less the
+// mean times rstd (or as they are), its target times tinv.
+struct MlpRows {
+    const float *x, *y;
+    const int *perm;
+    const float *mean, *rstd;
+    float tinv;
+};
+
+// Forward and backward pass of a batch of B rows and the gradient of the mean
+// squared error, in tiles of 64 rows: a tile goes through all layers in one
+// block, its activations in shared memory (as the tile products read them: rows
+// by columns and transposed) and its pre-activations in registers, and the
+// weight gradients of a block's tiles stay in registers until the end
+// (part[block][kNParam]).  256 threads, 4 x 4 outputs each, six 64 x 64 x 64
+// products a tile.  A batch of 8,192 is 128 blocks of one tile: 29 us, bound by
+// the FP32 pipe of one block per SM, and 6 us for the sum over the blocks with
+// Adam.  The products layer by layer that it replaces took 1.43 ms, four of them,
+// the weight gradients, on at most 16 blocks with a serial sum over the batch.
+constexpr int kTrRows = 64, kTrThreads = 256, kTrS = 68;   // kTrS: padded row of a 64 x 64 tile
+constexpr int kTrTile = 64 * kTrS;
+constexpr int kTrSmemFloats = 4 * kTrTile + 7 * kTrTile + 64 * 8 + kNW1 + 5 * 64 + 2 * 64 + 16;
+
+__device__ __forceinline__ void tile_mma(const float *a, const float *b, int ty, int tx, float (*acc)[4])
 {
-    __shared__ float sa[16][17], sb[16][17];
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-    const int i = blockIdx.y * 16 + ty, j = blockIdx.x * 16 + tx;
-    float acc = 0.0f;
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        const int ka = k0 + tx, kb = k0 + ty;
-        sa[ty][tx] = (i < M && ka < K) ? A[i * as0 + ka * as1] : 0.0f;
-        sb[ty][tx] = (kb < K && j < N) ? B[kb * bs0 + j * bs1] : 0.0f;
+#pragma unroll 8
+    for (int k = 0; k < 64; ++k) {
+        const float4 u = *reinterpret_cast<const float4 *>(a + k * kTrS + ty * 4);
+        const float4 v = *reinterpret_cast<const float4 *>(b + k * kTrS + tx * 4);
+        const float ua[4] = {u.x, u.y, u.z, u.w}, va[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] += ua[i] * va[j];
+    }
+}
+__device__ __forceinline__ void tile_put(float *rows, float *cols, int ty, int tx, const float (*v)[4])
+{
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<float4 *>(rows + (ty * 4 + i) * kTrS + tx * 4) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+    if (cols) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<float4 *>(cols + (tx * 4 + j) * kTrS + ty * 4) = make_float4(v[0][j], v[1][j], v[2][j], v[3][j]);
+    }
+}
+
+__global__ void __launch_bounds__(kTrThreads) mlp_grad_kernel(const float *p, MlpRows in, int B, float *part, float *loss)
+{
+    extern __shared__ __align__(16) float ts[];
+    float *w2t = ts, *w3t = w2t + kTrTile, *w2 = w3t + kTrTile, *w3 = w2 + kTrTile;
+    float *h1 = w3 + kTrTile, *h1t = h1 + kTrTile, *h2 = h1t + kTrTile, *h2t = h2 + kTrTile, *h3 = h2t + kTrTile;
+    float *dz = h3 + kTrTile, *dzt = dz + kTrTile;
+    float *x = dzt + kTrTile;                       // [64][8]
+    float *w1 = x + 64 * 8, *b1 = w1 + kNW1, *b2 = b1 + 64, *b3 = b2 + 64, *w4 = b3 + 64;
+    float *dy = w4 + 64, *err = dy + 64;            // [64], [64]
+    const int t = threadIdx.x, tx = t % 16, ty = t / 16;
+    for (int i = t; i < kNW2; i += kTrThreads) {
+        const int o = i / 64, k = i % 64;
+        const float a = p[kOffW2 + i], b = p[kOffW3 + i];
+        w2[o * kTrS + k] = a; w2t[k * kTrS + o] = a;
+        w3[o * kTrS + k] = b; w3t[k * kTrS + o] = b;
+    }
+    for (int i = t; i < kNW1; i += kTrThreads) w1[i] = p[kOffW1 + i];
+    if (t < 64) { b1[t] = p[kOffB1 + t]; b2[t] = p[kOffB2 + t]; b3[t] = p[kOffB3 + t]; w4[t] = p[kOffW4 + t]; }
+    const float b4 = p[kOffB4];
+    float g3[4][4] = {}, g2[4][4] = {};             // dW3, dW2 of rows ty * 4.., columns tx * 4..
+    float g1[2] = {0.0f, 0.0f};                     // dW1 of elements t, t + 256
+    float gb = 0.0f, gw4 = 0.0f, gb4 = 0.0f, sq = 0.0f;   // gb: b3, b2, b1 on threads 0-63, 64-127, 128-191
+    const int tiles = (B + kTrRows - 1) / kTrRows;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        __syncthreads();
+        for (int i = t; i < kTrRows * kMlpIn; i += kTrThreads) {
+            const int r = i / kMlpIn, k = i % kMlpIn, row = tile * kTrRows + r;
+            float v = 0.0f;
+            if (row < B) {
+                v = in.x[(size_t)(in.perm ? in.perm[row] : row) * kMlpIn + k];
+                if (in.mean) v = (v - in.mean[k]) * in.rstd[k];
+            }
+            x[r * 8 + k] = v;
+        }
+        __syncthreads();
+        // d silu / dz and the activations, layer by layer
+        float s1[4][4], s2[4][4], s3[4][4], v[4][4];
+        auto silu = [&](float (*z)[4], float (*d)[4]) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float q = z[i][j], sg = 1.0f / (1.0f + expf(-q));
+                    d[i][j] = sg * (1.0f + q * (1.0f - sg));
+                    z[i][j] = q * sg;
+                }
+        };
+        auto bias = [&](const float *b, float (*z)[4]) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) z[i][j] += b[tx * 4 + j];
+        };
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float z = 0.0f;
+#pragma unroll
+                for (int k = 0; k < kMlpIn; ++k) z += x[(ty * 4 + i) * 8 + k] * w1[(tx * 4 + j) * kMlpIn + k];
+                v[i][j] = z;
+            }
+        bias(b1, v);
+        silu(v, s1);
+        tile_put(h1, h1t, ty, tx, v);
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < 16; ++k) acc += sa[ty][k] * sb[k][tx];
-        __syncthreads();
-    }
-    if (i < M && j < N) {
-        if (bias) acc += bias[j];
-        float *cp = C + (size_t)i * ldc + j;
-        *cp = accumulate ? *cp + acc : acc;
-    }
-}
-
-void mlp_gemm(int M, int N, int K, const float *A, long long as0, long long as1, const float *B, long long bs0,
-              long long bs1, float *C, int ldc, const float *bias, bool accumulate, cudaStream_t s)
-{
-    dim3 grid((N + 15) / 16, (M + 15) / 16);
-    mlp_gemm_kernel<<<grid, 256, 0, s>>>(M, N, K, A, as0, as1, B, bs0, bs1, C, ldc, bias, accumulate ? 1 : 0);
-}
-
-// h = silu(z) (forward) or dz = dh * silu'(z) (backward), n elements.
-__global__ void mlp_silu_kernel(long long n, const float *z, float *h, const float *dh, float *dz)
-{
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float x = z[i];
-    const float sg = 1.0f / (1.0f + expf(-x));
-    if (h) h[i] = x * sg;
-    if (dz) dz[i] = dh[i] * (sg * (1.0f + x * (1.0f - sg)));
-}
-
-void mlp_silu(long long n, const float *z, float *h, const float *dh, float *dz, cudaStream_t s)
-{
-    mlp_silu_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, z, h, dh, dz);
-}
-
-// Rows gathered from the sample set by a permutation: x[b] = X[perm[off + b]].
-__global__ void mlp_gather_kernel(int nb, const int *perm, int off, const float *X, const float *Y, float *x, float *y,
-                                  const float *mean, const float *rstd, float tinv)
-{
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    const int r = perm[off + b];
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int k = 0; k < kMlpIn; ++k) x[b * kMlpIn + k] = (X[(size_t)r * kMlpIn + k] - mean[k]) * rstd[k];
-    y[b] = Y[r] * tinv;
+            for (int j = 0; j < 4; ++j) v[i][j] = 0.0f;
+        tile_mma(h1t, w2t, ty, tx, v);
+        bias(b2, v);
+        silu(v, s2);
+        tile_put(h2, h2t, ty, tx, v);
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[i][j] = 0.0f;
+        tile_mma(h2t, w3t, ty, tx, v);
+        bias(b3, v);
+        silu(v, s3);
+        tile_put(h3, nullptr, ty, tx, v);
+        __syncthreads();
+        // output, squared error, dy: four threads a row
+        {
+            const int r = t / 4, row = tile * kTrRows + r;
+            float y = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) y += h3[r * kTrS + (t & 3) * 16 + k] * w4[(t & 3) * 16 + k];
+            y += __shfl_xor_sync(0xffffffffu, y, 1);
+            y += __shfl_xor_sync(0xffffffffu, y, 2);
+            if ((t & 3) == 0) {
+                float e = 0.0f;
+                if (row < B) e = y + b4 - in.y[in.perm ? in.perm[row] : row] * in.tinv;
+                dy[r] = 2.0f * e / B;
+                err[r] = e * e;
+            }
+        }
+        __syncthreads();
+        // layer 3: dZ3 = dy w4 silu'(z3)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[i][j] = dy[ty * 4 + i] * w4[tx * 4 + j] * s3[i][j];
+        tile_put(dz, dzt, ty, tx, v);
+        if (t < 64) {
+            for (int r = 0; r < kTrRows; ++r) gw4 += dy[r] * h3[r * kTrS + t];
+        } else if (t == 64) {
+            for (int r = 0; r < kTrRows; ++r) { gb4 += dy[r]; sq += err[r]; }
+        }
+        __syncthreads();
+        tile_mma(dz, h2, ty, tx, g3);
+        if (t < 64)
+            for (int r = 0; r < kTrRows; ++r) gb += dz[r * kTrS + t];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[i][j] = 0.0f;
+        tile_mma(dzt, w3, ty, tx, v);
+        __syncthreads();
+        // layer 2
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[i][j] *= s2[i][j];
+        tile_put(dz, dzt, ty, tx, v);
+        __syncthreads();
+        tile_mma(dz, h1, ty, tx, g2);
+        if (t >= 64 && t < 128)
+            for (int r = 0; r < kTrRows; ++r) gb += dz[r * kTrS + t - 64];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[i][j] = 0.0f;
+        tile_mma(dzt, w2, ty, tx, v);
+        __syncthreads();
+        // layer 1
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[i][j] *= s1[i][j];
+        tile_put(dz, nullptr, ty, tx, v);
+        __syncthreads();
+        if (t >= 128 && t < 192)
+            for (int r = 0; r < kTrRows; ++r) gb += dz[r * kTrS + t - 128];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int e = t + q * kTrThreads;
+            if (e < kNW1)
+                for (int r = 0; r < kTrRows; ++r) g1[q] += dz[r * kTrS + e / kMlpIn] * x[r * 8 + e % kMlpIn];
+        }
+    }
+    float *o = part + (size_t)blockIdx.x * kNParam;
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+        if (t + q * kTrThreads < kNW1) o[kOffW1 + t + q * kTrThreads] = g1[q];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            o[kOffW2 + (ty * 4 + i) * 64 + tx * 4 + j] = g2[i][j];
+            o[kOffW3 + (ty * 4 + i) * 64 + tx * 4 + j] = g3[i][j];
+        }
+    if (t < 64) { o[kOffB3 + t] = gb; o[kOffW4 + t] = gw4; }
+    else if (t < 128) o[kOffB2 + t - 64] = gb;
+    else if (t < 192) o[kOffB1 + t - 128] = gb;
+    if (t == 64) {
+        o[kOffB4] = gb4;
+        loss[blockIdx.x] += sq;
+    }
 }
 
-// dy = 2 (y - t) / nb, and the squared error summed per block into loss[blockIdx.x]
-// (fixed order: warp shuffles, then the block's warps in order; the host sums
-// the block partials in order, so the reported loss does not depend on timing).
-__global__ void __launch_bounds__(256) mlp_loss_kernel(int nb, const float *y, const float *t, float *dy, float *loss)
+// Sum of the blocks' gradients (in their order, four runs of them at a time),
+// then Adam (Kingma & Ba 2015) on the parameter; or, without m, the gradient.
+__global__ void __launch_bounds__(256) mlp_adam_kernel(int nblk, const float *part, float *p, float *m, float *v, float lr,
+                                                       float b1, float b2, float eps, float c1, float c2)
 {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    float e = 0.0f;
-    if (b < nb) {
-        const float r = y[b] - t[b];
-        dy[b] = 2.0f * r / nb;
-        e = r * r;
+    __shared__ float run[4][64];
+    const int i = blockIdx.x * 64 + threadIdx.x % 64, q = threadIdx.x / 64;
+    float g = 0.0f;
+    if (i < kNParam) {
+        const int k1 = (q + 1) * nblk / 4;
+        for (int k = q * nblk / 4; k < k1; ++k) g += part[(size_t)k * kNParam + i];
     }
-    for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-    __shared__ float part[8];
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = e;
+    run[q][threadIdx.x % 64] = g;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float acc = 0.0f;
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) acc += part[i];
-        loss[blockIdx.x] += acc;
-    }
-}
-
-// Column sums of a [rows x cols] matrix (bias gradients).
-__global__ void mlp_colsum_kernel(int rows, int cols, const float *a, float *out)
-{
-    const int j = blockIdx.x;
-    float s = 0.0f;
-    for (int i = threadIdx.x; i < rows; i += blockDim.x) s += a[(size_t)i * cols + j];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    __shared__ float part[8];
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.0f;
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += part[i];
-        out[j] = t;
-    }
-}
-
-// Adam (Kingma & Ba 2015) over the flat parameter vector.
-__global__ void mlp_adam_kernel(int n, float *p, const float *gr, float *m, float *v, float lr, float b1, float b2,
-                                float eps, float c1, float c2)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = gr[i];
+    if (q != 0 || i >= kNParam) return;
+    const float gi = ((run[0][threadIdx.x] + run[1][threadIdx.x]) + run[2][threadIdx.x]) + run[3][threadIdx.x];
+    if (!m) { p[i] = gi; return; }
     const float mi = b1 * m[i] + (1.0f - b1) * gi;
     const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
     m[i] = mi;
@@ -545,21 +682,10 @@ __global__ void mlp_adam_kernel(int n, float *p, const float *gr, float *m, floa
     p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
-void mlp_train_kernels_launch_silu_cols(int rows, int cols, const float *a, float *out, cudaStream_t s)
-{
-    mlp_colsum_kernel<<<cols, 256, 0, s>>>(rows, cols, a, out);
-}
-
 // ---------------------------------------------------------------------------
 // Host side: training driver and packing of the weights into the MMA layout.
 // ---------------------------------------------------------------------------
 namespace {
-
-constexpr int kNW1 = kMlpH * kMlpIn, kNW2 = kMlpH * kMlpH, kNW3 = kMlpH * kMlpH;
-// flat parameter vector: w1 b1 w2 b2 w3 b3 w4 b4
-constexpr int kOffW1 = 0, kOffB1 = kOffW1 + kNW1, kOffW2 = kOffB1 + kMlpH, kOffB2 = kOffW2 + kNW2;
-constexpr int kOffW3 = kOffB2 + kMlpH, kOffB3 = kOffW3 + kNW3, kOffW4 = kOffB3 + kMlpH, kOffB4 = kOffW4 + kMlpH;
-constexpr int kNParam = kOffB4 + 1;
 
 struct DevBuf {
     std::vector<void *> p;
@@ -585,53 +711,17 @@ float uniform(uint64_t &x) { return (float)((splitmix(x) >> 11) * (1.0 / 9007199
 
 }  // namespace
 
-// Flat parameter vector (w1 b1 w2 b2 w3 b3 w4 b4) and the activation buffers
-// of one batch of B rows.
-struct MlpBatch {
-    float *z1, *h1, *z2, *h2, *z3, *h3, *dh, *dz, *yp, *dy;
-};
-
-// Forward pass of one batch (x: standardised inputs [B][6], yt: scaled
-// targets [B]) and the gradient of the mean squared error into gp; the batch's
-// squared error is added to loss[0 .. ceil(B / 256)).
-void mlp_forward_backward(const float *p, float *gp, const float *x, const float *yt, int B, const MlpBatch &a,
-                          float *loss, cudaStream_t s)
+// Blocks of the gradient kernel for batches of B rows on the current device, 0
+// if the device cannot run it.
+static int mlp_grad_blocks(int B)
 {
-    const int H = kMlpH;
-    // forward: z = a W^T + b (W row-major [out][in])
-    mlp_gemm(B, H, kMlpIn, x, kMlpIn, 1, p + kOffW1, 1, kMlpIn, a.z1, H, p + kOffB1, false, s);
-    mlp_silu((long long)B * H, a.z1, a.h1, nullptr, nullptr, s);
-    mlp_gemm(B, H, H, a.h1, H, 1, p + kOffW2, 1, H, a.z2, H, p + kOffB2, false, s);
-    mlp_silu((long long)B * H, a.z2, a.h2, nullptr, nullptr, s);
-    mlp_gemm(B, H, H, a.h2, H, 1, p + kOffW3, 1, H, a.z3, H, p + kOffB3, false, s);
-    mlp_silu((long long)B * H, a.z3, a.h3, nullptr, nullptr, s);
-    mlp_gemm(B, 1, H, a.h3, H, 1, p + kOffW4, 1, 1, a.yp, 1, p + kOffB4, false, s);
-    mlp_loss_kernel<<<(B + 255) / 256, 256, 0, s>>>(B, a.yp, yt, a.dy, loss);
-    // backward
-    mlp_gemm(1, H, B, a.dy, 1, 1, a.h3, H, 1, gp + kOffW4, H, nullptr, false, s);             // dW4 = dy^T h3
-    mlp_train_kernels_launch_silu_cols(B, 1, a.dy, gp + kOffB4, s);                           // db4
-    mlp_gemm(B, H, 1, a.dy, 1, 1, p + kOffW4, 1, 1, a.dh, H, nullptr, false, s);              // dH3 = dy w4
-    mlp_silu((long long)B * H, a.z3, nullptr, a.dh, a.dz, s);                                 // dZ3
-    mlp_gemm(H, H, B, a.dz, 1, H, a.h2, H, 1, gp + kOffW3, H, nullptr, false, s);             // dW3 = dZ3^T H2
-    mlp_train_kernels_launch_silu_cols(B, H, a.dz, gp + kOffB3, s);
-    mlp_gemm(B, H, H, a.dz, H, 1, p + kOffW3, H, 1, a.dh, H, nullptr, false, s);              // dH2 = dZ3 W3
-    mlp_silu((long long)B * H, a.z2, nullptr, a.dh, a.dz, s);
-    mlp_gemm(H, H, B, a.dz, 1, H, a.h1, H, 1, gp + kOffW2, H, nullptr, false, s);             // dW2
-    mlp_train_kernels_launch_silu_cols(B, H, a.dz, gp + kOffB2, s);
-    mlp_gemm(B, H, H, a.dz, H, 1, p + kOffW2, H, 1, a.dh, H, nullptr, false, s);              // dH1 = dZ2 W2
-    mlp_silu((long long)B * H, a.z1, nullptr, a.dh, a.dz, s);
-    mlp_gemm(H, kMlpIn, B, a.dz, 1, H, x, kMlpIn, 1, gp + kOffW1, kMlpIn, nullptr, false, s);  // dW1
-    mlp_train_kernels_launch_silu_cols(B, H, a.dz, gp + kOffB1, s);
-}
-
-// Device buffers of one batch of B rows (nullptr members if an allocation failed).
-static bool mlp_batch_alloc(DevBuf &db, int B, MlpBatch &a)
-{
-    const size_t bh = (size_t)B * kMlpH;
-    a.z1 = db.get<float>(bh); a.h1 = db.get<float>(bh); a.z2 = db.get<float>(bh); a.h2 = db.get<float>(bh);
-    a.z3 = db.get<float>(bh); a.h3 = db.get<float>(bh); a.dh = db.get<float>(bh); a.dz = db.get<float>(bh);
-    a.yp = db.get<float>(B); a.dy = db.get<float>(B);
-    return a.z1 && a.h1 && a.z2 && a.h2 && a.z3 && a.h3 && a.dh && a.dz && a.yp && a.dy;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kTrSmemFloats * (int)sizeof(float)) != cudaSuccess)
+        return 0;
+    return std::min((B + kTrRows - 1) / kTrRows, sms);
 }
 
 // Trains the MLP on n samples (raw features [n][6], targets [n]) with Adam and
@@ -675,50 +765,46 @@ int mlp_train(const float *X, const float *Y, long long n, int epochs, int batch
     init(kOffW3, kMlpH, kNW3);
     init(kOffW4, kMlpH, kMlpH);
     const int B = (int)std::min<long long>(batch, n);
+    const int nblk = mlp_grad_blocks(B);
+    if (nblk < 1) return (int)cudaGetLastError();
     DevBuf db;
     float *dX = db.get<float>((size_t)n * kMlpIn), *dY = db.get<float>(n);
     int *dperm = db.get<int>(n);
-    float *p = db.get<float>(kNParam), *gp = db.get<float>(kNParam), *m1 = db.get<float>(kNParam),
-          *m2 = db.get<float>(kNParam);
-    float *dmean = db.get<float>(kMlpIn), *drstd = db.get<float>(kMlpIn);
-    float *x = db.get<float>((size_t)B * kMlpIn), *yt = db.get<float>(B);
-    const int nLoss = (B + 255) / 256;
-    float *loss = db.get<float>(nLoss);
-    MlpBatch act;
-    const bool actOk = mlp_batch_alloc(db, B, act);
-    if (!dX || !dY || !dperm || !p || !gp || !m1 || !m2 || !dmean || !drstd || !x || !yt || !loss || !actOk)
-        return (int)cudaErrorMemoryAllocation;
+    // parameters, Adam moments, normalisation, the blocks' losses and gradients
+    float *p = db.get<float>(3 * (size_t)kNParam + 2 * kMlpIn + nblk + (size_t)nblk * kNParam);
+    if (!dX || !dY || !dperm || !p) return (int)cudaErrorMemoryAllocation;
+    float *m1 = p + kNParam, *m2 = m1 + kNParam, *dmean = m2 + kNParam, *drstd = dmean + kMlpIn, *loss = drstd + kMlpIn,
+          *part = loss + nblk;
     cudaMemcpyAsync(dX, X, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dY, Y, sizeof(float) * n, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(p, prm.data(), sizeof(float) * kNParam, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dmean, mean, sizeof(float) * kMlpIn, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(drstd, rstd, sizeof(float) * kMlpIn, cudaMemcpyHostToDevice, s);
-    cudaMemsetAsync(m1, 0, sizeof(float) * kNParam, s);
-    cudaMemsetAsync(m2, 0, sizeof(float) * kNParam, s);
+    cudaMemsetAsync(m1, 0, sizeof(float) * 2 * kNParam, s);
     std::vector<int> perm(n);
     for (long long i = 0; i < n; ++i) perm[i] = (int)i;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const int H = kMlpH;
     long long stepCount = 0;
-    std::vector<float> lossHost(nLoss);
     for (int ep = 0; ep < epochs; ++ep) {
+        // shuffled while the device still runs the epoch before
         for (long long i = n - 1; i > 0; --i) std::swap(perm[i], perm[splitmix(rs) % (uint64_t)(i + 1)]);
         cudaMemcpyAsync(dperm, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s);
-        cudaMemsetAsync(loss, 0, sizeof(float) * nLoss, s);
+        cudaMemsetAsync(loss, 0, sizeof(float) * nblk, s);
         for (long long off = 0; off + B <= n; off += B) {
-            mlp_gather_kernel<<<(B + 255) / 256, 256, 0, s>>>(B, dperm, (int)off, dX, dY, x, yt, dmean, drstd,
-                                                              1.0f / tscale);
-            mlp_forward_backward(p, gp, x, yt, B, act, loss, s);
+            const MlpRows rows{dX, dY, dperm + off, dmean, drstd, 1.0f / tscale};
+            mlp_grad_kernel<<<nblk, kTrThreads, kTrSmemFloats * sizeof(float), s>>>(p, rows, B, part, loss);
             ++stepCount;
             const float c1 = 1.0f - std::pow(b1, (float)stepCount), c2 = 1.0f - std::pow(b2, (float)stepCount);
-            mlp_adam_kernel<<<(kNParam + 255) / 256, 256, 0, s>>>(kNParam, p, gp, m1, m2, lr, b1, b2, eps, c1, c2);
+            mlp_adam_kernel<<<(kNParam + 63) / 64, 256, 0, s>>>(nblk, part, p, m1, m2, lr, b1, b2, eps, c1, c2);
         }
-        cudaMemcpyAsync(lossHost.data(), loss, sizeof(float) * nLoss, cudaMemcpyDeviceToHost, s);
-        cudaStreamSynchronize(s);
-        double lh = 0.0;
-        for (int i = 0; i < nLoss; ++i) lh += lossHost[i];
-        lastLoss = lh / (double)((n / B) * B);
     }
+    std::vector<float> lossHost(nblk);
+    cudaMemcpyAsync(lossHost.data(), loss, sizeof(float) * nblk, cudaMemcpyDeviceToHost, s);
+    if (cudaStreamSynchronize(s) != cudaSuccess) return (int)cudaGetLastError();
+    double lh = 0.0;
+    for (int i = 0; i < nblk; ++i) lh += lossHost[i];
+    lastLoss = lh / (double)((n / B) * B);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e;
     cudaMemcpyAsync(prm.data(), p, sizeof(float) * kNParam, cudaMemcpyDeviceToHost, s);
@@ -741,17 +827,20 @@ int mlp_loss_grad(const float *params, const float *x, const float *y, int B, fl
                   cudaStream_t s)
 {
     if (B < 1) return -1;
+    const int nLoss = mlp_grad_blocks(B);
+    if (nLoss < 1) return (int)cudaGetLastError();
     DevBuf db;
-    const int nLoss = (B + 255) / 256;
     float *p = db.get<float>(kNParam), *gp = db.get<float>(kNParam), *dx = db.get<float>((size_t)B * kMlpIn),
-          *dy = db.get<float>(B), *loss = db.get<float>(nLoss);
-    MlpBatch act;
-    if (!mlp_batch_alloc(db, B, act) || !p || !gp || !dx || !dy || !loss) return (int)cudaErrorMemoryAllocation;
+          *dy = db.get<float>(B), *loss = db.get<float>(nLoss), *part = db.get<float>((size_t)nLoss * kNParam);
+    if (!p || !gp || !dx || !dy || !loss || !part) return (int)cudaErrorMemoryAllocation;
     cudaMemcpyAsync(p, params, sizeof(float) * kNParam, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dx, x, sizeof(float) * B * kMlpIn, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dy, y, sizeof(float) * B, cudaMemcpyHostToDevice, s);
     cudaMemsetAsync(loss, 0, sizeof(float) * nLoss, s);
-    mlp_forward_backward(p, gp, dx, dy, B, act, loss, s);
+    mlp_grad_kernel<<<nLoss, kTrThreads, kTrSmemFloats * sizeof(float), s>>>(
+        p, MlpRows{dx, dy, nullptr, nullptr, nullptr, 1.0f}, B, part, loss);
+    mlp_adam_kernel<<<(kNParam + 63) / 64, 256, 0, s>>>(nLoss, part, gp, nullptr, nullptr, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f,
+                                                        1.0f);
     std::vector<float> lh(nLoss);
     cudaMemcpyAsync(grad, gp, sizeof(float) * kNParam, cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(lh.data(), loss, sizeof(float) * nLoss, cudaMemcpyDeviceToHost, s);
