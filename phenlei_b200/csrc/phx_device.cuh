@@ -200,41 +200,32 @@ struct RowPipe {
     }
 };
 
-// Factors of one face use in the sweeps: 16 values per lane of a row, in
-// 16-byte units rotated by the lane so that a warp reads them from shared
-// memory without bank conflicts.
-template <class T>
-__device__ __forceinline__ int use_unit(int k, int lane)
-{
-    return sizeof(T) == 4 ? (k + (lane >> 1)) & 3 : (k + lane) & 7;
-}
+// Factors of one face use (kUse values), in 16-byte units rotated by the lane so
+// that a warp reads them from shared memory without bank conflicts.
 __device__ __forceinline__ void put_use(float *use, int lane, const float *v)
 {
-    float4 *d = reinterpret_cast<float4 *>(use);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) d[use_unit<float>(k, lane)] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+    const int x = (lane >> 2) & 1;
+    st4(use + 4 * x, v);
+    st4(use + 4 * (1 - x), v + 4);
 }
 __device__ __forceinline__ void put_use(double *use, int lane, const double *v)
 {
-    double2 *d = reinterpret_cast<double2 *>(use);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) d[use_unit<double>(k, lane)] = make_double2(v[2 * k], v[2 * k + 1]);
+    for (int k = 0; k < 4; ++k)
+        reinterpret_cast<double2 *>(use)[(k + (lane >> 1)) & 3] = make_double2(v[2 * k], v[2 * k + 1]);
 }
-__device__ __forceinline__ void get_use(const float *row, int lane, float *v)
+__device__ __forceinline__ void get_use(const float *use, int lane, float *v)
 {
-    const float4 *d = reinterpret_cast<const float4 *>(row + lane * kUse);
+    const int x = (lane >> 2) & 1;
+    const float4 a = reinterpret_cast<const float4 *>(use)[x], b = reinterpret_cast<const float4 *>(use)[1 - x];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void get_use(const double *use, int lane, double *v)
+{
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const float4 a = d[use_unit<float>(k, lane)];
-        v[4 * k] = a.x; v[4 * k + 1] = a.y; v[4 * k + 2] = a.z; v[4 * k + 3] = a.w;
-    }
-}
-__device__ __forceinline__ void get_use(const double *row, int lane, double *v)
-{
-    const double2 *d = reinterpret_cast<const double2 *>(row + lane * kUse);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const double2 a = d[use_unit<double>(k, lane)];
+        const double2 a = reinterpret_cast<const double2 *>(use)[(k + (lane >> 1)) & 3];
         v[2 * k] = a.x; v[2 * k + 1] = a.y;
     }
 }

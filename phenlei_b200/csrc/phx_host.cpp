@@ -748,7 +748,7 @@ int make_work(phx_ctx *ctx, Work<T> &w, const std::vector<double> &limInit)
     r |= dalloc(ctx, &w.qrec, nt * kQ);
     r |= dalloc(ctx, &w.grec, nt * kG);
     r |= dalloc(ctx, &w.flux, nf * kFlux);
-    r |= dalloc(ctx, &w.coef, (size_t)ctx->nBFace * kCoef);
+    r |= dalloc(ctx, &w.coef, (size_t)ctx->nBFace * kUse);
     r |= make_rows(ctx, &w.rowf, 0, kRowNs<T, true>);
     r |= make_rows(ctx, &w.rowb, 1, kRowNs<T, false>);
     r |= dalloc(ctx, &w.crec, nc * kC);

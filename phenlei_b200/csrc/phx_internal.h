@@ -46,11 +46,11 @@ constexpr int kFlux = 16;  // face flux record: inviscid F0..4 (times area) | in
                            // spectral parts | pad | viscous F1..4 (times area; F0 is zero) | pad
 constexpr int kN = 8;      // nrec (GG-node): q node values (5), temperature node values of this
                            // iteration's state, those the gradient uses (the previous state's), pad
-constexpr int kCoef = 4;   // LU-SGS factors of a boundary face: l1 x1 x2 | viscous spectral term
-// LU-SGS factors of an interior face use, as the sweeps read them: unit normal
-// from the cell to the neighbour, area | l1 x1 x2, viscous spectral term | the
-// neighbour's u v w c2 | total enthalpy, normal velocity, (gamma - 1) / 2 |u|^2, pad
-constexpr int kUse = 16;
+// LU-SGS factors of a face use, as the sweeps read them (sweep_use): unit normal
+// from the cell to the neighbour times half the area, diagonal factor | the
+// neighbour's u v w, total enthalpy.  Whole 32-byte sectors: with 48-byte records
+// the passes that write them took 6 % longer.
+constexpr int kUse = 8;
 constexpr int kLeadF = 8;  // forward right-hand side of a cell: residual (5) | reciprocal diagonal | time step | pad
 constexpr int kLeadB = 16; // backward: residual less the forward sums (5), reciprocal diagonal, pad | boundary part (5), pad
 constexpr int kLeadT = 2;  // SA sweeps: right-hand side | reciprocal spectral radius
@@ -175,7 +175,7 @@ struct Work {
     T *qrec;        // [nTotal][kQ] working state, c2 = |gamma p / rho|, total enthalpy, limiter
     T *grec;        // [nTotal][kG] primitive gradients (ghost rows: interface ghosts only, from the halo exchange)
     T *flux;        // [nFace][kFlux] face flux times area and inviscid spectral radius term
-    T *coef;        // [nBFace][kCoef] LU-SGS factors of the boundary faces
+    T *coef;        // [nBFace][kUse] LU-SGS factors of the boundary faces' uses
     unsigned char *rowf, *rowb;   // [rows][kRowNs] LU-SGS rows of the forward and the backward sweep
     T *crec;        // [nCell][kC] residual, diagonal, spectral radii
     T *dtraw;       // [nCell] CFL * vol / spectral radius, before the ktmax clamp

@@ -389,27 +389,31 @@ void launch_gradient_limiter(const DevGrid &g, const NsConst &c, const Work<T> &
 // MXDQ_STD, :15097-15116, Jacobian.cpp:27-47).
 // ---------------------------------------------------------------------------
 
-// dq-independent part of the neighbour's MXDQ_STD term for the use (cell ->
-// neighbour, normal pointing from cell to neighbour); o[3] is the normal
-// velocity of the neighbour.
+// Roe-averaged spectral radius |vn| + c of a face (RoeAveragedVariables,
+// Flux_Inviscid.cpp:15440-15465, and GetRad) from the cell records, whose slot 6
+// is the total enthalpy: the same for both uses of the face.
 template <class T>
-__device__ __forceinline__ void lusgs_coef(const T *qc, const T *qn, T nx, T ny, T nz, T area, T gm, T *o)
+__device__ __forceinline__ T roe_radius(const T *qL, const T *qR, T nx, T ny, T nz, T gm)
 {
-    T fp[5];
-    roe_average<T>(qc, gm, qn, gm, fp);
-    const T vn = nx * fp[1] + ny * fp[2] + nz * fp[3];
-    const T rad = (fabs(vn) + sqrt(gm * fp[4] / fp[0])) * area;
-    const T c2 = fabs(gm * qn[4] / qn[0]);
-    const T cm = sqrt(c2);
-    const T cits = nx * qn[1] + ny * qn[2] + nz * qn[3];
-    const T ipnrad = -rad / tmax(T(kSmall), area);
-    const T a1 = T(0.5) * (cits + ipnrad);
-    const T a2 = T(0.5) * (cits + cm + ipnrad);
-    const T a3 = T(0.5) * (cits - cm + ipnrad);
-    o[0] = a1;
-    o[1] = (a1 + a1 - a2 - a3) / (c2 + c2);
-    o[2] = (a2 - a3) / (cm + cm);
-    o[3] = cits;
+    const T t0 = sqrt(qR[0] / qL[0]), t1 = T(1) / (T(1) + t0);
+    const T u = (qL[1] + qR[1] * t0) * t1, v = (qL[2] + qR[2] * t0) * t1, w = (qL[3] + qR[3] * t0) * t1;
+    const T hm = (qL[6] + qR[6] * t0) * t1;
+    return fabs(nx * u + ny * v + nz * w) + sqrt((gm - T(1)) * (hm - T(0.5) * (u * u + v * v + w * w)));
+}
+
+// The factors of a face use (kUse) for the sweeps: MXDQ_STD with ipn = -1
+// (Jacobian.cpp:13-86).  Its eigenvalues l1 = (vn - rad) / 2, l2 = l1 + c / 2 and
+// l3 = l1 - c / 2 make its coefficients (2 l1 - l2 - l3) / (2 c^2) and (l2 - l3) /
+// (2 c) zero and one half, so the neighbour's term is
+//   area (l1 dq - dc / 2 (1, u, h) + dh / 2 (0, n, vn)) - vspec dq
+// with dc = vn dq0 - n . dq123 and dh of the neighbour's state (delta_flux).
+template <class T>
+__device__ __forceinline__ void sweep_use(const T *qn, T nx, T ny, T nz, T area, T rad, T vspec, T *v)
+{
+    const T vn = nx * qn[1] + ny * qn[2] + nz * qn[3], ha = T(0.5) * area;
+    v[0] = ha * nx; v[1] = ha * ny; v[2] = ha * nz;
+    v[3] = ha * (vn - rad) - vspec;
+    v[4] = qn[1]; v[5] = qn[2]; v[6] = qn[3]; v[7] = qn[6];
 }
 
 // Where the sweeps' rows hold the factors of a face use (DevGrid::use), and a
@@ -426,20 +430,6 @@ __device__ __forceinline__ T *lead_at(const Work<T> &w, int slot)
 {
     unsigned char *row = (kForward ? w.rowf : w.rowb) + (size_t)(slot / kSweepSlots) * kRowNs<T, kForward>;
     return reinterpret_cast<T *>(row) + 32 * kUse + (slot % kSweepSlots) * (kForward ? kLeadF : kLeadB);
-}
-
-// The factors of a face use (kUse) for the sweeps.
-template <class T>
-__device__ __forceinline__ void sweep_use(const T *qc, const T *qn, T nx, T ny, T nz, T area, T gm, T vspec, T *v)
-{
-    T cf[4];
-    lusgs_coef<T>(qc, qn, nx, ny, nz, area, gm, cf);
-    v[0] = nx; v[1] = ny; v[2] = nz; v[3] = area;
-    v[4] = cf[0]; v[5] = cf[1]; v[6] = cf[2]; v[7] = vspec;
-    v[8] = qn[1]; v[9] = qn[2]; v[10] = qn[3]; v[11] = qn[5];
-    v[12] = qn[6]; v[13] = cf[3];
-    v[14] = T(0.5) * (gm - T(1)) * (qn[1] * qn[1] + qn[2] * qn[2] + qn[3] * qn[3]);
-    v[15] = T(0);
 }
 
 // MUSCL state of one side (boundary ghosts carry a zero gradient, so their
@@ -685,17 +675,15 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1) face_flux_ke
     fl[7] = T(0);
     st8(w.flux + (size_t)f * kFlux, fl);
     // LU-SGS factors of the left cell's and the right cell's use
+    const T rad = roe_radius<T>(qL, qR, xn, yn, zn, gm);
+    T v[kUse];
+    sweep_use<T>(qR, xn, yn, zn, area, rad, vspec, v);
     if (f < g.nBFace) {
-        T cf[4];
-        lusgs_coef<T>(qL, qR, xn, yn, zn, area, gm, cf);
-        cf[3] = vspec;
-        st4(w.coef + (size_t)f * kCoef, cf);
+        put_use(w.coef + (size_t)f * kUse, 0, v);
     } else {
         const int2 at = ld(g.use + f);
-        T v[kUse];
-        sweep_use<T>(qL, qR, xn, yn, zn, area, gm, vspec, v);
         put_use(use_at<T>(w, at.x), (at.x < 0 ? ~at.x : at.x) & 31, v);
-        sweep_use<T>(qR, qL, -xn, -yn, -zn, area, gm, vspec, v);
+        sweep_use<T>(qL, -xn, -yn, -zn, area, rad, vspec, v);
         put_use(use_at<T>(w, at.y), (at.y < 0 ? ~at.y : at.y) & 31, v);
     }
 }
@@ -861,28 +849,20 @@ __device__ __forceinline__ void ghost_dq(int kind, T xn, T yn, T zn, const T *ql
     }
 }
 
-// Delta flux of one neighbour (SolveLUSGSForward, NSSolverUnstruct.cpp:15118-15357):
-// MXDQ_STD with the use's factors u (kUse) and the neighbour's dq; the viscous
-// part for viscous runs.
+// Delta flux of one neighbour (SolveLUSGSForward, NSSolverUnstruct.cpp:15118-15357)
+// from the use's factors u (sweep_use) and the neighbour's dq; g1 = gamma - 1.
 template <class T>
-__device__ __forceinline__ void delta_flux(const T *u, T g1, int viscous, const T *dq, T *df)
+__device__ __forceinline__ void delta_flux(const T *u, T g1, const T *dq, T *df)
 {
-    const T nx = u[0], ny = u[1], nz = u[2], area = u[3], um = u[8], vm = u[9], wm = u[10], cits = u[13];
-    const T dc = cits * dq[0] - nx * dq[1] - ny * dq[2] - nz * dq[3];
-    const T c2dc = u[11] * dc;
-    T dh = -g1 * (um * dq[1] + vm * dq[2] + wm * dq[3] - dq[4]);
-    dh += u[14] * dq[0];
-    const T a = dh * u[5] + dc * u[6];
-    const T b = c2dc * u[5] + dh * u[6];
-    df[0] = (u[4] * dq[0] - a) * area;
-    df[1] = (u[4] * dq[1] - um * a + nx * b) * area;
-    df[2] = (u[4] * dq[2] - vm * a + ny * b) * area;
-    df[3] = (u[4] * dq[3] - wm * a + nz * b) * area;
-    df[4] = (u[4] * dq[4] - u[12] * a + cits * b) * area;
-    if (viscous) {
-#pragma unroll
-        for (int m = 0; m < 5; ++m) df[m] -= u[7] * dq[m];
-    }
+    const T vn = u[0] * u[4] + u[1] * u[5] + u[2] * u[6];
+    const T ek = T(0.5) * g1 * (u[4] * u[4] + u[5] * u[5] + u[6] * u[6]);
+    const T dc = vn * dq[0] - u[0] * dq[1] - u[1] * dq[2] - u[2] * dq[3];
+    const T dh = ek * dq[0] - g1 * (u[4] * dq[1] + u[5] * dq[2] + u[6] * dq[3] - dq[4]);
+    df[0] = u[3] * dq[0] - dc;
+    df[1] = u[3] * dq[1] - u[4] * dc + u[0] * dh;
+    df[2] = u[3] * dq[2] - u[5] * dc + u[1] * dh;
+    df[3] = u[3] * dq[3] - u[6] * dc + u[2] * dh;
+    df[4] = u[3] * dq[4] - u[7] * dc + vn * dh;
 }
 
 // Boundary part of the backward sweep: per cell with boundary faces the sum of
@@ -911,16 +891,12 @@ __global__ void __launch_bounds__(kThreads) sweep_ghost_kernel(DevGrid g, NsCons
         const int kind = ld(g.bkind + f), ghost = g.nCell + f;
         double fr[4];
         ld4(g.frec + (size_t)f * kF, fr);
-        const T nx = (T)fr[0], ny = (T)fr[1], nz = (T)fr[2], area = (T)fr[3];
-        T qg[8], cf[4], dq[8], df[5];
+        T qg[8], u[kUse], dq[8], df[5];
         ld8(w.qrec + (size_t)ghost * kQ, qg);
-        ld4(w.coef + (size_t)f * kCoef, cf);
+        get_use(w.coef + (size_t)f * kUse, 0, u);
         if (kind == BK_INTERFACE) ld8(w.dqghost + (size_t)f * kD, dq);
-        else ghost_dq<T>(kind, nx, ny, nz, ql, qg, gm, dl, dq);
-        const T v2 = qg[1] * qg[1] + qg[2] * qg[2] + qg[3] * qg[3];
-        const T u[kUse] = {nx, ny, nz, area, cf[0], cf[1], cf[2], cf[3], qg[1], qg[2], qg[3], qg[5], qg[6],
-                           nx * qg[1] + ny * qg[2] + nz * qg[3], T(0.5) * (gm - T(1)) * v2, T(0)};
-        delta_flux<T>(u, gm - T(1), c.viscous, dq, df);
+        else ghost_dq<T>(kind, (T)fr[0], (T)fr[1], (T)fr[2], ql, qg, gm, dl, dq);
+        delta_flux<T>(u, gm - T(1), dq, df);
 #pragma unroll
         for (int m = 0; m < 5; ++m) sum[m] += df[m];
     }
@@ -979,7 +955,7 @@ __global__ void __launch_bounds__(32) lusgs_kernel(DevGrid g, NsConst c, Work<T>
         const int4 info = reinterpret_cast<const int4 *>(row + kRowOff + 128)[slot];
         const T *lead = reinterpret_cast<const T *>(row + kLeadOff) + slot * kLead;
         T u[kUse];
-        get_use(reinterpret_cast<const T *>(row), t, u);
+        get_use(reinterpret_cast<const T *>(row) + t * kUse, t, u);
         if (en < 0) {
             const T *a = loc + ~en * 8;
             T b[4];
@@ -1005,7 +981,7 @@ __global__ void __launch_bounds__(32) lusgs_kernel(DevGrid g, NsConst c, Work<T>
             } while (!__all_sync(0xffffffffu, ready));
         }
         T df[5];
-        delta_flux<T>(u, g1, viscous, v, df);
+        delta_flux<T>(u, g1, v, df);
         // the row after next, while this row's sum is formed
         entry(reinterpret_cast<const int *>(row + kRowOff), en, v);
         // sum in the cell's face order, on the cell's first lane; the backward

@@ -481,52 +481,4 @@ __device__ __forceinline__ T venfun(T x, T y, T eps)
     return (x2 + eps + T(2) * xy) / (x2 + T(2) * y2 + xy + eps);
 }
 
-// RoeAveragedVariables (API/Physics/src/Flux_Inviscid.cpp:15440-15465).
-template <class T>
-__device__ __forceinline__ void roe_average(const T *a, T ga, const T *b, T gb, T *o)
-{
-    T hL = ga / (ga - T(1)) * a[4] / a[0] + T(0.5) * (a[1] * a[1] + a[2] * a[2] + a[3] * a[3]);
-    T hR = gb / (gb - T(1)) * b[4] / b[0] + T(0.5) * (b[1] * b[1] + b[2] * b[2] + b[3] * b[3]);
-    T t0 = sqrt(b[0] / a[0]);
-    T t1 = T(1) / (T(1) + t0);
-    o[0] = sqrt(b[0] * a[0]);
-    o[1] = (a[1] + b[1] * t0) * t1;
-    o[2] = (a[2] + b[2] * t0) * t1;
-    o[3] = (a[3] + b[3] * t0) * t1;
-    T hm = (hL + hR * t0) * t1;
-    o[4] = o[0] * (hm - T(0.5) * (o[1] * o[1] + o[2] * o[2] + o[3] * o[3])) * (ga - T(1)) / ga;
-}
-
-// MXDQ_STD with ipn = -1 (API/Physics/src/Jacobian.cpp:13-86) and
-// PerfectGas::ComputeTotalEnthalpyAndDH (API/Physics/src/PerfectGas.cpp:368-395):
-// the split flux-Jacobian product used by the LU-SGS sweeps.
-template <class T>
-__device__ __forceinline__ void mxdq(const T *prim, T nx, T ny, T nz, T area, T gama, const T *dq, T *f, T radius)
-{
-    T rm = prim[0], um = prim[1], vm = prim[2], wm = prim[3], pm = prim[4];
-    T c2 = fabs(gama * pm / rm);
-    T cm = sqrt(c2);
-    T cits = nx * um + ny * vm + nz * wm;
-    T ipnrad = -radius / tmax(T(kSmall), area);
-    T l1 = T(0.5) * (cits + ipnrad);
-    T l2 = T(0.5) * (cits + cm + ipnrad);
-    T l3 = T(0.5) * (cits - cm + ipnrad);
-    T x1 = (l1 + l1 - l2 - l3) / (c2 + c2);
-    T x2 = (l2 - l3) / (cm + cm);
-    T dc = cits * dq[0] - nx * dq[1] - ny * dq[2] - nz * dq[3];
-    T c2dc = c2 * dc;
-    T v2 = um * um + vm * vm + wm * wm;
-    T g1 = gama - T(1);
-    T dh = -g1 * (um * dq[1] + vm * dq[2] + wm * dq[3] - dq[4]);
-    dh += T(0.5) * g1 * v2 * dq[0];
-    T hm = (gama / g1) * (pm / rm) + T(0.5) * v2;
-    T a = dh * x1 + dc * x2;
-    T b = c2dc * x1 + dh * x2;
-    f[0] = (l1 * dq[0] - a) * area;
-    f[1] = (l1 * dq[1] - um * a + nx * b) * area;
-    f[2] = (l1 * dq[2] - vm * a + ny * b) * area;
-    f[3] = (l1 * dq[3] - wm * a + nz * b) * area;
-    f[4] = (l1 * dq[4] - hm * a + cits * b) * area;
-}
-
 }  // namespace phx
