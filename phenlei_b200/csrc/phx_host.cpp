@@ -747,6 +747,8 @@ int make_work(phx_ctx *ctx, Work<T> &w, const std::vector<double> &limInit)
     int r = 0;
     r |= dalloc(ctx, &w.qrec, nt * kQ);
     r |= dalloc(ctx, &w.grec, nt * kG);
+    r |= dalloc(ctx, &w.fnrm, nf * kNrm);
+    r |= dalloc(ctx, &w.fgeo, nf * (ctx->prm.viscousType ? kGeo<true> : kGeo<false>));
     r |= dalloc(ctx, &w.flux, nf * kFlux);
     r |= dalloc(ctx, &w.coef, (size_t)ctx->nBFace * kUse);
     r |= make_rows(ctx, &w.rowf, 0, kRowNs<T, true>);
@@ -768,6 +770,8 @@ int make_work(phx_ctx *ctx, Work<T> &w, const std::vector<double> &limInit)
     PHX_CUDA(ctx, cudaMemset(w.dqghost, 0, sizeof(T) * (size_t)ctx->nBFace * kD));   // until the first exchange
     PHX_CUDA(ctx, cudaMemset(w.grec, 0, sizeof(T) * nt * kG));
     PHX_CUDA(ctx, cudaMemset(w.crec, 0, sizeof(T) * nc * kC));
+    launch_face_geometry<T>(ctx->g, ctx->nc, w, ctx->stream);
+    PHX_CUDA(ctx, cudaGetLastError());
     return PHX_OK;
 }
 
@@ -1070,10 +1074,15 @@ int phx_ctx_create(const phx_grid_desc *gd, const phx_params *prm, phx_ctx **out
         volpow[i] = std::pow(std::pow(ctx->geom[10][ord[i]], 1.0 / 3.0), 3.0);
     }
     std::vector<int> sc2f_off(nc + 1, 0), sc2f(c2f.size());
+    std::vector<int2> sc2x(c2f.size());
     for (int i = 0; i < nc; ++i) sc2f_off[i + 1] = sc2f_off[i] + (c2f_off[ord[i] + 1] - c2f_off[ord[i]]);
     for (int i = 0; i < nc; ++i) {
         const int c = ord[i];
-        for (int j = c2f_off[c], k = sc2f_off[i]; j < c2f_off[c + 1]; ++j, ++k) sc2f[k] = fpos[c2f[j]];
+        for (int j = c2f_off[c], k = sc2f_off[i]; j < c2f_off[c + 1]; ++j, ++k) {
+            const int f = fpos[c2f[j]];
+            sc2f[k] = f;
+            sc2x[k] = lr[f].x == i ? make_int2(f, lr[f].y) : make_int2(~f, lr[f].x);
+        }
     }
 
     // constants
@@ -1143,6 +1152,7 @@ int phx_ctx_create(const phx_grid_desc *gd, const phx_params *prm, phx_ctx **out
     rc |= upload(ctx, &g.volpow, volpow);
     rc |= upload(ctx, &g.c2f_off, sc2f_off);
     rc |= upload(ctx, &g.c2f, sc2f);
+    rc |= upload(ctx, &g.c2x, sc2x);
     rc |= upload(ctx, &g.orig, origv);
     rc |= upload(ctx, &g.bkind, bkind);
     rc |= upload(ctx, &g.btype, btype);
@@ -1749,6 +1759,9 @@ int phx_swap_geometry(phx_ctx *ctx, int64_t n, const int32_t *bfaces, const doub
         for (int fs = 0; fs < nf; ++fs) vflag[fs] = vref[ctx->forder[fs]];
         PHX_CUDA(ctx, cudaMemcpy(const_cast<uint8_t *>(ctx->g.vflag), vflag.data(), nf, cudaMemcpyHostToDevice));
     }
+    if (ctx->mixed) launch_face_geometry<float>(ctx->g, ctx->nc, ctx->w32, ctx->stream);
+    else launch_face_geometry<double>(ctx->g, ctx->nc, ctx->w64, ctx->stream);
+    if (const int rc = check_launch(ctx)) return rc;
     if (avg_vol > 0.0) {
         // the Venkatakrishnan threshold scales with the average cell volume of all zones
         const double K = prm->venkatCoeff;

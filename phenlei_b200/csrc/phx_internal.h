@@ -42,8 +42,19 @@ constexpr int kC = 8;      // crec: res0..4 | 1 / LU-SGS diagonal (unclamped dt)
 constexpr int kD = 8;      // dqrec / dflux: 5 values | pad
 constexpr int kF = 8;      // frec (FP64): nx ny nz area xfc yfc zfc | least-squares face weight
 constexpr int kX = 4;      // xrec (FP64): xcc ycc zcc vol
-constexpr int kFlux = 16;  // face flux record: inviscid F0..4 (times area) | inviscid and viscous
-                           // spectral parts | pad | viscous F1..4 (times area; F0 is zero) | pad
+constexpr int kFlux = 12;  // face flux record: inviscid F0..4 (times area) | inviscid and viscous spectral parts |
+                           // viscous F1..4 (times area; F0 is zero) | pad
+// Face geometry in the working precision, formed once in FP64 from the metrics
+// (face_geometry_kernel).  fnrm: unit normal times area (least squares: vector
+// from the left to the right centre, weight).  fgeo: unit normal, area | face
+// centre less left centre, left weight of the face gradient | less right centre,
+// A | for viscous runs: left offset, B | right offset, centre distance along the
+// normal.  A and B are the weights of the left and right difference to the face
+// value in the normal derivative, the offsets lead from a centre to its foot on
+// the normal line (zero where a face has no such term).
+constexpr int kNrm = 4;
+template <bool kVisc>
+constexpr int kGeo = kVisc ? 20 : 12;
 constexpr int kN = 8;      // nrec (GG-node): q node values (5), temperature node values of this
                            // iteration's state, those the gradient uses (the previous state's), pad
 // LU-SGS factors of a face use, as the sweeps read them (sweep_use): unit normal
@@ -109,6 +120,7 @@ struct DevGrid {
     // decided on the host
     const uint8_t *vflag;
     const int *c2f_off, *c2f;    // faces of each cell, ordered by the reference face number
+    const int2 *c2x;             // and alike {face, ~ it where the cell is the right cell; cell or ghost behind it}
     const int *orig;             // [nTotal] reference number of each cell (ghost: nCell + reference face)
     const int32_t *bkind;        // [nBFace] BcKind
     const int32_t *btype;        // [nBFace] bcType
@@ -173,6 +185,7 @@ struct NsConst {
 template <class T>
 struct Work {
     T *qrec;        // [nTotal][kQ] working state, c2 = |gamma p / rho|, total enthalpy, limiter
+    T *fnrm, *fgeo; // [nFace][kNrm], [nFace][kGeo] face geometry
     T *grec;        // [nTotal][kG] primitive gradients (ghost rows: interface ghosts only, from the halo exchange)
     T *flux;        // [nFace][kFlux] face flux times area and inviscid spectral radius term
     T *coef;        // [nBFace][kUse] LU-SGS factors of the boundary faces' uses
@@ -210,6 +223,9 @@ struct Reduce {
 };
 
 // Kernel launchers (phx_kernels.cu).
+// Face geometry in the working precision from the FP64 metrics.
+template <class T>
+void launch_face_geometry(const DevGrid &g, const NsConst &c, const Work<T> &w, cudaStream_t s);
 template <class T>
 void launch_boundary(const DevGrid &g, const NsConst &c, double *q64, const Work<T> &w, cudaStream_t s);
 template <class T>

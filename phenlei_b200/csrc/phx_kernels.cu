@@ -125,6 +125,68 @@ void launch_sync_qrec(const DevGrid &g, const NsConst &c, const double *q64, con
 }
 
 // ---------------------------------------------------------------------------
+// Face geometry for the working precision (layout: kNrm, kGeo), in FP64 from the
+// metrics: FaceWeight (Geo_UnstructGrid.cpp:2420-2478) and the geometric part of
+// ComputeVisflux (NSSolverUnstruct.cpp:13147-13236).  Interface faces are
+// interior faces (FaceWeight, Geo_UnstructGrid.cpp:2475).  Formed in every pass
+// before, it took three square roots, five divisions and most conversions of the
+// mixed face pass, and 128 bytes of FP64 metrics a face.
+// ---------------------------------------------------------------------------
+template <class T>
+__global__ void __launch_bounds__(kThreads) face_geometry_kernel(DevGrid g, NsConst c, Work<T> w)
+{
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= g.nFace) return;
+    const int2 lr = ld(g.lr + f);
+    double fr[8], xl[4], xr[4];
+    ld8(g.frec + (size_t)f * kF, fr);
+    ld4(g.xrec + (size_t)lr.x * kX, xl);
+    ld4(g.xrec + (size_t)lr.y * kX, xr);
+    T *nrm = w.fnrm + (size_t)f * kNrm;
+    for (int k = 0; k < 3; ++k) nrm[k] = c.gradient == 1 ? (T)(xr[k] - xl[k]) : (T)(fr[k] * fr[3]);
+    nrm[3] = (T)fr[7];
+    T *o = w.fgeo + (size_t)f * (c.viscous ? kGeo<true> : kGeo<false>);
+    double dl[3], dr[3];
+    for (int k = 0; k < 3; ++k) {
+        dl[k] = fr[4 + k] - xl[k];
+        dr[k] = fr[4 + k] - xr[k];
+        o[k] = (T)fr[k];
+        o[4 + k] = (T)dl[k];
+        o[8 + k] = (T)dr[k];
+    }
+    o[3] = (T)fr[3];
+    o[7] = T(1);
+    o[11] = T(0);
+    if (!c.viscous) return;
+    const bool bnd = f < g.nBFace && g.bkind[f] != BK_INTERFACE;
+    const double d1 = sqrt(dl[0] * dl[0] + dl[1] * dl[1] + dl[2] * dl[2]);
+    const double d2 = sqrt(dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2]);
+    if (!bnd) o[7] = (T)(d2 / (d1 + d2 + kSmall));
+    const double dL = -(fr[0] * dl[0] + fr[1] * dl[1] + fr[2] * dl[2]);
+    const double dR = -(fr[0] * dr[0] + fr[1] * dr[1] + fr[2] * dr[2]);
+    const int vf = g.vflag[f];
+    double A = 0.0, B = 0.0;
+    if (vf & 2) {
+        const double wl = bnd ? 1.0 : dL * dL / (dL * dL + dR * dR);
+        A = wl / dL;
+        B = (1.0 - wl) / dR;
+    }
+    o[11] = (T)A;
+    for (int k = 0; k < 3; ++k) {
+        o[12 + k] = vf & 1 ? (T)(fr[k] * dL + dl[k]) : T(0);
+        o[16 + k] = vf & 1 ? (T)(fr[k] * dR + dr[k]) : T(0);
+    }
+    o[15] = (T)B;
+    o[19] = (T)fabs(fr[0] * (xr[0] - xl[0]) + fr[1] * (xr[1] - xl[1]) + fr[2] * (xr[2] - xl[2]));
+}
+
+template <class T>
+void launch_face_geometry(const DevGrid &g, const NsConst &c, const Work<T> &w, cudaStream_t s)
+{
+    face_geometry_kernel<T><<<(g.nFace + kThreads - 1) / kThreads, kThreads, 0, s>>>(g, c, w);
+}
+
+// ---------------------------------------------------------------------------
 // Gradient + limiter, fused per cell:
 //  Green-Gauss cell gradient (UnstructGrid::CompGradientGGCell,
 //  Geo_UnstructGrid.cpp:3220-3284) or least-squares gradient
@@ -204,20 +266,19 @@ __global__ void __launch_bounds__(kThreads) gradient_limiter_kernel(DevGrid g, N
 #pragma unroll
     for (int k = 0; k < 5; ++k) vc[k] = qc[k];
     if (kTemp) vc[NV - 1] = temperature(qc, coef);
-    double xc[4];
-    ld4(g.xrec + (size_t)cell * kX, xc);
+    const T vol = (T)ld(g.xrec + (size_t)cell * kX + 3);
     T gx[NV], gy[NV], gz[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) gx[k] = gy[k] = gz[k] = T(0);
     T rmin = qc[0], rmax = qc[0], pmin = qc[4], pmax = qc[4];
     const int j0 = g.c2f_off[cell], j1 = g.c2f_off[cell + 1];
     for (int j = j0; j < j1; ++j) {
-        const int f = ld(g.c2f + j);
-        const int2 lr = ld(g.lr + f);
-        const bool isLeft = (lr.x == cell);
-        const int nb = isLeft ? lr.y : lr.x;
-        T qn[8];
-        ld8(w.qrec + (size_t)nb * kQ, qn);
+        const int2 e = ld(g.c2x + j);
+        const bool isLeft = e.x >= 0;
+        const int f = isLeft ? e.x : ~e.x;
+        T qn[8], nr[4];
+        ld8(w.qrec + (size_t)e.y * kQ, qn);
+        ld4(w.fnrm + (size_t)f * kNrm, nr);
         T vn[NV];
 #pragma unroll
         for (int k = 0; k < 5; ++k) vn[k] = qn[k];
@@ -225,22 +286,13 @@ __global__ void __launch_bounds__(kThreads) gradient_limiter_kernel(DevGrid g, N
         if (kLsq) {
             // (q[re] - q[le]) (x[re] - x[le]) iwt in the face's own orientation,
             // added to both sides
-            double xn[4];
-            ld4(g.xrec + (size_t)nb * kX, xn);
-            const double iw = ld(g.frec + (size_t)f * kF + 7);
-            const T dx = (T)(isLeft ? xn[0] - xc[0] : xc[0] - xn[0]);
-            const T dy = (T)(isLeft ? xn[1] - xc[1] : xc[1] - xn[1]);
-            const T dz = (T)(isLeft ? xn[2] - xc[2] : xc[2] - xn[2]);
 #pragma unroll
             for (int k = 0; k < NV; ++k) {
-                const T dq = (T)iw * (isLeft ? vn[k] - vc[k] : vc[k] - vn[k]);
-                gx[k] += dq * dx; gy[k] += dq * dy; gz[k] += dq * dz;
+                const T dq = nr[3] * (isLeft ? vn[k] - vc[k] : vc[k] - vn[k]);
+                gx[k] += dq * nr[0]; gy[k] += dq * nr[1]; gz[k] += dq * nr[2];
             }
         } else {
-            double fr[4];
-            ld4(g.frec + (size_t)f * kF, fr);
-            const double a = fr[3];
-            const T nx = (T)(fr[0] * a), ny = (T)(fr[1] * a), nz = (T)(fr[2] * a);
+            const T nx = nr[0], ny = nr[1], nz = nr[2];
             T qf[NV];
 #pragma unroll
             for (int k = 0; k < NV; ++k) qf[k] = T(0.5) * (isLeft ? (vc[k] + vn[k]) : (vn[k] + vc[k]));
@@ -285,11 +337,10 @@ __global__ void __launch_bounds__(kThreads) gradient_limiter_kernel(DevGrid g, N
             gz[k] = ixz * tx + iyz * ty + izz * tz;
         }
     } else if (kGrad == 2) {
-        const T vol = (T)xc[3];
 #pragma unroll
         for (int k = 0; k < NV; ++k) { gx[k] /= vol; gy[k] /= vol; gz[k] /= vol; }
     } else {
-        const T ovol = T(1) / (T)xc[3];
+        const T ovol = T(1) / vol;
 #pragma unroll
         for (int k = 0; k < NV; ++k) { gx[k] *= ovol; gy[k] *= ovol; gz[k] *= ovol; }
     }
@@ -319,14 +370,16 @@ __global__ void __launch_bounds__(kThreads) gradient_limiter_kernel(DevGrid g, N
         const T dminp = pmin - qc[4], dmaxp = pmax - qc[4];
         const T small = (T)kSmall;
         for (int j = j0; j < j1; ++j) {
-            const int f = ld(g.c2f + j);
-            double fn[4], fc[4];
-            ld4(g.frec + (size_t)f * kF, fn);
-            ld4(g.frec + (size_t)f * kF + 4, fc);
-            const T dx = (T)(fc[0] - xc[0]), dy = (T)(fc[1] - xc[1]), dz = (T)(fc[2] - xc[2]);
+            const int e = ld(&g.c2x[j].x);
+            const bool isLeft = e >= 0;
+            const T *geo = w.fgeo + (size_t)(isLeft ? e : ~e) * kGeo<kTemp>;
+            T fn[4], dc[4];
+            ld4(geo, fn);
+            ld4(geo + (isLeft ? 4 : 8), dc);
+            const T dx = dc[0], dy = dc[1], dz = dc[2];
             const T ds = sqrt(dx * dx + dy * dy + dz * dz);
-            const T nd = (T)fn[0] * dx + (T)fn[1] * dy + (T)fn[2] * dz;
-            const T dot = (ld(g.lr + f).x == cell ? nd : -nd) / (ds + small);
+            const T nd = fn[0] * dx + fn[1] * dy + fn[2] * dz;
+            const T dot = (isLeft ? nd : -nd) / (ds + small);
             if (dot < T(0)) { lim = T(0); continue; }
             T d = gx[0] * dx + gy[0] * dy + gz[0] * dz;
             if (d > dmaxr) lim = tmin(lim, dmaxr / (d + small));
@@ -344,10 +397,10 @@ __global__ void __launch_bounds__(kThreads) gradient_limiter_kernel(DevGrid g, N
         const T dminp = pmin - qc[4], dmaxp = pmax - qc[4];
         const T small = (T)kSmall;
         for (int j = j0; j < j1; ++j) {
-            const int f = ld(g.c2f + j);
-            double fc[4];
-            ld4(g.frec + (size_t)f * kF + 4, fc);
-            const T dx = (T)(fc[0] - xc[0]), dy = (T)(fc[1] - xc[1]), dz = (T)(fc[2] - xc[2]);
+            const int e = ld(&g.c2x[j].x);
+            T dc[4];
+            ld4(w.fgeo + (size_t)(e >= 0 ? e : ~e) * kGeo<kTemp> + (e >= 0 ? 4 : 8), dc);
+            const T dx = dc[0], dy = dc[1], dz = dc[2];
             T d = gx[0] * dx + gy[0] * dy + gz[0] * dz;
             if (d > small) lim = tmin(lim, venfun(dmaxr, d, er));
             else if (d < -small) lim = tmin(lim, venfun(dminr, d, er));
@@ -432,206 +485,129 @@ __device__ __forceinline__ T *lead_at(const Work<T> &w, int slot)
     return reinterpret_cast<T *>(row) + 32 * kUse + (slot % kSweepSlots) * (kForward ? kLeadF : kLeadB);
 }
 
-// MUSCL state of one side (boundary ghosts carry a zero gradient, so their
-// state is used as is; an interface ghost has the neighbouring zone's
-// gradient, limiter and centre, and is reconstructed like a cell).
-template <class T>
-__device__ __forceinline__ void reconstruct(const DevGrid &g, const Work<T> &w, int cell, const double *fc, T lim,
-                                            const T *qs, T *qo, bool interfaceGhost = false)
+// One side of a face: the MUSCL state qo from the cell state qs and the cell's
+// gradient (kept where its density or pressure is not positive), and for viscous
+// runs, added to what the other side gave, the face gradient of u, v, w (weight
+// wt) and the side's velocity and temperature at the foot of the normal line
+// (offset x).  gp: the gradient record to use, null for none; recon: whether this
+// side is reconstructed (boundary ghosts are used as they are; an interface ghost
+// has the neighbouring zone's gradient, limiter and centre).
+template <class T, bool kVisc>
+__device__ __forceinline__ void face_side(const T *gp, bool recon, T lim, const T *d, const T *qs, T *qo, T wt, const T *x,
+                                          T *F, T *foot, T &tfoot)
 {
 #pragma unroll
     for (int k = 0; k < 5; ++k) qo[k] = qs[k];
-    if (cell >= g.nCell && !interfaceGhost) return;
-    double xc[4];
-    ld4(g.xrec + (size_t)cell * kX, xc);
-    const T dx = (T)(fc[0] - xc[0]), dy = (T)(fc[1] - xc[1]), dz = (T)(fc[2] - xc[2]);
-    T gr[16];
-    const T *gp = w.grec + (size_t)cell * kG;
-    ld8(gp, gr);
-    ld8(gp + 8, gr + 8);
-    T tr[5];
+    if (kVisc) {
 #pragma unroll
-    for (int k = 0; k < 5; ++k) tr[k] = qs[k] + lim * (gr[3 * k] * dx + gr[3 * k + 1] * dy + gr[3 * k + 2] * dz);
-    if (tr[0] > T(0) && tr[4] > T(0)) {
-#pragma unroll
-        for (int k = 0; k < 5; ++k) qo[k] = tr[k];
+        for (int k = 0; k < 3; ++k) foot[k] = qs[k + 1];
     }
-}
-
-// Gradients of u, v, w (9 values) and of the temperature (3) of one side of
-// a face; a boundary ghost has the owner's gradient (least squares, GG-node)
-// or none (GG-cell), as the reference's gradient routines leave them; an
-// interface ghost has the neighbouring zone's.
-template <class T>
-__device__ __forceinline__ void side_gradients(const DevGrid &g, const NsConst &c, const Work<T> &w, int cell,
-                                               int owner, T *gv, T *gt, bool interfaceGhost = false)
-{
-    const int src = (cell < g.nCell || interfaceGhost) ? cell : (c.gradient != 0 ? owner : -1);
-    if (src < 0) {
-#pragma unroll
-        for (int k = 0; k < 9; ++k) gv[k] = T(0);
-        gt[0] = gt[1] = gt[2] = T(0);
-        return;
-    }
-    const T *gp = w.grec + (size_t)src * kG;
+    if (!gp) return;
     T a[16];
     ld8(gp, a);
     ld8(gp + 8, a + 8);
+    if (recon) {
+        T tr[5];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) gv[k] = a[3 + k];
-    T b[4];
-    ld4(gp + 16, b);
-    gt[0] = b[0]; gt[1] = b[1]; gt[2] = b[2];
-}
-
-// Viscous flux of one face times the area, F1..F4 (F0 is zero), and the
-// face's viscous spectral-radius term, which is also the LU-SGS viscous
-// factor of both face uses (SpectrumRadiusViscous method 2,
-// NSSolverUnstruct.cpp:5930-5960; SolveLUSGSForward :15339-15357).
-// FaceWeight (Geo_UnstructGrid.cpp:2420-2478), GetVisFaceValue
-// (NSSolverUnstruct.cpp:7126-7375, static adiabatic walls) and ComputeVisflux
-// (:12977-13378, perfect gas).  Geometry is formed in FP64.
-template <class T>
-__device__ __forceinline__ void viscous_face(const DevGrid &g, const NsConst &c, const Work<T> &w, int f, int le,
-                                             int re, const double *fr, const T *qL, const T *qR, T *fv, T &vspec)
-{
-    // interface faces are interior faces here (FaceWeight, Geo_UnstructGrid.cpp:2475;
-    // GetVisFaceValue and ComputeVisflux, NSSolverUnstruct.cpp:7292, :13261)
-    const bool itf = f < g.nBFace && g.bkind[f] == BK_INTERFACE;
-    const bool bnd = f < g.nBFace && !itf;
-    const bool wall = bnd && g.bkind[f] == BK_WALL;
-    double xl[4], xr[4];
-    ld4(g.xrec + (size_t)le * kX, xl);
-    ld4(g.xrec + (size_t)re * kX, xr);
-    const double nxs = fr[0], nys = fr[1], nzs = fr[2], area = fr[3];
-    const T coef = (T)c.coefState, S = (T)c.tsuth;
-    const T tl0 = temperature(qL, coef), tr0 = temperature(qR, coef);
-    const T mul = T(0.5) * (sutherland(tl0, S) + sutherland(tr0, S));
-    const T mut = w.trec ? T(0.5) * (w.trec[(size_t)le * kTr + 1] + w.trec[(size_t)re * kTr + 1]) : T(0);
-    // spectral radius / LU-SGS viscous factor
-    {
-        const double ds = fabs(nxs * (xr[0] - xl[0]) + nys * (xr[1] - xl[1]) + nzs * (xr[2] - xl[2]));
-        const T rho = T(0.5) * (qL[0] + qR[0]);
-        T vs = T(2) * (mul + mut) / (rho * (T)ds * (T)c.reynolds + (T)kSmall);
-        vs *= T(0.5) * (T)area;
-        vspec = vs;
-    }
-    // FaceWeight
-    double dwl = 1.0, dwr = 0.0;
-    if (!bnd) {
-        const double ax = fr[4] - xl[0], ay = fr[5] - xl[1], az = fr[6] - xl[2];
-        const double bx = fr[4] - xr[0], by = fr[5] - xr[1], bz = fr[6] - xr[2];
-        const double d1 = sqrt(ax * ax + ay * ay + az * az), d2 = sqrt(bx * bx + by * by + bz * bz);
-        const double dl = 1.0 / (d1 + d2 + kSmall);
-        dwl = d2 * dl;
-        dwr = d1 * dl;
-    }
-    // tangents
-    double t1x, t1y, t1z;
-    if (fabs(nxs) > kSmall) { t1x = nys; t1y = -nxs; t1z = 0.0; }
-    else if (fabs(nys) > kSmall) { t1x = -nys; t1y = nxs; t1z = 0.0; }
-    else if (fabs(nzs) > kSmall) { t1x = 0.0; t1y = -nzs; t1z = nys; }
-    else { fv[0] = fv[1] = fv[2] = fv[3] = T(0); return; }
-    const double on = 1.0 / sqrt(t1x * t1x + t1y * t1y + t1z * t1z);
-    t1x *= on; t1y *= on; t1z *= on;
-    const double t2x = nys * t1z - nzs * t1y, t2y = nzs * t1x - nxs * t1z, t2z = nxs * t1y - nys * t1x;
-    const double dxL = xl[0] - fr[4], dyL = xl[1] - fr[5], dzL = xl[2] - fr[6];
-    const double dxR = xr[0] - fr[4], dyR = xr[1] - fr[5], dzR = xr[2] - fr[6];
-    const double dL = nxs * dxL + nys * dyL + nzs * dzL;
-    const double dR = nxs * dxR + nys * dyR + nzs * dzR;
-    const int vf = g.vflag[f];
-    T gvl[9], gtl[3], gvr[9], gtr[3];
-    side_gradients<T>(g, c, w, le, le, gvl, gtl);
-    side_gradients<T>(g, c, w, re, le, gvr, gtr, itf);
-    T f1[3] = {qL[1], qL[2], qL[3]}, f2[3] = {qR[1], qR[2], qR[3]};
-    T tL = tl0, tR = tr0;
-    T fm[3];
+        for (int k = 0; k < 5; ++k) tr[k] = qs[k] + lim * (a[3 * k] * d[0] + a[3 * k + 1] * d[1] + a[3 * k + 2] * d[2]);
+        if (tr[0] > T(0) && tr[4] > T(0)) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) fm[k] = T(0.5) * (f1[k] + f2[k]);
-    const T tmf = T(0.5) * (tl0 + tr0);
-    T tM = tmf;
-    if (vf & 1) {
-        const T xnl = (T)(nxs * dL - dxL), ynl = (T)(nys * dL - dyL), znl = (T)(nzs * dL - dzL);
-        const T xnr = (T)(nxs * dR - dxR), ynr = (T)(nys * dR - dyR), znr = (T)(nzs * dR - dzR);
+            for (int k = 0; k < 5; ++k) qo[k] = tr[k];
+        }
+    }
+    if (kVisc) {
+        T b[4];
+        ld4(gp + 16, b);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            f1[k] += gvl[3 * k] * xnl + gvl[3 * k + 1] * ynl + gvl[3 * k + 2] * znl;
-            f2[k] += gvr[3 * k] * xnr + gvr[3 * k + 1] * ynr + gvr[3 * k + 2] * znr;
+            const T *gk = a + 3 * (k + 1);
+            foot[k] += gk[0] * x[0] + gk[1] * x[1] + gk[2] * x[2];
+#pragma unroll
+            for (int m = 0; m < 3; ++m) F[3 * k + m] += wt * gk[m];
         }
-        tL += gtl[0] * xnl + gtl[1] * ynl + gtl[2] * znl;
-        tR += gtr[0] * xnr + gtr[1] * ynr + gtr[2] * znr;
-        if (tL < (T)kSmall) tL = tl0;
-        if (tR < (T)kSmall) tR = tr0;
-        // face values of GetVisFaceValue: the mean, no-slip at walls
-#pragma unroll
-        for (int k = 0; k < 3; ++k) fm[k] = wall ? T(0) : T(0.5) * (qL[k + 1] + qR[k + 1]);
-        tM = tmf;
+        const T t0 = tfoot;
+        tfoot += b[0] * x[0] + b[1] * x[1] + b[2] * x[2];
+        if (tfoot < (T)kSmall) tfoot = t0;
     }
-    T dfdn[3] = {0, 0, 0}, dtdn = T(0);
-    if (vf & 2) {
-        const T dLt = (T)dL, dRt = (T)dR;
-        T wL = dLt * dLt / (dLt * dLt + dRt * dRt);
-        T wR = T(1) - wL;
-        if (bnd) { wL = T(1); wR = T(0); }
-#pragma unroll
-        for (int k = 0; k < 3; ++k) dfdn[k] = wL * ((f1[k] - fm[k]) / dLt) + wR * ((f2[k] - fm[k]) / dRt);
-        dtdn = ((tL - tM) / dLt) * wL + ((tR - tM) / dRt) * wR;
-    }
-    T gx[3], gy[3], gz[3];
-    const T wl = (T)dwl, wr = (T)dwr;
-    const T n1 = (T)nxs, n2 = (T)nys, n3 = (T)nzs;
-    const T a1 = (T)t1x, a2 = (T)t1y, a3 = (T)t1z, b1 = (T)t2x, b2 = (T)t2y, b3 = (T)t2z;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const T fx = wl * gvl[3 * k] + wr * gvr[3 * k];
-        const T fy = wl * gvl[3 * k + 1] + wr * gvr[3 * k + 1];
-        const T fz = wl * gvl[3 * k + 2] + wr * gvr[3 * k + 2];
-        const T d1 = a1 * fx + a2 * fy + a3 * fz;
-        const T d2 = b1 * fx + b2 * fy + b3 * fz;
-        gx[k] = n1 * dfdn[k] + a1 * d1 + b1 * d2;
-        gy[k] = n2 * dfdn[k] + a2 * d1 + b2 * d2;
-        gz[k] = n3 * dfdn[k] + a3 * d1 + b3 * d2;
-    }
-    const T kcp = (mul * (T)c.oPrl + mut * (T)c.oPrt) * (T)c.cp;
-    const T qn = kcp * dtdn;
-    const T div = T(2.0 / 3.0) * (gx[0] + gy[1] + gz[2]);
-    const T vis = mul + mut;
-    const T txx = vis * (T(2) * gx[0] - div), tyy = vis * (T(2) * gy[1] - div), tzz = vis * (T(2) * gz[2] - div);
-    const T txy = vis * (gy[0] + gx[1]), txz = vis * (gz[0] + gx[2]), tyz = vis * (gz[1] + gy[2]);
-    const T v1 = n1 * txx + n2 * txy + n3 * txz;
-    const T v2 = n1 * txy + n2 * tyy + n3 * tyz;
-    const T v3 = n1 * txz + n2 * tyz + n3 * tzz;
-    const T v4 = fm[0] * v1 + fm[1] * v2 + fm[2] * v3 + qn;
-    const T sc = -(T)c.oRe * (T)area;
-    fv[0] = sc * v1; fv[1] = sc * v2; fv[2] = sc * v3; fv[3] = sc * v4;
 }
 
-// Three blocks per SM on the mixed path (at most 85 registers): the face pass
-// is latency-bound on its arithmetic, and 16M cells take 5.3 ms against 6.2 ms
-// at the two blocks its natural 101 registers allow.
+// Viscous flux times the area, F1..F4 (F0 is zero), and the face's viscous
+// spectral-radius term, which is also the LU-SGS viscous factor of both face uses
+// (SpectrumRadiusViscous method 2, NSSolverUnstruct.cpp:5930-5960;
+// SolveLUSGSForward :15339-15357): GetVisFaceValue (:7126-7375, static adiabatic
+// walls: the mean of a wall's two sides is at rest) and ComputeVisflux
+// (:12977-13378, perfect gas).  The face gradient F of u, v, w has its normal part
+// replaced by the normal derivative; what ComputeVisflux takes along two tangents
+// is F less its normal part.
+//
+// The pass is bound by memory latency: three blocks per SM, of 256 threads on the
+// mixed path and of 128 in double precision (at most 168 registers), and one side
+// after the other, so that little is held at a time.  With the cell pass, on the
+// 1M-cell bump: mixed 335 -> 255 us, FP64 918 -> 607 us against geometry formed
+// in the pass, gradients read twice and 256 threads at 166 registers.
+template <class T>
+constexpr int kFaceThreads = sizeof(T) == 4 ? 256 : 128;
+
 template <class T, bool kVisc, int kScheme>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1) face_flux_kernel(DevGrid g, NsConst c, Work<T> w)
+__global__ void __launch_bounds__(kFaceThreads<T>, 3) face_flux_kernel(DevGrid g, NsConst c, Work<T> w)
 {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= g.nFace) return;
     const int2 lr = ld(g.lr + f);
     const int le = lr.x, re = lr.y;
-    double fr[8];
-    ld8(g.frec + (size_t)f * kF, fr);
+    const T *geo = w.fgeo + (size_t)f * kGeo<kVisc>;
+    T gn[4], gl[4], gr[4], xl[4], xr[4];
+    ld4(geo, gn);
+    ld4(geo + 4, gl);
+    ld4(geo + 8, gr);
+    if (kVisc) { ld4(geo + 12, xl); ld4(geo + 16, xr); }
     T qL[8], qR[8];
     ld8(w.qrec + (size_t)le * kQ, qL);
     ld8(w.qrec + (size_t)re * kQ, qR);
+    const T xn = gn[0], yn = gn[1], zn = gn[2], area = gn[3];
+    const bool cellR = re < g.nCell || g.bkind[f] == BK_INTERFACE;
     T limL = qL[7], limR = qR[7];
     if (c.reconMethod == 1) { const T m = tmin(limL, limR); limL = limR = m; }
-    T ql[5], qr[5];
-    if (kScheme != 0 && c.firstOrder) {
+    const bool recon = !(kScheme != 0 && c.firstOrder);
+    const T gm = (T)c.gama;
+    T ql[5], qr[5], fl[8], fv[4], vspec = T(0);
+    {
+        T F[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, f1[3], f2[3];
+        const T coef = (T)c.coefState;
+        const T tl0 = kVisc ? temperature(qL, coef) : T(0), tr0 = kVisc ? temperature(qR, coef) : T(0);
+        T tL = tl0, tR = tr0;
+        face_side<T, kVisc>(w.grec + (size_t)le * kG, recon, limL, gl, qL, ql, gl[3], xl, F, f1, tL);
+        // a boundary ghost has the owner's gradient (least squares, GG-node) or
+        // none (GG-cell), as the reference's gradient routines leave them
+        const T *gp = cellR ? w.grec + (size_t)re * kG : (kVisc && c.gradient != 0 ? w.grec + (size_t)le * kG : nullptr);
+        face_side<T, kVisc>(gp, recon && cellR, limR, gr, qR, qr, cellR ? T(1) - gl[3] : T(0), xr, F, f2, tR);
+        if (kVisc) {
+            const T S = (T)c.tsuth, A = gr[3], B = xl[3], ds = xr[3];
+            const T mul = T(0.5) * (sutherland(tl0, S) + sutherland(tr0, S));
+            const T mut = w.trec ? T(0.5) * (w.trec[(size_t)le * kTr + 1] + w.trec[(size_t)re * kTr + 1]) : T(0);
+            const T vis = mul + mut;
+            vspec = T(2) * vis / (T(0.5) * (qL[0] + qR[0]) * ds * (T)c.reynolds + (T)kSmall) * (T(0.5) * area);
+            T fm[3];
 #pragma unroll
-        for (int k = 0; k < 5; ++k) { ql[k] = qL[k]; qr[k] = qR[k]; }
-    } else {
-        reconstruct<T>(g, w, le, fr + 4, limL, qL, ql);
-        reconstruct<T>(g, w, re, fr + 4, limR, qR, qr, f < g.nBFace && g.bkind[f] == BK_INTERFACE);
+            for (int k = 0; k < 3; ++k) {
+                fm[k] = T(0.5) * (qL[k + 1] + qR[k + 1]);
+                const T dn = A * (f1[k] - fm[k]) + B * (f2[k] - fm[k]);
+                const T dt = dn - (F[3 * k] * xn + F[3 * k + 1] * yn + F[3 * k + 2] * zn);
+                F[3 * k] += xn * dt; F[3 * k + 1] += yn * dt; F[3 * k + 2] += zn * dt;
+            }
+            const T tM = T(0.5) * (tl0 + tr0);
+            const T qn = (mul * (T)c.oPrl + mut * (T)c.oPrt) * (T)c.cp * (A * (tL - tM) + B * (tR - tM));
+            const T div = T(2.0 / 3.0) * (F[0] + F[4] + F[8]);
+            const T txx = vis * (T(2) * F[0] - div), tyy = vis * (T(2) * F[4] - div), tzz = vis * (T(2) * F[8] - div);
+            const T txy = vis * (F[1] + F[3]), txz = vis * (F[2] + F[6]), tyz = vis * (F[5] + F[7]);
+            const T v1 = xn * txx + yn * txy + zn * txz;
+            const T v2 = xn * txy + yn * tyy + zn * tyz;
+            const T v3 = xn * txz + yn * tyz + zn * tzz;
+            const T v4 = fm[0] * v1 + fm[1] * v2 + fm[2] * v3 + qn;
+            const T sc = -(T)c.oRe * area;
+            fv[0] = sc * v1; fv[1] = sc * v2; fv[2] = sc * v3; fv[3] = sc * v4;
+        }
     }
-    const T xn = (T)fr[0], yn = (T)fr[1], zn = (T)fr[2], area = (T)fr[3];
     if (f < g.nBFace) {
         const int bt = g.btype[f];
         if (bt == PHX_BC_SOLID_SURFACE || bt == PHX_BC_SYMMETRY) {
@@ -646,8 +622,6 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1) face_flux_ke
             }
         }
     }
-    const T gm = (T)c.gama;
-    T fl[8];
     if (kScheme == 0) roe_flux<T>(ql, qr, gm, gm, xn, yn, zn, (T)c.acoustic, (T)c.convective, fl);
     else if (kScheme == 2) vanleer_rotate_flux_fp64<T>(ql, qr, gm, gm, xn, yn, zn, fl);
     else other_flux<T>(c.scheme, ql, qr, gm, gm, xn, yn, zn, (T)c.ausmpwLim, fl);
@@ -664,16 +638,13 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1) face_flux_ke
         const T cm = sqrt(gmm * pm / rm);
         fl[5] = T(0.5) * area * (fabs(vn) + cm);
     }
-    T vspec = T(0);
-    if (kVisc) {
-        T fv[4];
-        viscous_face<T>(g, c, w, f, le, re, fr, qL, qR, fv, vspec);
-        T vr[8] = {fv[0], fv[1], fv[2], fv[3], T(0), T(0), T(0), T(0)};
-        st8(w.flux + (size_t)f * kFlux + 8, vr);
-    }
     fl[6] = vspec;
-    fl[7] = T(0);
+    fl[7] = kVisc ? fv[0] : T(0);
     st8(w.flux + (size_t)f * kFlux, fl);
+    if (kVisc) {
+        const T r[4] = {fv[1], fv[2], fv[3], T(0)};
+        st4(w.flux + (size_t)f * kFlux + 8, r);
+    }
     // LU-SGS factors of the left cell's and the right cell's use
     const T rad = roe_radius<T>(qL, qR, xn, yn, zn, gm);
     T v[kUse];
@@ -704,40 +675,31 @@ __global__ void __launch_bounds__(kThreads) cell_residual_kernel(DevGrid g, NsCo
     const int cell = blockIdx.x * blockDim.x + threadIdx.x;
     double mydt = kLarge;
     if (cell < g.nCell) {
-        T res[5] = {0, 0, 0, 0, 0};
+        // ViscousFlux is loaded after InviscidFlux (NSSolver::UpdateResiduals,
+        // NSSolver.cpp:71-80): its sum, in the same face order, is added at the end
+        T res[5] = {0, 0, 0, 0, 0}, rv[4] = {0, 0, 0, 0};
         T spec = T(0), vis = T(0);
-        const int j0 = g.c2f_off[cell], j1 = g.c2f_off[cell + 1];
-        for (int j = j0; j < j1; ++j) {
-            const int f = ld(g.c2f + j);
-            const bool isLeft = ld(&g.lr[f].x) == cell;
+        const int j1 = g.c2f_off[cell + 1];
+        for (int j = g.c2f_off[cell]; j < j1; ++j) {
+            const int e = ld(&g.c2x[j].x);
+            const T *rec = w.flux + (size_t)(e >= 0 ? e : ~e) * kFlux, sg = e >= 0 ? T(-1) : T(1);
             T fl[8];
-            ld8(w.flux + (size_t)f * kFlux, fl);
-            if (isLeft) {
+            ld8(rec, fl);
 #pragma unroll
-                for (int k = 0; k < 5; ++k) res[k] -= fl[k];
-            } else {
-#pragma unroll
-                for (int k = 0; k < 5; ++k) res[k] += fl[k];
-            }
+            for (int k = 0; k < 5; ++k) res[k] += sg * fl[k];
             spec += fl[5];
-            if (kVisc) vis += fl[6];
+            if (kVisc) {
+                T fv[4];
+                ld4(rec + 8, fv);
+                vis += fl[6];
+                rv[0] += sg * fl[7];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) rv[k + 1] += sg * fv[k];
+            }
         }
         if (kVisc) {
-            // ViscousFlux is loaded after InviscidFlux (NSSolver::UpdateResiduals,
-            // NSSolver.cpp:71-80): a second pass in the same face order
-            for (int j = j0; j < j1; ++j) {
-                const int f = ld(g.c2f + j);
-                const bool isLeft = ld(&g.lr[f].x) == cell;
-                T fv[4];
-                ld4(w.flux + (size_t)f * kFlux + 8, fv);
-                if (isLeft) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) res[k + 1] -= fv[k];
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) res[k + 1] += fv[k];
-                }
-            }
+            for (int k = 0; k < 4; ++k) res[k + 1] += rv[k];
         }
         T tot = spec;
         if (c.viscous) tot += vis;
@@ -781,17 +743,18 @@ __global__ void __launch_bounds__(kThreads) cell_residual_kernel(DevGrid g, NsCo
 template <class T>
 void launch_residual(const DevGrid &g, const NsConst &c, const Work<T> &w, Reduce *red, double cfl, cudaStream_t s)
 {
-    const int fb = (g.nFace + kThreads - 1) / kThreads, cb = (g.nCell + kThreads - 1) / kThreads;
+    constexpr int ft = kFaceThreads<T>;
+    const int fb = (g.nFace + ft - 1) / ft, cb = (g.nCell + kThreads - 1) / kThreads;
     const int kind = c.scheme == PHX_SCHEME_ROE ? 0 : c.scheme == PHX_SCHEME_VANLEER_ROTATE ? 2 : 1;
     if (c.viscous) {
-        if (kind == 0) face_flux_kernel<T, true, 0><<<fb, kThreads, 0, s>>>(g, c, w);
-        else if (kind == 2) face_flux_kernel<T, true, 2><<<fb, kThreads, 0, s>>>(g, c, w);
-        else face_flux_kernel<T, true, 1><<<fb, kThreads, 0, s>>>(g, c, w);
+        if (kind == 0) face_flux_kernel<T, true, 0><<<fb, ft, 0, s>>>(g, c, w);
+        else if (kind == 2) face_flux_kernel<T, true, 2><<<fb, ft, 0, s>>>(g, c, w);
+        else face_flux_kernel<T, true, 1><<<fb, ft, 0, s>>>(g, c, w);
         cell_residual_kernel<T, true><<<cb, kThreads, 0, s>>>(g, c, w, red, cfl);
     } else {
-        if (kind == 0) face_flux_kernel<T, false, 0><<<fb, kThreads, 0, s>>>(g, c, w);
-        else if (kind == 2) face_flux_kernel<T, false, 2><<<fb, kThreads, 0, s>>>(g, c, w);
-        else face_flux_kernel<T, false, 1><<<fb, kThreads, 0, s>>>(g, c, w);
+        if (kind == 0) face_flux_kernel<T, false, 0><<<fb, ft, 0, s>>>(g, c, w);
+        else if (kind == 2) face_flux_kernel<T, false, 2><<<fb, ft, 0, s>>>(g, c, w);
+        else face_flux_kernel<T, false, 1><<<fb, ft, 0, s>>>(g, c, w);
         cell_residual_kernel<T, false><<<cb, kThreads, 0, s>>>(g, c, w, red, cfl);
     }
 }
@@ -1404,6 +1367,7 @@ void launch_finish_step(Reduce *r, double *hist, int i, double ncell, cudaStream
 
 // Explicit instantiations for the FP64 and mixed paths.
 #define PHX_INSTANTIATE(T)                                                                                         \
+    template void launch_face_geometry<T>(const DevGrid &, const NsConst &, const Work<T> &, cudaStream_t);        \
     template void launch_boundary<T>(const DevGrid &, const NsConst &, double *, const Work<T> &, cudaStream_t);   \
     template void launch_gradient_limiter<T>(const DevGrid &, const NsConst &, const Work<T> &, int, cudaStream_t); \
     template void launch_residual<T>(const DevGrid &, const NsConst &, const Work<T> &, Reduce *, double,           \
