@@ -749,6 +749,7 @@ int make_work(phx_ctx *ctx, Work<T> &w, const std::vector<double> &limInit)
     r |= dalloc(ctx, &w.grec, nt * kG);
     r |= dalloc(ctx, &w.fnrm, nf * kNrm);
     r |= dalloc(ctx, &w.fgeo, nf * (ctx->prm.viscousType ? kGeo<true> : kGeo<false>));
+    if (ctx->sa) r |= dalloc(ctx, &w.fsa, nf * kGeoSa);
     r |= dalloc(ctx, &w.flux, nf * kFlux);
     r |= dalloc(ctx, &w.coef, (size_t)ctx->nBFace * kUse);
     r |= make_rows(ctx, &w.rowf, 0, kRowNs<T, true>);

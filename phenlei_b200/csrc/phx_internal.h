@@ -91,8 +91,12 @@ constexpr int kMaxDevices = 64;                       // per-device launch cache
 constexpr int kTr = 4;     // trec: nu~ | eddy viscosity | laminar viscosity of the NS step | pad
 constexpr int kTg = 4;     // tgrad: d nu~ / dx, dy, dz | pad
 constexpr int kTc = 4;     // tcrec: res_turb | spec_turb | pad
-constexpr int kTf = 8;     // tface: convective flux | diffusion flux1, flux2 | upwind Jacobians L, R |
-                           // diffusion spectral term | pad
+constexpr int kTf = 4;     // tface: convection and first diffusion flux | second diffusion flux (times the side's own
+                           // diffusivity) | spectral terms of the left and of the right cell
+// SA face geometry (working precision, formed once in FP64): unit normal, area |
+// factor of the difference right less left in the normal derivative | one over
+// the mean volume | pad.
+constexpr int kGeoSa = 8;
 
 // Schedule of one LU-SGS sweep (phx_schedule.cpp): warp w runs rows
 // [row_off[w], row_off[w + 1]).
@@ -186,6 +190,7 @@ template <class T>
 struct Work {
     T *qrec;        // [nTotal][kQ] working state, c2 = |gamma p / rho|, total enthalpy, limiter
     T *fnrm, *fgeo; // [nFace][kNrm], [nFace][kGeo] face geometry
+    T *fsa;         // [nFace][kGeoSa] SA face geometry (SA runs; else null)
     T *grec;        // [nTotal][kG] primitive gradients (ghost rows: interface ghosts only, from the halo exchange)
     T *flux;        // [nFace][kFlux] face flux times area and inviscid spectral radius term
     T *coef;        // [nBFace][kUse] LU-SGS factors of the boundary faces' uses

@@ -177,6 +177,23 @@ __global__ void __launch_bounds__(kThreads) face_geometry_kernel(DevGrid g, NsCo
         o[16 + k] = vf & 1 ? (T)(fr[k] * dR + dr[k]) : T(0);
     }
     o[15] = (T)B;
+    if (w.fsa) {
+        // normal derivative of TurbSolverUnstr::ComputeVisflux (TurbSolverUnstr.cpp:
+        // 4438-4674): the weighted differences to the mean of both sides, or across
+        // the whole distance on boundary faces other than symmetry
+        double C = 0.0;
+        if (vf & 4) {
+            const double wl = dL * dL / (dL * dL + dR * dR);
+            C = 0.5 * ((1.0 - wl) / dR - wl / dL);
+            if (bnd && g.btype[f] != PHX_BC_SYMMETRY)
+                C = 1.0 / ((xr[0] - xl[0]) * fr[0] + (xr[1] - xl[1]) * fr[1] + (xr[2] - xl[2]) * fr[2]);
+        }
+        T *sa = w.fsa + (size_t)f * kGeoSa;
+        for (int k = 0; k < 4; ++k) sa[k] = (T)fr[k];
+        sa[4] = (T)C;
+        sa[5] = (T)(1.0 / (0.5 * (xl[3] + xr[3])));
+        sa[6] = sa[7] = T(0);
+    }
     o[19] = (T)fabs(fr[0] * (xr[0] - xl[0]) + fr[1] * (xr[1] - xl[1]) + fr[2] * (xr[2] - xl[2]));
 }
 

@@ -134,30 +134,20 @@ __global__ void __launch_bounds__(kThreads) sa_visc_grad_kernel(DevGrid g, NsCon
         vist = rho * fv1 * nue;
     }
     w.trec[(size_t)cell * kTr + 1] = vist;
-    double xc[4];
-    ld4(g.xrec + (size_t)cell * kX, xc);
+    const T vol = (T)ld(g.xrec + (size_t)cell * kX + 3);
     T gx = T(0), gy = T(0), gz = T(0);
     const int j0 = g.c2f_off[cell], j1 = g.c2f_off[cell + 1];
     for (int j = j0; j < j1; ++j) {
-        const int f = ld(g.c2f + j);
-        const int2 lr = ld(g.lr + f);
-        const bool isLeft = (lr.x == cell);
-        const int nb = isLeft ? lr.y : lr.x;
-        const T vn = ldcg(w.trec + (size_t)nb * kTr);   // slot 1 of the rows is written by this kernel
+        const int2 e = ld(g.c2x + j);
+        const bool isLeft = e.x >= 0;
+        const int f = isLeft ? e.x : ~e.x;
+        const T vn = ldcg(w.trec + (size_t)e.y * kTr);   // slot 1 of the rows is written by this kernel
+        T nr[4];
+        ld4(w.fnrm + (size_t)f * kNrm, nr);
         if (kLsq) {
-            double xn[4];
-            ld4(g.xrec + (size_t)nb * kX, xn);
-            const double iw = ld(g.frec + (size_t)f * kF + 7);
-            const T dx = (T)(isLeft ? xn[0] - xc[0] : xc[0] - xn[0]);
-            const T dy = (T)(isLeft ? xn[1] - xc[1] : xc[1] - xn[1]);
-            const T dz = (T)(isLeft ? xn[2] - xc[2] : xc[2] - xn[2]);
-            const T dq = (T)iw * (isLeft ? vn - nue : nue - vn);
-            gx += dq * dx; gy += dq * dy; gz += dq * dz;
+            const T dq = nr[3] * (isLeft ? vn - nue : nue - vn);
+            gx += dq * nr[0]; gy += dq * nr[1]; gz += dq * nr[2];
         } else {
-            double fr[4];
-            ld4(g.frec + (size_t)f * kF, fr);
-            const double a = fr[3];
-            const T nx = (T)(fr[0] * a), ny = (T)(fr[1] * a), nz = (T)(fr[2] * a);
             T qf = T(0.5) * (isLeft ? (nue + vn) : (vn + nue));
             if (kGrad == 2 && (f >= g.nBFace || ld(g.btype + f) == PHX_BC_SYMMETRY)) {
                 // UnstructGrid::CompGradientGGNode_NEW (Geo_UnstructGrid.cpp:4202-4309)
@@ -166,8 +156,8 @@ __global__ void __launch_bounds__(kThreads) sa_visc_grad_kernel(DevGrid g, NsCon
                 for (int k = a0; k < a1; ++k) sn += t.qtnode[ld(g.fn_idx + k)];
                 qf = sn / (T)(a1 - a0);
             }
-            if (isLeft) { gx += qf * nx; gy += qf * ny; gz += qf * nz; }
-            else { gx -= qf * nx; gy -= qf * ny; gz -= qf * nz; }
+            if (isLeft) { gx += qf * nr[0]; gy += qf * nr[1]; gz += qf * nr[2]; }
+            else { gx -= qf * nr[0]; gy -= qf * nr[1]; gz -= qf * nr[2]; }
         }
     }
     if (kLsq) {
@@ -178,10 +168,9 @@ __global__ void __launch_bounds__(kThreads) sa_visc_grad_kernel(DevGrid g, NsCon
         gy = (T)m6[3] * tx + (T)m6[1] * ty + (T)m6[5] * tz;
         gz = (T)m6[4] * tx + (T)m6[5] * ty + (T)m6[2] * tz;
     } else if (kGrad == 2) {
-        const T vol = (T)xc[3];
         gx /= vol; gy /= vol; gz /= vol;
     } else {
-        const T ovol = T(1) / (T)xc[3];
+        const T ovol = T(1) / vol;
         gx *= ovol; gy *= ovol; gz *= ovol;
     }
     T o[4] = {gx, gy, gz, T(0)};
@@ -225,18 +214,17 @@ __global__ void __launch_bounds__(kThreads) sa_face_kernel(DevGrid g, NsConst c,
     // GetQlQrNS, TurbSolverUnstr.cpp:5041, :5125) and the normal derivative (:4569)
     const bool bnd = f < g.nBFace && g.bkind[f] != BK_INTERFACE;
     const int bt = bnd ? g.btype[f] : 0;
-    double fr[8];
-    ld8(g.frec + (size_t)f * kF, fr);
-    T qL[8], qR[8], tl[4], tr[4];
+    T geo[8], qL[8], qR[8], tl[4], tr[4];
+    ld8(w.fsa + (size_t)f * kGeoSa, geo);
     ld8(w.qrec + (size_t)le * kQ, qL);
     ld8(w.qrec + (size_t)re * kQ, qR);
     ld4(w.trec + (size_t)le * kTr, tl);
     ld4(w.trec + (size_t)re * kTr, tr);
-    const T nx = (T)fr[0], ny = (T)fr[1], nz = (T)fr[2], area = (T)fr[3];
+    const T nx = geo[0], ny = geo[1], nz = geo[2], area = geo[3];
     const T oRe = (T)c.oRe;
     const T cb2 = T(0.622);
     const T osigma = T(1) / T(2.0 / 3.0);
-    T out[8];
+    T out[4];
     // convection
     {
         T ql = tl[0], qr = tr[0];
@@ -269,27 +257,9 @@ __global__ void __launch_bounds__(kThreads) sa_face_kernel(DevGrid g, NsConst c,
             nr = positive_sa(nr, vr, rr);
         }
         const T mlt = osigma * T(0.5) * (vl / rl + vr / rr + nl + nr);
-        T dfdn = T(0);
-        if (g.vflag[f] & 4) {
-            double xl[4], xr[4];
-            ld4(g.xrec + (size_t)le * kX, xl);
-            ld4(g.xrec + (size_t)re * kX, xr);
-            const double dL = fr[0] * (xl[0] - fr[4]) + fr[1] * (xl[1] - fr[5]) + fr[2] * (xl[2] - fr[6]);
-            const double dR = fr[0] * (xr[0] - fr[4]) + fr[1] * (xr[1] - fr[5]) + fr[2] * (xr[2] - fr[6]);
-            const T f1 = tl[0], f2 = tr[0];
-            const T fm = T(0.5) * (f1 + f2);
-            const T dLt = (T)dL, dRt = (T)dR;
-            const T d1 = (f1 - fm) / dLt, d2 = (f2 - fm) / dRt;
-            const T wl = dLt * dLt / (dLt * dLt + dRt * dRt);
-            const T wr = T(1) - wl;
-            dfdn = wl * d1 + wr * d2;
-            if (bnd && bt != PHX_BC_SYMMETRY) {
-                const double nd = (xr[0] - xl[0]) * fr[0] + (xr[1] - xl[1]) * fr[1] + (xr[2] - xl[2]) * fr[2];
-                dfdn = (f2 - f1) / (T)nd;
-            }
-        }
-        out[1] = -oRe * (T(1) + cb2) * mlt * dfdn * area;
-        out[2] = oRe * cb2 * osigma * dfdn * area;
+        const T dfdn = geo[4] * (tr[0] - tl[0]);
+        out[0] += -oRe * (T(1) + cb2) * mlt * dfdn * area;
+        out[1] = oRe * cb2 * osigma * dfdn * area;
     }
     // spectral radius and face matrices
     T matR, matL;
@@ -305,13 +275,11 @@ __global__ void __launch_bounds__(kThreads) sa_face_kernel(DevGrid g, NsConst c,
         const T effl = tl[2] * orl + fabs(nuel);
         const T effr = tr[2] * orr + fabs(nuer);
         const T eff = T(0.5) * (effl + effr);
-        const T ovol = T(1) / (T(0.5) * ((T)g.xrec[(size_t)le * kX + 3] + (T)g.xrec[(size_t)re * kX + 3]));
+        const T ovol = geo[5];
         const T ns2 = area * area;
         const T vterm = oRe * ovol * (T(1) + cb2) * (osigma * eff * ns2);
-        out[3] = ijl;
-        out[4] = ijr;
-        out[5] = vterm;
-        out[6] = out[7] = T(0);
+        out[2] = ijl + vterm;
+        out[3] = vterm - ijr;
         matR = ijr;
         matL = -ijl;
         matL += -oRe * ovol * (T(1) + cb2) * (osigma * eff * ns2);
@@ -320,7 +288,7 @@ __global__ void __launch_bounds__(kThreads) sa_face_kernel(DevGrid g, NsConst c,
         matL += oRe * ovol * ns2 * cl;
         matR += oRe * ovol * ns2 * cr;
     }
-    st8(t.tface + (size_t)f * kTf, out);
+    st4(t.tface + (size_t)f * kTf, out);
     if (f >= g.nBFace) {
         const int2 at = ld(g.use + f);
         *sa_use_at<T>(t, at.x) = matR;
@@ -333,9 +301,9 @@ __global__ void __launch_bounds__(kThreads) sa_face_kernel(DevGrid g, NsConst c,
 // 1025-1072) with the NS step's final dt, the exact source and its implicit
 // part (SourceFluxOneEquationOriginal, :2702-2916, NSMB formation: the cb2
 // gradient term is carried by the diffusion flux), then the face terms in the
-// reference's order: convection over all faces (InviscidFlux), diffusion over
-// all faces (ViscousFlux), and, into the spectral radius, the Jacobians of
-// SpectrumRadiusOfOneEquation (called by Diagonal before the sweeps).
+// reference's face order: convection (InviscidFlux) and diffusion (ViscousFlux),
+// and, into the spectral radius, the Jacobians of SpectrumRadiusOfOneEquation
+// (called by Diagonal before the sweeps).
 // ---------------------------------------------------------------------------
 template <class T>
 __global__ void __launch_bounds__(kThreads) sa_cell_kernel(DevGrid g, NsConst c, Work<T> w, TurbWork<T> t,
@@ -376,32 +344,19 @@ __global__ void __launch_bounds__(kThreads) sa_cell_kernel(DevGrid g, NsConst c,
     res += src * (T)vol;
     T spec = T(0) * (T)vol + T(1) / ((T)c.turbCflScale * dt + (T)kSmall);
     spec += sspec * (T)vol;
-    const int j0 = g.c2f_off[cell], j1 = g.c2f_off[cell + 1];
-    for (int j = j0; j < j1; ++j) {
-        const int f = ld(g.c2f + j);
-        const bool isLeft = ld(&g.lr[f].x) == cell;
-        const T fl = ld(t.tface + (size_t)f * kTf);
-        if (isLeft) res -= fl;
-        else res += fl;
+    const int j1 = g.c2f_off[cell + 1];
+    T flux = T(0), own = T(0);
+    for (int j = g.c2f_off[cell]; j < j1; ++j) {
+        const int e = ld(&g.c2x[j].x);
+        T tf[4];
+        ld4(t.tface + (size_t)(e >= 0 ? e : ~e) * kTf, tf);
+        const T sg = e >= 0 ? T(-1) : T(1);
+        flux += sg * tf[0];
+        own += sg * tf[1];
+        spec += e >= 0 ? tf[2] : tf[3];
     }
-    const T own = visl / rho + positive_sa(nue, visl, rho);
-    for (int j = j0; j < j1; ++j) {
-        const int f = ld(g.c2f + j);
-        const bool isLeft = ld(&g.lr[f].x) == cell;
-        T tf[8];
-        ld8(t.tface + (size_t)f * kTf, tf);
-        if (isLeft) { res -= tf[1]; res -= tf[2] * own; }
-        else { res += tf[1]; res += tf[2] * own; }
-    }
-    for (int j = j0; j < j1; ++j) {
-        const int f = ld(g.c2f + j);
-        const bool isLeft = ld(&g.lr[f].x) == cell;
-        T tf[8];
-        ld8(t.tface + (size_t)f * kTf, tf);
-        if (isLeft) spec += tf[3];
-        else spec -= tf[4];
-        spec += tf[5];
-    }
+    res += flux;
+    res += own * (visl / rho + positive_sa(nue, visl, rho));
     T o[4] = {res, spec, idiv(T(1), spec), T(0)};   // the sweep multiplies by the reciprocal
     st4(t.tcrec + (size_t)cell * kTc, o);
     T *lead = sa_lead_at<T>(t.trowf, ld(g.lead + cell));

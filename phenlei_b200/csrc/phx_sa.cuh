@@ -34,7 +34,7 @@ __device__ __forceinline__ void sa_source_exact(T nue, T omega, T olam, T odist2
     const T kap2 = karm * karm, okap2 = T(1) / kap2;
     const T cw1 = cb1 * okap2 + (T(1) + cb2) / sigma;
     const T cv13 = cv1 * cv1 * cv1;
-    const T cw36 = pow(cw3, T(6));
+    const T cw36 = cw3 * cw3 * cw3 * cw3 * cw3 * cw3;
     const T or6 = T(1) / T(6);
     const T ct3 = T(1.2);
     const T saC2 = T(0.7), saC3 = T(0.9);
@@ -53,9 +53,9 @@ __device__ __forceinline__ void sa_source_exact(T nue, T omega, T olam, T odist2
     const T ostd = T(1) / (std_ + (T)kSmall);
     T r = rs * ostd;
     r = tmin(r, T(10));
-    const T r5 = pow(r, T(5));
+    const T r5 = r * r * (r * r) * r;
     const T gg = r + cw2 * (r5 * r - r);
-    const T g6 = pow(gg, T(6));
+    const T g6 = gg * gg * gg * (gg * gg * gg);
     const T fw = gg * pow((T(1) + cw36) / (g6 + cw36), or6);
     const T ft2 = T(0);
     T production = cb1 * (T(1) - ft2) * std_ * nue;
@@ -66,7 +66,8 @@ __device__ __forceinline__ void sa_source_exact(T nue, T omega, T olam, T odist2
         walldest = -destrAlpha * cw1kap2 * nuetrs;
     }
     src = production - walldest;
-    const T dfv2dk = (T(3) * cv13 * pow(fv1 / (xsi + (T)kSmall), T(2)) - T(1)) / pow(T(1) + xsi * fv1, T(2));
+    const T fx = fv1 / (xsi + (T)kSmall), ox = T(1) + xsi * fv1;
+    const T dfv2dk = (T(3) * cv13 * (fx * fx) - T(1)) / (ox * ox);
     const T dsdnu = oRe * okap2 * odist2 * (fv2 + xsi * dfv2dk);
     const T dfwdg = fw / (gg + (T)kSmall) * (T(1) - g6 / (g6 + cw36));
     const T dgdr = T(1) + cw2 * (T(6) * r5 - T(1));
