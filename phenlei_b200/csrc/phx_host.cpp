@@ -39,10 +39,10 @@ struct phx_ctx {
     int device = 0;
     int numSMs = 148;
     cudaStream_t stream = nullptr;
-    // second stream of the fused driver: the next step's NS boundary and
-    // gradient run on it while the SA sweep runs (phx_ns_relaxation)
+    // second stream of the fused driver: the SA sweeps run on it beside the next
+    // step's NS boundary, gradient and residual (phx_ns_relaxation)
     cudaStream_t aux = nullptr;
-    cudaEvent_t evFork = nullptr, evHead = nullptr;
+    cudaEvent_t evFork = nullptr, evTail = nullptr;
     std::string err;
     int64_t launches = 0;
     phx_params prm{};
@@ -1227,7 +1227,7 @@ int phx_ctx_destroy(phx_ctx *ctx)
         cudaStreamSynchronize(ctx->aux);
         cudaStreamDestroy(ctx->aux);
         cudaEventDestroy(ctx->evFork);
-        cudaEventDestroy(ctx->evHead);
+        cudaEventDestroy(ctx->evTail);
     }
     for (void *p : ctx->allocs) cudaFree(p);
     delete ctx;
@@ -1607,27 +1607,28 @@ int phx_sa_update(phx_ctx *ctx)
 }
 
 // One outer step.  With `headDone` the step's NS boundary, gradient and
-// residual have already run on the second stream (see below) and are only
-// joined, before the NS sweep.  With `prefetch` and SA, the next step's NS
-// boundary, gradient and residual are issued on the second stream right after
-// this step's SA residual, so that they run while the latency-bound SA sweep
-// and SA update run.  They need the updated NS state and the eddy viscosity,
-// which the SA residual has formed (the SA update changes nu~ only, and the SA
-// boundary after it writes the ghosts' eddy viscosity again with the same
-// values); they write ghost states, gradients, the limiter, the laminar
-// viscosity slot, the face fluxes and LU-SGS factors, the NS residual record,
-// the time step and the NS reduction fields, none of which the SA sweep, SA
-// update or SA boundary reads (they read the SA records, the owner cells'
-// FP64 state and the eddy viscosity).  The two cooperative sweeps never
-// overlap: the NS sweep waits for both streams.
+// residual have already run (see below).  With `prefetch` and SA, the SA sweeps
+// and the SA update of this step run on the second stream, and the next step's NS
+// boundary, gradient and residual on the context's stream beside them: the sweeps
+// are bound by latency and leave the memory system idle.  The next step's phases
+// need the updated NS state and the eddy viscosity, which the SA residual has
+// formed (the SA update changes nu~ only, and the SA boundary after it writes the
+// ghosts' eddy viscosity again with the same values); they write ghost states,
+// gradients, the limiter, the laminar viscosity slot, the face fluxes and LU-SGS
+// rows, the NS residual record, the time step and the NS reduction fields, none of
+// which the SA sweep, SA update or SA boundary reads (they read the SA records,
+// the owner cells' FP64 state and the eddy viscosity).  The second stream has
+// priority, so that the sweeps, all of whose warps must be resident, do not queue
+// behind the passes' thousands of blocks (1M-cell bump, mixed: 1.97 ms a step in
+// order, 1.96 with the passes first, 1.93 so; FP64 2.97, 2.77, 2.77).  The NS and
+// SA sweeps never overlap: the context's stream waits for the second before it
+// goes on.
 static int relax_one(phx_ctx *ctx, double *dhist, int i, bool headDone, bool prefetch, bool &prefetched)
 {
     ctx->step += 1;   // Simulation::UpdateOuterIterationStep
     prefetched = false;
     int rc;
-    if (headDone) {
-        PHX_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->evHead, 0));
-    } else {
+    if (!headDone) {
         if ((rc = phx_ns_boundary(ctx))) return rc;
         if ((rc = phx_ns_gradient_limiter(ctx))) return rc;
         if ((rc = phx_ns_residual(ctx))) return rc;
@@ -1637,23 +1638,29 @@ static int relax_one(phx_ctx *ctx, double *dhist, int i, bool headDone, bool pre
     launch_finish_step(ctx->red, dhist, i, (double)ctx->nCell, ctx->stream);
     if (ctx->sa) {
         if ((rc = phx_sa_residual(ctx))) return rc;
+        cudaStream_t main = ctx->stream;
         if (prefetch) {
-            PHX_CUDA(ctx, cudaEventRecord(ctx->evFork, ctx->stream));
+            PHX_CUDA(ctx, cudaEventRecord(ctx->evFork, main));
             PHX_CUDA(ctx, cudaStreamWaitEvent(ctx->aux, ctx->evFork, 0));
-            cudaStream_t main = ctx->stream;
             ctx->stream = ctx->aux;
-            ctx->step += 1;   // the next step's flow-initialisation phase and CFL
-            rc = phx_ns_boundary(ctx);
-            if (!rc) rc = phx_ns_gradient_limiter(ctx);
-            if (!rc) rc = phx_ns_residual(ctx);
-            ctx->step -= 1;
-            ctx->stream = main;
-            if (rc) return rc;
-            PHX_CUDA(ctx, cudaEventRecord(ctx->evHead, ctx->aux));
-            prefetched = true;
         }
-        if ((rc = phx_sa_lusgs(ctx))) return rc;
-        if ((rc = phx_sa_update(ctx))) return rc;
+        rc = phx_sa_lusgs(ctx);
+        if (!rc) rc = phx_sa_update(ctx);
+        ctx->stream = main;
+        if (prefetch) {
+            if (!rc) {
+                ctx->step += 1;   // the next step's flow-initialisation phase and CFL
+                rc = phx_ns_boundary(ctx);
+                if (!rc) rc = phx_ns_gradient_limiter(ctx);
+                if (!rc) rc = phx_ns_residual(ctx);
+                ctx->step -= 1;
+                prefetched = true;
+            }
+            // after an error too: nothing of this call stays in flight on the second stream
+            PHX_CUDA(ctx, cudaEventRecord(ctx->evTail, ctx->aux));
+            PHX_CUDA(ctx, cudaStreamWaitEvent(main, ctx->evTail, 0));
+        }
+        if (rc) return rc;
     }
     return check_launch(ctx);
 }
@@ -1669,24 +1676,22 @@ int phx_ns_relaxation(phx_ctx *ctx, int nsteps, double *res_hist)
         ctx->hist = h;
         ctx->histCap = nsteps;
     }
-    // the overlap of the SA tail with the next step's NS head (relax_one);
+    // the overlap of the SA sweeps with the next step's NS head (relax_one);
     // PHX_OVERLAP=0 runs every phase on the context's stream, in order
     const char *ov = getenv("PHX_OVERLAP");
     const bool overlap = ctx->sa && !(ov && atoi(ov) == 0);
     if (overlap && !ctx->aux) {
-        PHX_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking));
+        int least = 0, greatest = 0;
+        PHX_CUDA(ctx, cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        PHX_CUDA(ctx, cudaStreamCreateWithPriority(&ctx->aux, cudaStreamNonBlocking, greatest));
         PHX_CUDA(ctx, cudaEventCreateWithFlags(&ctx->evFork, cudaEventDisableTiming));
-        PHX_CUDA(ctx, cudaEventCreateWithFlags(&ctx->evHead, cudaEventDisableTiming));
+        PHX_CUDA(ctx, cudaEventCreateWithFlags(&ctx->evTail, cudaEventDisableTiming));
     }
     bool headDone = false;
     for (int i = 0; i < nsteps; ++i) {
         bool prefetched = false;
         const int rc = relax_one(ctx, ctx->hist, i, headDone, overlap && i + 1 < nsteps, prefetched);
-        if (rc) {
-            // nothing of this call stays in flight on the second stream
-            if (prefetched) cudaStreamWaitEvent(ctx->stream, ctx->evHead, 0);
-            return rc;
-        }
+        if (rc) return rc;
         headDone = prefetched;
     }
     Reduce red;
