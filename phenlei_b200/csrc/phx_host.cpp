@@ -74,6 +74,7 @@ struct phx_ctx {
     double *tmp = nullptr;                // [5][nTotal] staging buffer in the reference's order
     double *hist = nullptr;
     int histCap = 0;
+    unsigned char *result = nullptr;      // pinned: Reduce, residual history of a phx_ns_relaxation call
     bool nodePrev = false;                // GG-node: node values of a previous state are in nrec (slot 5)
     bool turbNodeValid = false;           // GG-node with SA: qtnode holds node values for the next SA gradient
     int step = 0;
@@ -1230,6 +1231,7 @@ int phx_ctx_destroy(phx_ctx *ctx)
         cudaEventDestroy(ctx->evTail);
     }
     for (void *p : ctx->allocs) cudaFree(p);
+    cudaFreeHost(ctx->result);
     delete ctx;
     return PHX_OK;
 }
@@ -1474,12 +1476,11 @@ int phx_ns_residual(phx_ctx *ctx)
 {
     if (!ctx) return PHX_ERR_ARG;
     init_phase(ctx);
-    launch_reset_reduce(ctx->red, ctx->stream);
     const double cfl = cfl_at(ctx->nc, ctx->step);
     if (ctx->mixed) launch_residual<float>(ctx->g, ctx->nc, ctx->w32, ctx->red, cfl, ctx->stream);
     else launch_residual<double>(ctx->g, ctx->nc, ctx->w64, ctx->red, cfl, ctx->stream);
     ctx->haveResidual = true;
-    return check_launch(ctx, 3);
+    return check_launch(ctx, 2);
 }
 
 static int ns_lusgs(phx_ctx *ctx, int sweeps)
@@ -1512,17 +1513,17 @@ int phx_ns_lusgs(phx_ctx *ctx)
 int phx_ns_lusgs_forward(phx_ctx *ctx) { return ctx ? ns_lusgs(ctx, kSweepForward) : PHX_ERR_ARG; }
 int phx_ns_lusgs_backward(phx_ctx *ctx) { return ctx ? ns_lusgs(ctx, kSweepBackward) : PHX_ERR_ARG; }
 
-int phx_ns_update(phx_ctx *ctx)
+// hist: where the step's residual monitor goes (null: nowhere)
+static int ns_update(phx_ctx *ctx, double *hist)
 {
-    if (!ctx) return PHX_ERR_ARG;
     const int nxt = 1 - ctx->cur;
     double *qo = ctx->q64[ctx->cur], *qn = ctx->q64[nxt];
     if (ctx->mixed) {
         launch_update<float>(ctx->g, ctx->nc, ctx->w32, qo, qn, ctx->red, ctx->neglist, ctx->numSMs, ctx->stream);
-        launch_solution_fix<float>(ctx->g, ctx->nc, ctx->w32, qo, qn, ctx->red, ctx->neglist, ctx->stream);
+        launch_solution_fix<float>(ctx->g, ctx->nc, ctx->w32, qo, qn, ctx->red, ctx->neglist, hist, ctx->stream);
     } else {
         launch_update<double>(ctx->g, ctx->nc, ctx->w64, qo, qn, ctx->red, ctx->neglist, ctx->numSMs, ctx->stream);
-        launch_solution_fix<double>(ctx->g, ctx->nc, ctx->w64, qo, qn, ctx->red, ctx->neglist, ctx->stream);
+        launch_solution_fix<double>(ctx->g, ctx->nc, ctx->w64, qo, qn, ctx->red, ctx->neglist, hist, ctx->stream);
     }
     ctx->cur = nxt;
     // Controller::PostSolve (Controller.cpp:5063-5090): ghost states of the
@@ -1531,6 +1532,8 @@ int phx_ns_update(phx_ctx *ctx)
     else launch_boundary_post<double>(ctx->g, ctx->nc, ctx->q64[ctx->cur], ctx->w64, ctx->stream);
     return check_launch(ctx, 3);
 }
+
+int phx_ns_update(phx_ctx *ctx) { return ctx ? ns_update(ctx, nullptr) : PHX_ERR_ARG; }
 
 int phx_sa_boundary(phx_ctx *ctx)
 {
@@ -1634,8 +1637,7 @@ static int relax_one(phx_ctx *ctx, double *dhist, int i, bool headDone, bool pre
         if ((rc = phx_ns_residual(ctx))) return rc;
     }
     if ((rc = phx_ns_lusgs(ctx))) return rc;
-    if ((rc = phx_ns_update(ctx))) return rc;
-    launch_finish_step(ctx->red, dhist, i, (double)ctx->nCell, ctx->stream);
+    if ((rc = ns_update(ctx, dhist + i))) return rc;
     if (ctx->sa) {
         if ((rc = phx_sa_residual(ctx))) return rc;
         cudaStream_t main = ctx->stream;
@@ -1662,18 +1664,23 @@ static int relax_one(phx_ctx *ctx, double *dhist, int i, bool headDone, bool pre
         }
         if (rc) return rc;
     }
-    return check_launch(ctx);
+    return check_launch(ctx, 0);
 }
 
 int phx_ns_relaxation(phx_ctx *ctx, int nsteps, double *res_hist)
 {
     if (!ctx || nsteps < 0) return PHX_ERR_ARG;
     if (ctx->hasInterface) return refuse_zone(ctx, "phx_ns_relaxation");
-    if (nsteps > ctx->histCap) {
+    if (nsteps > ctx->histCap || !ctx->result) {
         double *h = nullptr;
         const int rc = dalloc(ctx, &h, (size_t)nsteps);
         if (rc) return rc;
         ctx->hist = h;
+        // the status and the history come back through pinned memory: a copy to
+        // pageable memory waits for the stream each time
+        cudaFreeHost(ctx->result);
+        ctx->result = nullptr;
+        PHX_CUDA(ctx, cudaMallocHost((void **)&ctx->result, sizeof(Reduce) + sizeof(double) * (size_t)nsteps));
         ctx->histCap = nsteps;
     }
     // the overlap of the SA sweeps with the next step's NS head (relax_one);
@@ -1694,11 +1701,14 @@ int phx_ns_relaxation(phx_ctx *ctx, int nsteps, double *res_hist)
         if (rc) return rc;
         headDone = prefetched;
     }
-    Reduce red;
-    PHX_CUDA(ctx, cudaMemcpyAsync(&red, ctx->red, sizeof(Reduce), cudaMemcpyDeviceToHost, ctx->stream));
+    double *hist = reinterpret_cast<double *>(ctx->result + sizeof(Reduce));
+    PHX_CUDA(ctx, cudaMemcpyAsync(ctx->result, ctx->red, sizeof(Reduce), cudaMemcpyDeviceToHost, ctx->stream));
     if (res_hist && nsteps > 0)
-        PHX_CUDA(ctx, cudaMemcpyAsync(res_hist, ctx->hist, sizeof(double) * nsteps, cudaMemcpyDeviceToHost, ctx->stream));
+        PHX_CUDA(ctx, cudaMemcpyAsync(hist, ctx->hist, sizeof(double) * nsteps, cudaMemcpyDeviceToHost, ctx->stream));
     PHX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    Reduce red;
+    std::memcpy(&red, ctx->result, sizeof(Reduce));
+    if (res_hist && nsteps > 0) std::memcpy(res_hist, hist, sizeof(double) * nsteps);
     if (red.error != 0) {
         // reported once: the next call starts with a clear status
         PHX_CUDA(ctx, cudaMemsetAsync(&ctx->red->error, 0, sizeof(int), ctx->stream));

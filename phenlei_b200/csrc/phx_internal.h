@@ -251,9 +251,10 @@ int launch_lusgs(const DevGrid &g, const NsConst &c, const Work<T> &w, Reduce *r
 template <class T>
 void launch_update(const DevGrid &g, const NsConst &c, const Work<T> &w, const double *q64, double *q64_new,
                    Reduce *red, int *neglist, int numSMs, cudaStream_t s);
+// The ordered repair pass; with hist, also the step's residual monitor into it.
 template <class T>
 void launch_solution_fix(const DevGrid &g, const NsConst &c, const Work<T> &w, const double *q64, double *q64_new,
-                         Reduce *red, int *neglist, cudaStream_t s);
+                         Reduce *red, int *neglist, double *hist, cudaStream_t s);
 // Refreshes qrec (state, c2, hm) of all cells and ghosts from the FP64 master state.
 template <class T>
 void launch_sync_qrec(const DevGrid &g, const NsConst &c, const double *q64, const Work<T> &w, cudaStream_t s);
@@ -266,7 +267,6 @@ void launch_export(const DevGrid &g, const T *rec, int stride, int first, int co
 // q64[k][i] = in[k][orig[i]] and the inverse.
 void launch_import_q(const DevGrid &g, const double *in, double *q64, cudaStream_t s);
 void launch_export_q(const DevGrid &g, const double *q64, double *out, cudaStream_t s);
-void launch_reset_reduce(Reduce *r, cudaStream_t s);
 // out[m] = sum over cells of res_m^2 (FP64 device reduction of the residual record).
 template <class T>
 void launch_resnorm(const DevGrid &g, const Work<T> &w, double *out, int numSMs, cudaStream_t s);
@@ -305,7 +305,6 @@ void launch_forces(const DevGrid &g, const NsConst &c, const Work<T> &w, const d
 // qt64[i] = in[orig[i]] and the working copy in trec, cells and ghosts.
 template <class T>
 void launch_import_turb(const DevGrid &g, const double *in, const TurbWork<T> &t, const Work<T> &w, cudaStream_t s);
-void launch_finish_step(Reduce *r, double *hist, int i, double ncell, cudaStream_t s);
 // trec slot 1 (eddy viscosity) of cells and ghosts from in[orig[i]].
 template <class T>
 void launch_import_vist(const DevGrid &g, const double *in, const Work<T> &w, cudaStream_t s);

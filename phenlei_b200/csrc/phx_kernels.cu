@@ -268,9 +268,15 @@ __global__ void __launch_bounds__(kThreads) node_value_kernel(DevGrid g, NsConst
     st8(r, o);
 }
 
+// Threads of a block in the passes with many registers: in double precision
+// (142 here, 150 in the face pass) three blocks of 128 fit an SM, where one of 256
+// did (1M-cell bump, FP64: 394 -> 289 us).
+template <class T>
+constexpr int kPassThreads = sizeof(T) == 4 ? 256 : 128;
+
 // kGrad: 0 GG-cell, 1 least squares, 2 GG-node.
 template <class T, bool kTemp, int kGrad>
-__global__ void __launch_bounds__(kThreads) gradient_limiter_kernel(DevGrid g, NsConst c, Work<T> w)
+__global__ void __launch_bounds__(kPassThreads<T>) gradient_limiter_kernel(DevGrid g, NsConst c, Work<T> w)
 {
     constexpr bool kLsq = kGrad == 1;
     const int cell = blockIdx.x * blockDim.x + threadIdx.x;
@@ -433,17 +439,18 @@ __global__ void __launch_bounds__(kThreads) gradient_limiter_kernel(DevGrid g, N
 template <class T>
 void launch_gradient_limiter(const DevGrid &g, const NsConst &c, const Work<T> &w, int nodePrev, cudaStream_t s)
 {
-    const int blocks = (g.nCell + kThreads - 1) / kThreads;
+    constexpr int pt = kPassThreads<T>;
+    const int blocks = (g.nCell + pt - 1) / pt;
     if (c.gradient == 2)
         node_value_kernel<T><<<(g.nNode + kThreads - 1) / kThreads, kThreads, 0, s>>>(g, c, w, nodePrev);
     if (c.viscous) {
-        if (c.gradient == 1) gradient_limiter_kernel<T, true, 1><<<blocks, kThreads, 0, s>>>(g, c, w);
-        else if (c.gradient == 2) gradient_limiter_kernel<T, true, 2><<<blocks, kThreads, 0, s>>>(g, c, w);
-        else gradient_limiter_kernel<T, true, 0><<<blocks, kThreads, 0, s>>>(g, c, w);
+        if (c.gradient == 1) gradient_limiter_kernel<T, true, 1><<<blocks, pt, 0, s>>>(g, c, w);
+        else if (c.gradient == 2) gradient_limiter_kernel<T, true, 2><<<blocks, pt, 0, s>>>(g, c, w);
+        else gradient_limiter_kernel<T, true, 0><<<blocks, pt, 0, s>>>(g, c, w);
     } else {
-        if (c.gradient == 1) gradient_limiter_kernel<T, false, 1><<<blocks, kThreads, 0, s>>>(g, c, w);
-        else if (c.gradient == 2) gradient_limiter_kernel<T, false, 2><<<blocks, kThreads, 0, s>>>(g, c, w);
-        else gradient_limiter_kernel<T, false, 0><<<blocks, kThreads, 0, s>>>(g, c, w);
+        if (c.gradient == 1) gradient_limiter_kernel<T, false, 1><<<blocks, pt, 0, s>>>(g, c, w);
+        else if (c.gradient == 2) gradient_limiter_kernel<T, false, 2><<<blocks, pt, 0, s>>>(g, c, w);
+        else gradient_limiter_kernel<T, false, 0><<<blocks, pt, 0, s>>>(g, c, w);
     }
 }
 
@@ -548,6 +555,13 @@ __device__ __forceinline__ void face_side(const T *gp, bool recon, T lim, const 
     }
 }
 
+__device__ __forceinline__ void reset_reduce(Reduce *r)
+{
+    r->mindt_bits = 0x7FEFFFFFFFFFFFFFULL;  // largest finite double
+    for (int k = 0; k < 5; ++k) r->resnorm[k] = 0.0;
+    r->negcount = 0;
+}
+
 // Viscous flux times the area, F1..F4 (F0 is zero), and the face's viscous
 // spectral-radius term, which is also the LU-SGS viscous factor of both face uses
 // (SpectrumRadiusViscous method 2, NSSolverUnstruct.cpp:5930-5960;
@@ -562,13 +576,11 @@ __device__ __forceinline__ void face_side(const T *gp, bool recon, T lim, const 
 // after the other, so that little is held at a time.  With the cell pass, on the
 // 1M-cell bump: mixed 335 -> 255 us, FP64 918 -> 607 us against geometry formed
 // in the pass, gradients read twice and 256 threads at 166 registers.
-template <class T>
-constexpr int kFaceThreads = sizeof(T) == 4 ? 256 : 128;
-
 template <class T, bool kVisc, int kScheme>
-__global__ void __launch_bounds__(kFaceThreads<T>, 3) face_flux_kernel(DevGrid g, NsConst c, Work<T> w)
+__global__ void __launch_bounds__(kPassThreads<T>, 3) face_flux_kernel(DevGrid g, NsConst c, Work<T> w, Reduce *red)
 {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f == 0) reset_reduce(red);   // for the cell pass and the update
     if (f >= g.nFace) return;
     const int2 lr = ld(g.lr + f);
     const int le = lr.x, re = lr.y;
@@ -760,18 +772,18 @@ __global__ void __launch_bounds__(kThreads) cell_residual_kernel(DevGrid g, NsCo
 template <class T>
 void launch_residual(const DevGrid &g, const NsConst &c, const Work<T> &w, Reduce *red, double cfl, cudaStream_t s)
 {
-    constexpr int ft = kFaceThreads<T>;
+    constexpr int ft = kPassThreads<T>;
     const int fb = (g.nFace + ft - 1) / ft, cb = (g.nCell + kThreads - 1) / kThreads;
     const int kind = c.scheme == PHX_SCHEME_ROE ? 0 : c.scheme == PHX_SCHEME_VANLEER_ROTATE ? 2 : 1;
     if (c.viscous) {
-        if (kind == 0) face_flux_kernel<T, true, 0><<<fb, ft, 0, s>>>(g, c, w);
-        else if (kind == 2) face_flux_kernel<T, true, 2><<<fb, ft, 0, s>>>(g, c, w);
-        else face_flux_kernel<T, true, 1><<<fb, ft, 0, s>>>(g, c, w);
+        if (kind == 0) face_flux_kernel<T, true, 0><<<fb, ft, 0, s>>>(g, c, w, red);
+        else if (kind == 2) face_flux_kernel<T, true, 2><<<fb, ft, 0, s>>>(g, c, w, red);
+        else face_flux_kernel<T, true, 1><<<fb, ft, 0, s>>>(g, c, w, red);
         cell_residual_kernel<T, true><<<cb, kThreads, 0, s>>>(g, c, w, red, cfl);
     } else {
-        if (kind == 0) face_flux_kernel<T, false, 0><<<fb, ft, 0, s>>>(g, c, w);
-        else if (kind == 2) face_flux_kernel<T, false, 2><<<fb, ft, 0, s>>>(g, c, w);
-        else face_flux_kernel<T, false, 1><<<fb, ft, 0, s>>>(g, c, w);
+        if (kind == 0) face_flux_kernel<T, false, 0><<<fb, ft, 0, s>>>(g, c, w, red);
+        else if (kind == 2) face_flux_kernel<T, false, 2><<<fb, ft, 0, s>>>(g, c, w, red);
+        else face_flux_kernel<T, false, 1><<<fb, ft, 0, s>>>(g, c, w, red);
         cell_residual_kernel<T, false><<<cb, kThreads, 0, s>>>(g, c, w, red, cfl);
     }
 }
@@ -1208,9 +1220,15 @@ static constexpr int kFixThreads = 1024;
 
 template <class T>
 __global__ void __launch_bounds__(kFixThreads) solution_fix_kernel(DevGrid g, NsConst c, Work<T> w, const double *qo,
-                                                                   double *qn, Reduce *red, int *neglist)
+                                                                   double *qn, Reduce *red, int *neglist, double *hist)
 {
     __shared__ int key[kMaxNeg], val[kMaxNeg];
+    if (hist && threadIdx.x == 0) {
+        // the residual monitor of the step
+        const double v = sqrt(red->resnorm[0] / (double)g.nCell);
+        if ((!(v == v) || v > 1.0e300) && red->error == 0) red->error = PHX_ERR_NUMERIC;
+        *hist = v;
+    }
     const int n = red->negcount;
     if (n <= 0) return;
     if (n > kMaxNeg) {
@@ -1271,9 +1289,9 @@ __global__ void __launch_bounds__(kFixThreads) solution_fix_kernel(DevGrid g, Ns
 
 template <class T>
 void launch_solution_fix(const DevGrid &g, const NsConst &c, const Work<T> &w, const double *q64, double *q64_new,
-                         Reduce *red, int *neglist, cudaStream_t s)
+                         Reduce *red, int *neglist, double *hist, cudaStream_t s)
 {
-    solution_fix_kernel<T><<<1, kFixThreads, 0, s>>>(g, c, w, q64, q64_new, red, neglist);
+    solution_fix_kernel<T><<<1, kFixThreads, 0, s>>>(g, c, w, q64, q64_new, red, neglist, hist);
 }
 
 // ---------------------------------------------------------------------------
@@ -1323,20 +1341,6 @@ void launch_export_q(const DevGrid &g, const double *q64, double *out, cudaStrea
     export_q_kernel<<<(g.nTotal + kThreads - 1) / kThreads, kThreads, 0, s>>>(g, q64, out);
 }
 
-static __global__ void reset_reduce_kernel(Reduce *r)
-{
-    r->mindt_bits = 0x7FEFFFFFFFFFFFFFULL;  // largest finite double
-    for (int k = 0; k < 5; ++k) r->resnorm[k] = 0.0;
-    r->negcount = 0;
-}
-
-static __global__ void finish_step_kernel(Reduce *r, double *hist, int i, double ncell)
-{
-    const double v = sqrt(r->resnorm[0] / ncell);
-    if ((!(v == v) || v > 1.0e300) && r->error == 0) r->error = PHX_ERR_NUMERIC;
-    if (hist) hist[i] = v;
-}
-
 // Residual monitor of the current residual record: out[m] += sum_c res_m^2
 // (FP64; block sums, one atomic per block and equation; out zeroed first).
 template <class T>
@@ -1376,12 +1380,6 @@ void launch_resnorm(const DevGrid &g, const Work<T> &w, double *out, int numSMs,
 template void launch_resnorm<double>(const DevGrid &, const Work<double> &, double *, int, cudaStream_t);
 template void launch_resnorm<float>(const DevGrid &, const Work<float> &, double *, int, cudaStream_t);
 
-void launch_reset_reduce(Reduce *r, cudaStream_t s) { reset_reduce_kernel<<<1, 1, 0, s>>>(r); }
-void launch_finish_step(Reduce *r, double *hist, int i, double ncell, cudaStream_t s)
-{
-    finish_step_kernel<<<1, 1, 0, s>>>(r, hist, i, ncell);
-}
-
 // Explicit instantiations for the FP64 and mixed paths.
 #define PHX_INSTANTIATE(T)                                                                                         \
     template void launch_face_geometry<T>(const DevGrid &, const NsConst &, const Work<T> &, cudaStream_t);        \
@@ -1396,7 +1394,7 @@ void launch_finish_step(Reduce *r, double *hist, int i, double ncell, cudaStream
     template void launch_update<T>(const DevGrid &, const NsConst &, const Work<T> &, const double *, double *,     \
                                    Reduce *, int *, int, cudaStream_t);                                             \
     template void launch_solution_fix<T>(const DevGrid &, const NsConst &, const Work<T> &, const double *,         \
-                                         double *, Reduce *, int *, cudaStream_t);                                  \
+                                         double *, Reduce *, int *, double *, cudaStream_t);                        \
     template void launch_sync_qrec<T>(const DevGrid &, const NsConst &, const double *, const Work<T> &,            \
                                       cudaStream_t);                                                                \
     template void launch_export<T>(const DevGrid &, const T *, int, int, int, int, int, double *, int, cudaStream_t, \
