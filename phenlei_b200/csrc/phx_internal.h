@@ -68,7 +68,7 @@ constexpr int kLeadT = 2;  // SA sweeps: right-hand side | reciprocal spectral r
 constexpr int kSweepLanes = 4;   // LU-SGS lanes (neighbour entries) per slot of a schedule row
 constexpr int kSweepSlots = 8;   // slots (cells) of a row: one warp
 constexpr int kMaxCellFaces = 8; // faces of a cell
-constexpr int kSweepLocal = 4;   // shared-memory rows of a warp's own results
+constexpr int kSweepLocal = 8;   // rows whose results a warp's shared memory holds
 constexpr int kSweepFirst = 8, kSweepLast = 16;   // flags of the host schedule: first, last row of a cell
 // A schedule row on the device (kSweepRow words): per lane the entry of the row
 // after next of its warp, the place of the neighbour's record (>= 0: it is

@@ -394,8 +394,8 @@ void launch_sa_residual(const DevGrid &g, const NsConst &c, const double *q64, c
 // sweeps (Controller::CommunicationDQ, CFD/Solver/src/Controller.cpp:2874-2880).
 // ---------------------------------------------------------------------------
 // Bound by the chain of rows as the NS sweep (0.23 us a row); a row is small, so
-// 16 of them are in flight.  Both sweeps, mixed: 256x122x32 hexahedra 767 -> 351
-// us, the 1M-cell bump with prisms 771 -> 533 us.
+// 16 of them are in flight.  Both sweeps, mixed, against levels dealt out over
+// all SMs: the 200k plate 400 -> 202 us, the 1M-cell bump 779 -> 441 us.
 static constexpr int kSaStages = 8;
 
 template <class T, bool kForward>

@@ -6,7 +6,10 @@
 // arithmetic, so the schedule keeps dependent cells on the warp that computed
 // their neighbour: every cell follows one of its neighbours in that
 // neighbour's slot (a chain; on a mesh numbered along i, the pencils along i),
-// and eight chains make a warp, which hands their results on in shared memory.
+// and eight chains make a warp, which hands the results of its last eight rows on
+// in shared memory (chains of a warp are often two or three levels apart; with
+// one row a chain kept, the 1M-cell bump's warps read their own results through
+// L2, and its sweeps took 754 and 537 us, NS and SA, instead of 608 and 441).
 // A chain that begins joins the warp of its nearest neighbour in the numbering,
 // or the warp that this one's chains spill into, where the distance is like that
 // of the chains already there (on the same mesh: eight pencils next to one
@@ -141,8 +144,8 @@ SweepRows build_sweep(const SweepGraph &g, bool forward, int maxWarps)
         }
     }
 
-    // rows: chain warp v runs on warp v % nWarps and keeps its results in the
-    // warp's shared-memory row (v / nWarps) % kSweepLocal
+    // rows: chain warp v runs on warp v % nWarps; a warp's shared memory holds the
+    // results of its last kSweepLocal rows
     const int nv = (int)spill.size(), nw = std::max(1, std::min(maxWarps, nv));
     out.nWarps = nw;
     auto parts = [&](int c) { return std::max(1, (noff[c + 1] - noff[c] + kSweepLanes - 1) / kSweepLanes); };
@@ -170,11 +173,13 @@ SweepRows build_sweep(const SweepGraph &g, bool forward, int maxWarps)
     out.loc.assign(nrow * kSweepSlots * kSweepLanes, -1);
     std::vector<int> next(out.rowOff.begin(), out.rowOff.end() - 1);
     std::vector<int> held((size_t)nw * kSweepLocal * kSweepSlots, -1);   // cell whose result a shared-memory slot holds
+    std::vector<int> place(nc, -1);                                      // shared-memory slot of a cell's result
     groups([&](int v, int a, int b, int need) {
-        const int w = v % nw, lr = (v / nw) % kSweepLocal, r0 = next[w];
+        const int w = v % nw, r0 = next[w];
         int *h = &held[(size_t)w * kSweepLocal * kSweepSlots];
         next[w] += need;
         for (int p = 0; p < need; ++p) {
+            const int lr = (r0 + p - out.rowOff[w]) % kSweepLocal;
             out.store[r0 + p] = lr;
             for (int i = a; i < b; ++i) {
                 const int c = cells[i], np = parts(c);
@@ -185,13 +190,15 @@ SweepRows build_sweep(const SweepGraph &g, bool forward, int maxWarps)
                 out.flags[at] = std::max(0, j1 - j0) | (p == 0 ? kSweepFirst : 0) | (p == np - 1 ? kSweepLast : 0);
                 for (int j = j0; j < j1; ++j) {
                     out.ent[at * kSweepLanes + (j - j0)] = pos[j];
-                    const int ov = slot[nbr[j]] / kSweepSlots;
-                    const int q = ((ov / nw) % kSweepLocal) * kSweepSlots + slot[nbr[j]] % kSweepSlots;
-                    if (ov % nw == w && h[q] == nbr[j]) out.loc[at * kSweepLanes + (j - j0)] = q;
+                    const int q = place[nbr[j]];
+                    if (slot[nbr[j]] / kSweepSlots % nw == w && h[q] == nbr[j]) out.loc[at * kSweepLanes + (j - j0)] = q;
                 }
             }
             for (int i = a; i < b; ++i)   // results are stored after the row's reads
-                if (parts(cells[i]) == p + 1) h[lr * kSweepSlots + slot[cells[i]] % kSweepSlots] = cells[i];
+                if (parts(cells[i]) == p + 1) {
+                    place[cells[i]] = lr * kSweepSlots + slot[cells[i]] % kSweepSlots;
+                    h[place[cells[i]]] = cells[i];
+                }
         }
     });
     return out;
