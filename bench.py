@@ -206,42 +206,45 @@ def kernel_bytes(m, precision: str, viscous: int = 0, gradient: str = "ggcell") 
     # NS boundary: owner master state + normal -> ghost master state + working record (5 + c2, hm)
     bnd = nb * (5 * 8 + 3 * 8 + 4 + 5 * 8 + 7 * E) + (nb * E if sa else 0)
     out["boundary"] = bnd
-    # gradient + limiter: working state of cells and ghosts, per face normal*area (GG) or weight + centres (LSQ),
-    # face centre (limiter), lr, c2f; cell centre, volume, volpow (+ LSQ matrix); writes gradients + limiter
+    # gradient + limiter: working state of cells and ghosts, per face normal*area (GG) or centre difference and weight
+    # (LSQ), the face centre less each side's centre, the cells' face entries; volume, volpow (+ LSQ matrix); writes
+    # gradients + limiter
     nvar = 6 if vis else 5
-    g = nt * (5 * E) + nf * (4 * 8 + 3 * 8 + 8) + (L + nc + 1) * 4 + nc * (4 * 8 + 8) + nc * (3 * nvar * E + E)
+    g = nt * (5 * E) + nf * (4 * E + 8 * E) + L * 8 + (nc + 1) * 4 + nc * 2 * 8 + nc * (3 * nvar * E + E)
     if lsq:
-        g += nt * 3 * 8 + nc * 6 * 8 + nf * 8
+        g += nc * 6 * 8
     if sa:
         g += nc * E
     out["gradient_limiter"] = g
-    # face pass: state + limiter of both sides (once per cell), gradients, cell centres, face geometry and lr;
-    # writes face flux (5 + spectral parts) and the MXDQ factors of each face use (3 + viscous term)
-    fp = nt * 6 * E + nc * 15 * E + nt * 3 * 8 + nf * (7 * 8 + 8) + nf * 6 * E + L * (3 + (1 if vis else 0)) * E
+    # face pass: state + limiter of both sides (once per cell), gradients, face geometry, lr, places of the two uses;
+    # writes face flux (5 + spectral parts, viscous 4) and the 8 sweep factors of each interior face use
+    ni = nf - nb
+    fp = nt * 6 * E + nc * 15 * E + nf * ((20 if vis else 12) * E + 8 + 8) + nf * 8 * E + (2 * ni + nb) * 8 * E
     if vis:
-        fp += nc * 3 * E + nf * (4 + 1) * E + nf * 1
+        fp += nc * 3 * E + nf * 4 * E
     if sa:
         fp += nt * E
-    # cell pass: face fluxes through c2f + lr, skew, volume, pressure; writes residual, spectral radii, dt
-    cp = nf * 6 * E + (L + nc + 1) * 4 + nf * 4 + nc * (8 + 8 + E) + nc * (8 * E)
+    # cell pass: face fluxes through the cells' face entries, skew, volume, pressure; writes the residual record, dt
+    # and the forward sweep's right-hand side
+    cp = nf * 7 * E + L * 8 + (nc + 1) * 4 + nc * (8 + 8 + E + 4) + nc * (8 + 1 + 8) * E
     if vis:
-        cp += nf * 5 * E
+        cp += nf * 4 * E
     out["residual"] = fp + cp
-    # LU-SGS, two sweeps: per entry neighbour / face / factor indices and the factors, face normal + area,
-    # neighbour state (u v w c2 hm) and dq once per cell per sweep, own res + spectral radii + dt + volume,
-    # dq / delta-flux writes and reads, and the sentinel fill of the three 8-slot write-once records
-    lu = (L * 3 * 4 + L * 4 * E + 2 * nf * 4 * 8 + 2 * nc * 5 * E + 2 * nc * 5 * E
-          + 2 * nc * (7 * E + E + 8) + 2 * nc * 5 * E + 2 * nc * 5 * E + 3 * nc * 8 * E)
+    # LU-SGS, two sweeps: the factors of each interior face use once, a quarter of a 256-byte schedule row per two
+    # cells, right-hand sides (forward read; backward written and read with the boundary part), dq published and
+    # polled, the sentinel fill of both, and the boundary cells' ghost terms
+    lu = (2 * ni * 8 * E + 2 * nc * 32 + nc * (8 + 8 + 16) * E + 2 * nc * (8 + 5) * E + 2 * nc * 8 * E
+          + nb * (2 * 8 * E + 32))
     out["lusgs"] = lu
     # update: FP64 master state in and out (ghosts copied), dq, residual (monitor); working record out
     out["update"] = nc * (5 * 8 + 5 * E + 5 * E + 5 * 8 + 7 * E) + nb * 2 * 5 * 8 + bnd
     if sa:
         sb = nb * (8 + 2 * E + 5 * 8 + 3 * 8 + 4 + 8 + 2 * E)
-        vg = nt * E + nc * (2 * E + E) + nf * (4 * 8 + 8) + (L + nc + 1) * 4 + nc * 4 * 8 + nc * (E + 3 * E)
-        sf = nt * (4 * E + 3 * E + 4 * 8) + nf * (7 * 8 + 8) + nf * 6 * E + L * E
-        sc = nc * (6 * E + 3 * E + 3 * E + E + 8 + E + 8) + nf * 6 * E + (L + nc + 1) * 4 + nf * 4 + nc * 2 * E
+        vg = nt * E + nc * (2 * E + E) + nf * 4 * E + L * 8 + (nc + 1) * 4 + nc * 8 + nc * (E + 3 * E)
+        sf = nt * (4 * E + 3 * E) + nf * (8 * E + 8 + 8) + nf * 4 * E + 2 * ni * E
+        sc = nc * (6 * E + 3 * E + 3 * E + E + 8 + E + 8) + nf * 4 * E + L * 8 + (nc + 1) * 4 + nc * (4 + 2) * E
         out["sa_residual"] = 2 * sb + vg + sf + sc
-        out["sa_lusgs"] = L * 2 * 4 + L * E + 2 * nc * 2 * E + 2 * nc * E + 2 * nc * E + 2 * nc * E + 3 * nc * E
+        out["sa_lusgs"] = 2 * ni * E + 2 * nc * 32 + nc * 6 * E + 2 * nc * 2 * E + 2 * nc * E
         out["sa_update"] = nc * (8 + E + 8 + E) + sb
     out["iteration"] = sum(out.values())
     return out

@@ -1775,6 +1775,7 @@ int phx_swap_geometry(phx_ctx *ctx, int64_t n, const int32_t *bfaces, const doub
         for (int fs = 0; fs < nf; ++fs) vflag[fs] = vref[ctx->forder[fs]];
         PHX_CUDA(ctx, cudaMemcpy(const_cast<uint8_t *>(ctx->g.vflag), vflag.data(), nf, cudaMemcpyHostToDevice));
     }
+    PHX_CUDA(ctx, cudaStreamSynchronize(nullptr));   // the copies above, before a kernel on the context's stream
     if (ctx->mixed) launch_face_geometry<float>(ctx->g, ctx->nc, ctx->w32, ctx->stream);
     else launch_face_geometry<double>(ctx->g, ctx->nc, ctx->w64, ctx->stream);
     if (const int rc = check_launch(ctx)) return rc;

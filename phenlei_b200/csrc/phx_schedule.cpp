@@ -11,9 +11,11 @@
 // one row a chain kept, the 1M-cell bump's warps read their own results through
 // L2, and its sweeps took 754 and 537 us, NS and SA, instead of 608 and 441).
 // A chain that begins joins the warp of its nearest neighbour in the numbering,
-// or the warp that this one's chains spill into, where the distance is like that
-// of the chains already there (on the same mesh: eight pencils next to one
-// another in j, none from another plane), so that warps mostly depend on one
+// or the warp that this one's chains spill into, where the distance is at most 1.5
+// times that of the chains already there (on the same mesh: eight pencils next to
+// one another in j, none from another plane; at twice the distance the prism
+// layers' warps mix and the backward sweep of the 1M-cell bump takes 318 us
+// instead of 245, below 1.5 grown numberings fill their warps half), so that warps mostly depend on one
 // another in one direction: a warp that has fallen behind the ones it reads from
 // finds their results already there and runs at the speed of its arithmetic.
 // The latency between SMs is then paid once per warp boundary on the way through
@@ -116,7 +118,7 @@ SweepRows build_sweep(const SweepGraph &g, bool forward, int maxWarps)
                 for (int j = noff[c]; j < noff[c + 1]; ++j)
                     if (near < 0 || std::abs(nbr[j] - c) < std::abs(near - c)) near = nbr[j];
                 const int d = near < 0 ? 0 : std::abs(near - c), from = near < 0 ? -1 : slot[near] / kSweepSlots;
-                const bool like = from < 0 || reach[from] == 0 || d <= 2 * reach[from];
+                const bool like = from < 0 || reach[from] == 0 || 2LL * d <= 3LL * reach[from];
                 if (like && from >= 0) {
                     s = free_slot(from, l);
                     if (s >= 0 && reach[from] == 0) reach[from] = d;
@@ -144,13 +146,12 @@ SweepRows build_sweep(const SweepGraph &g, bool forward, int maxWarps)
         }
     }
 
-    // rows: chain warp v runs on warp v % nWarps; a warp's shared memory holds the
-    // results of its last kSweepLocal rows
-    const int nv = (int)spill.size(), nw = std::max(1, std::min(maxWarps, nv));
-    out.nWarps = nw;
     auto parts = [&](int c) { return std::max(1, (noff[c + 1] - noff[c] + kSweepLanes - 1) / kSweepLanes); };
-    for (int l = 0; l < nlev; ++l)   // the cells of a level by chain warp
-        std::sort(cells.begin() + loff[l], cells.begin() + loff[l + 1], [&](int a, int b) { return slot[a] < slot[b]; });
+    // the cells of a level by chain warp
+    auto order = [&]() {
+        for (int l = 0; l < nlev; ++l)
+            std::sort(cells.begin() + loff[l], cells.begin() + loff[l + 1], [&](int a, int b) { return slot[a] < slot[b]; });
+    };
     // calls fn(chain warp, first, last, rows) for every chain warp with cells at a level, in the order of the levels
     auto groups = [&](auto &&fn) {
         for (int l = 0; l < nlev; ++l)
@@ -162,6 +163,31 @@ SweepRows build_sweep(const SweepGraph &g, bool forward, int maxWarps)
                 fn(v, a, b, need);
             }
     };
+    order();
+    size_t rows = 0;
+    groups([&](int, int, int, int need) { rows += need; });
+    if (rows * kSweepSlots > 2 * (size_t)nc) {
+        // a numbering without chains to follow would leave more than half of the
+        // slots idle: full rows of each level instead, dealt out over the warps
+        // (524k hexahedra numbered at random, both sweeps, mixed: 130 us, 313 with
+        // every cell in its storage place; modelled, chains take as long there and
+        // move four times the rows)
+        spill.clear();
+        for (int l = 0; l < nlev; ++l) {
+            std::sort(cells.begin() + loff[l], cells.begin() + loff[l + 1],
+                      [&](int a, int b) { return parts(a) != parts(b) ? parts(a) > parts(b) : a < b; });
+            for (int i = loff[l]; i < loff[l + 1]; ++i) {
+                if ((i - loff[l]) % kSweepSlots == 0) spill.push_back(-1);
+                slot[cells[i]] = ((int)spill.size() - 1) * kSweepSlots + (i - loff[l]) % kSweepSlots;
+            }
+        }
+        order();
+    }
+
+    // rows: chain warp v runs on warp v % nWarps; a warp's shared memory holds the
+    // results of its last kSweepLocal rows
+    const int nv = (int)spill.size(), nw = std::max(1, std::min(maxWarps, nv));
+    out.nWarps = nw;
     out.rowOff.assign(nw + 1, 0);
     groups([&](int v, int, int, int need) { out.rowOff[v % nw + 1] += need; });
     for (int w = 0; w < nw; ++w) out.rowOff[w + 1] += out.rowOff[w];
