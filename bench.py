@@ -180,14 +180,6 @@ def measured_peaks():
     return 6650.0, "fallback"
 
 
-# DRAM bytes per cell of one launch of a sweep kernel, mixed precision:
-# dram__bytes_read.sum + dram__bytes_write.sum of one ncu --set full capture
-# of lusgs_kernel<float> on the 0.999M-cell SA bump (940.16 MB + 95.03 MB).
-# Both sweeps read every cell's records once, so a launch's traffic at
-# another mesh size is this figure times the cells.
-MEASURED_TRAFFIC_PER_CELL = {("lusgs", "mixed"): (940.16e6 + 95.03e6) / 999424}
-
-
 def kernel_bytes(m, precision: str, viscous: int = 0, gradient: str = "ggcell") -> dict:
     """Algorithmic bytes per launch of each phase under the compulsory-byte rule
     (each array element counted once per pass that reads or writes it; cell
@@ -890,8 +882,6 @@ def main():
     phase = r["phase_ms"]
     dom = max(phase, key=phase.get)
     achieved = kb[dom] / (phase[dom] / 1e3) / 1e9
-    tpc = MEASURED_TRAFFIC_PER_CELL.get((dom, args.precision))
-    traffic = round(tpc * nc) if tpc else None
     line = {
         "metric": METRIC, "value": round(value, 3), "unit": "Mcell-iters/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(ms / args.steps, 4),
@@ -905,7 +895,7 @@ def main():
         "phase_ms": {k: round(v, 4) for k, v in phase.items()},
         "roofline": {"kernel": dom, "bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "peak_kind": peak_kind,
-                     "algorithmic_bytes": kb[dom], "traffic": traffic},
+                     "algorithmic_bytes": kb[dom], "traffic": None},
         "iteration_bytes": kb["iteration"],
         "iteration_roofline_frac": round(kb["iteration"] / (ms / args.steps / 1e3) / 1e9 / peak, 4),
         # the same over the minimal pass structure's compulsory bytes (no records of this implementation)

@@ -904,7 +904,7 @@ __global__ void __launch_bounds__(kThreads) sweep_ghost_kernel(DevGrid g, NsCons
 // cell passes or by the schedule, and a row arrives by one copy.
 // Both sweeps, mixed, against levels dealt out over all SMs with every result
 // through L2: 8k hexahedra 170 -> 106 us, the 200k plate 515 -> 256 us, 1M
-// tetrahedra 960 -> 592 us, the 1M-cell bump with prisms 978 -> 608 us.
+// tetrahedra 960 -> 590 us, the 1M-cell bump with prisms 978 -> 537 us.
 // Shared memory in front of the stages: the warp's results and a zero, barriers.
 template <class T>
 constexpr int kSweepHead = (kSweepZero + 1) * 8 * (int)sizeof(T) + (sizeof(T) == 4 ? 96 : 64);

@@ -395,7 +395,7 @@ void launch_sa_residual(const DevGrid &g, const NsConst &c, const double *q64, c
 // ---------------------------------------------------------------------------
 // Bound by the chain of rows as the NS sweep (0.23 us a row); a row is small, so
 // 16 of them are in flight.  Both sweeps, mixed, against levels dealt out over
-// all SMs: the 200k plate 400 -> 202 us, the 1M-cell bump 779 -> 441 us.
+// all SMs: the 200k plate 400 -> 202 us, the 1M-cell bump 779 -> 400 us.
 static constexpr int kSaStages = 8;
 
 template <class T, bool kForward>
