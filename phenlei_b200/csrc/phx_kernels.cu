@@ -566,8 +566,7 @@ __device__ __forceinline__ void reset_reduce(Reduce *r)
 // spectral-radius term, which is also the LU-SGS viscous factor of both face uses
 // (SpectrumRadiusViscous method 2, NSSolverUnstruct.cpp:5930-5960;
 // SolveLUSGSForward :15339-15357): GetVisFaceValue (:7126-7375, static adiabatic
-// walls: the mean of a wall's two sides is at rest) and ComputeVisflux
-// (:12977-13378, perfect gas).  The face gradient F of u, v, w has its normal part
+// walls) and ComputeVisflux (:12977-13378, perfect gas).  The face gradient F of u, v, w has its normal part
 // replaced by the normal derivative; what ComputeVisflux takes along two tangents
 // is F less its normal part.
 //
@@ -616,10 +615,13 @@ __global__ void __launch_bounds__(kPassThreads<T>, 3) face_flux_kernel(DevGrid g
             const T mut = w.trec ? T(0.5) * (w.trec[(size_t)le * kTr + 1] + w.trec[(size_t)re * kTr + 1]) : T(0);
             const T vis = mul + mut;
             vspec = T(2) * vis / (T(0.5) * (qL[0] + qR[0]) * ds * (T)c.reynolds + (T)kSmall) * (T(0.5) * area);
+            // a wall's face velocity is zero whatever its ghost holds (GetVisFaceValue), where both
+            // centres are projected; elsewhere ComputeVisflux takes the mean
+            const bool rest = f < g.nBFace && g.bkind[f] == BK_WALL && (g.vflag[f] & 1);
             T fm[3];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                fm[k] = T(0.5) * (qL[k + 1] + qR[k + 1]);
+                fm[k] = rest ? T(0) : T(0.5) * (qL[k + 1] + qR[k + 1]);
                 const T dn = A * (f1[k] - fm[k]) + B * (f2[k] - fm[k]);
                 const T dt = dn - (F[3 * k] * xn + F[3 * k + 1] * yn + F[3 * k + 2] * zn);
                 F[3 * k] += xn * dt; F[3 * k + 1] += yn * dt; F[3 * k + 2] += zn * dt;
