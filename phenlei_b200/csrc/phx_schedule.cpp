@@ -164,14 +164,23 @@ SweepRows build_sweep(const SweepGraph &g, bool forward, int maxWarps)
             }
     };
     order();
+    // Where a numbering has no chains to follow they leave most slots idle, and the
+    // warps run many more rows than there are levels: full rows of each level then,
+    // dealt out over the warps.  Both have to hold.  With at most about a row a level
+    // on the longest warp, idle slots cost nothing: each level then takes a row's
+    // time, and dealt out a hop through L2 as well.  Both NS sweeps, mixed, chains
+    // against dealt-out rows, with rows of the longest warp a level:
+    //   ducts of 4000x1x1 (1.0) 2489 and 3723 us, 200x3x2 (1.0) 159 and 217,
+    //   300x4x4 (1.0) 231 and 334, a block of 16x8x2 (1.0) 40 and 49;
+    //   numbered at random: 8k hexahedra (1.6) 43 and 49, 48k tetrahedra (1.2) 42
+    //   and 44, 162k tetrahedra (2.3) 65 and 56, 524k hexahedra (8) 249 and 124;
+    //   66k hexahedra, FP64: forward (1.9) 54 and 45, backward (1.7) 42 and 42.
+    const int chainWarps = std::max(1, std::min(maxWarps, (int)spill.size()));
+    std::vector<int> warpRows(chainWarps, 0);
     size_t rows = 0;
-    groups([&](int, int, int, int need) { rows += need; });
-    if (rows * kSweepSlots > 2 * (size_t)nc) {
-        // a numbering without chains to follow would leave more than half of the
-        // slots idle: full rows of each level instead, dealt out over the warps
-        // (524k hexahedra numbered at random, both sweeps, mixed: 130 us, 313 with
-        // every cell in its storage place; modelled, chains take as long there and
-        // move four times the rows)
+    groups([&](int v, int, int, int need) { rows += need; warpRows[v % chainWarps] += need; });
+    const int longest = *std::max_element(warpRows.begin(), warpRows.end());
+    if (rows * kSweepSlots > 2 * (size_t)nc && 4LL * longest > 7LL * nlev) {
         spill.clear();
         for (int l = 0; l < nlev; ++l) {
             std::sort(cells.begin() + loff[l], cells.begin() + loff[l + 1],

@@ -2,6 +2,7 @@
 // warps take turns, one row at a time, a row runs when its polled neighbours are
 // done, and the shared-memory slots are kept as the kernels keep them.  Returns
 // 0, or the number of the first rule that does not hold.
+#include <algorithm>
 #include <vector>
 
 #include "../phenlei_b200/csrc/phx_internal.h"
@@ -72,4 +73,22 @@ extern "C" int replay(int nc, int nb, const int *off, const int *c2f, const int 
         if (done[c] != 1 || seen[c] != n) return 10;
     }
     return 0;
+}
+
+// Rows of the schedule, warps, rows of the longest warp, and the share of the neighbours
+// that a warp's shared memory holds.
+extern "C" void shape(int nc, int nb, const int *off, const int *c2f, const int *left, const int *right, int forward,
+                      int maxWarps, double *out)
+{
+    using namespace phx;
+    const SweepRows s = build_sweep(SweepGraph{nc, nb, off, c2f, left, right}, forward != 0, maxWarps);
+    int longest = 0;
+    for (int w = 0; w < s.nWarps; ++w) longest = std::max(longest, s.rowOff[w + 1] - s.rowOff[w]);
+    long long held = 0, all = 0;
+    for (size_t e = 0; e < s.ent.size(); ++e)
+        if (s.ent[e] >= 0) { ++all; held += s.loc[e] >= 0; }
+    out[0] = s.rowOff[s.nWarps];
+    out[1] = s.nWarps;
+    out[2] = longest;
+    out[3] = all ? (double)held / all : 1.0;
 }
