@@ -71,7 +71,11 @@ struct phx_ctx {
     double *forces = nullptr;               // [16] wall force sums
     Reduce *red = nullptr;
     int *neglist = nullptr;
-    double *tmp = nullptr;                // [5][nTotal] staging buffer in the reference's order
+    // Memory of what lives within one call only, so that they share it: the face
+    // fluxes (phx_ns_residual), the SA face terms (phx_sa_residual), and tmp, the
+    // [5][nTotal] staging buffer in the reference's order (state I/O)
+    unsigned char *scratch = nullptr;
+    double *tmp = nullptr;
     double *hist = nullptr;
     int histCap = 0;
     unsigned char *result = nullptr;      // pinned: Reduce, residual history of a phx_ns_relaxation call
@@ -708,13 +712,13 @@ int make_rows(phx_ctx *ctx, unsigned char **rows, int which, size_t bytes)
 template <class T>
 int make_turb(phx_ctx *ctx, Work<T> &w, TurbWork<T> &t)
 {
-    const size_t nt = ctx->nTotal, nc = ctx->nCell, nf = ctx->nFace;
+    const size_t nt = ctx->nTotal, nc = ctx->nCell;
     int r = 0;
     r |= dalloc(ctx, &w.trec, nt * kTr);
     r |= dalloc(ctx, &t.qt64, nt);
     r |= dalloc(ctx, &t.tgrad, nc * kTg);
     r |= dalloc(ctx, &t.tcrec, nc * kTc);
-    r |= dalloc(ctx, &t.tface, nf * kTf);
+    t.tface = reinterpret_cast<T *>(ctx->scratch);
     r |= make_rows(ctx, &t.trowf, 0, kRowSa<T>);
     r |= make_rows(ctx, &t.trowb, 1, kRowSa<T>);
     r |= dalloc(ctx, &t.tdq, (size_t)ctx->g.bwd.nRows * kSweepSlots);
@@ -751,7 +755,7 @@ int make_work(phx_ctx *ctx, Work<T> &w, const std::vector<double> &limInit)
     r |= dalloc(ctx, &w.fnrm, nf * kNrm);
     r |= dalloc(ctx, &w.fgeo, nf * (ctx->prm.viscousType ? kGeo<true> : kGeo<false>));
     if (ctx->sa) r |= dalloc(ctx, &w.fsa, nf * kGeoSa);
-    r |= dalloc(ctx, &w.flux, nf * kFlux);
+    w.flux = reinterpret_cast<T *>(ctx->scratch);
     r |= dalloc(ctx, &w.coef, (size_t)ctx->nBFace * kUse);
     r |= make_rows(ctx, &w.rowf, 0, kRowNs<T, true>);
     r |= make_rows(ctx, &w.rowb, 1, kRowNs<T, false>);
@@ -1075,14 +1079,13 @@ int phx_ctx_create(const phx_grid_desc *gd, const phx_params *prm, phx_ctx **out
         skew[i] = ctx->geom[11][ord[i]];
         volpow[i] = std::pow(std::pow(ctx->geom[10][ord[i]], 1.0 / 3.0), 3.0);
     }
-    std::vector<int> sc2f_off(nc + 1, 0), sc2f(c2f.size());
+    std::vector<int> sc2f_off(nc + 1, 0);
     std::vector<int2> sc2x(c2f.size());
     for (int i = 0; i < nc; ++i) sc2f_off[i + 1] = sc2f_off[i] + (c2f_off[ord[i] + 1] - c2f_off[ord[i]]);
     for (int i = 0; i < nc; ++i) {
         const int c = ord[i];
         for (int j = c2f_off[c], k = sc2f_off[i]; j < c2f_off[c + 1]; ++j, ++k) {
             const int f = fpos[c2f[j]];
-            sc2f[k] = f;
             sc2x[k] = lr[f].x == i ? make_int2(f, lr[f].y) : make_int2(~f, lr[f].x);
         }
     }
@@ -1153,7 +1156,6 @@ int phx_ctx_create(const phx_grid_desc *gd, const phx_params *prm, phx_ctx **out
     rc |= upload(ctx, &g.skew, skew);
     rc |= upload(ctx, &g.volpow, volpow);
     rc |= upload(ctx, &g.c2f_off, sc2f_off);
-    rc |= upload(ctx, &g.c2f, sc2f);
     rc |= upload(ctx, &g.c2x, sc2x);
     rc |= upload(ctx, &g.orig, origv);
     rc |= upload(ctx, &g.bkind, bkind);
@@ -1190,7 +1192,10 @@ int phx_ctx_create(const phx_grid_desc *gd, const phx_params *prm, phx_ctx **out
     rc |= upload(ctx, &g.ghost_cell, ghostCell);
     rc |= dalloc(ctx, &ctx->q64[0], (size_t)5 * nt);
     rc |= dalloc(ctx, &ctx->q64[1], (size_t)5 * nt);
-    rc |= dalloc(ctx, &ctx->tmp, (size_t)5 * nt);
+    static_assert(kFlux >= kTf, "the scratch holds the SA face terms");
+    rc |= dalloc(ctx, &ctx->scratch,
+                 std::max((size_t)nf * kFlux * (ctx->mixed ? sizeof(float) : sizeof(double)), sizeof(double) * 5 * (size_t)nt));
+    ctx->tmp = reinterpret_cast<double *>(ctx->scratch);
     rc |= dalloc(ctx, &ctx->red, 1);
     rc |= dalloc(ctx, &ctx->neglist, 1 << 16);
     if (!rc) rc = ctx->mixed ? make_work(ctx, ctx->w32, limInit) : make_work(ctx, ctx->w64, limInit);

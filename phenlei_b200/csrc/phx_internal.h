@@ -123,8 +123,8 @@ struct DevGrid {
     // |dL|, |dR| > TINY (the SA diffusion's normal derivative); pure geometry,
     // decided on the host
     const uint8_t *vflag;
-    const int *c2f_off, *c2f;    // faces of each cell, ordered by the reference face number
-    const int2 *c2x;             // and alike {face, ~ it where the cell is the right cell; cell or ghost behind it}
+    const int *c2f_off;          // faces of each cell, ordered by the reference face number:
+    const int2 *c2x;             // {face, ~ it where the cell is the right cell; cell or ghost behind it}
     const int *orig;             // [nTotal] reference number of each cell (ghost: nCell + reference face)
     const int32_t *bkind;        // [nBFace] BcKind
     const int32_t *btype;        // [nBFace] bcType
@@ -192,7 +192,7 @@ struct Work {
     T *fnrm, *fgeo; // [nFace][kNrm], [nFace][kGeo] face geometry
     T *fsa;         // [nFace][kGeoSa] SA face geometry (SA runs; else null)
     T *grec;        // [nTotal][kG] primitive gradients (ghost rows: interface ghosts only, from the halo exchange)
-    T *flux;        // [nFace][kFlux] face flux times area and inviscid spectral radius term
+    T *flux;        // [nFace][kFlux] face flux times area and inviscid spectral radius term (in the scratch)
     T *coef;        // [nBFace][kUse] LU-SGS factors of the boundary faces' uses
     unsigned char *rowf, *rowb;   // [rows][kRowNs] LU-SGS rows of the forward and the backward sweep
     T *crec;        // [nCell][kC] residual, diagonal, spectral radii
@@ -212,7 +212,7 @@ struct TurbWork {
     double *qt64;   // [nTotal] master nu~
     T *tgrad;       // [nCell][kTg] gradient of nu~
     T *tcrec;       // [nCell][kTc] residual, spectral radius, its reciprocal, pad
-    T *tface;       // [nFace][kTf] face terms
+    T *tface;       // [nFace][kTf] face terms (in the scratch)
     unsigned char *trowf, *trowb;   // [rows][kRowSa] LU-SGS rows
     T *tdq;         // [backward rows][kSweepSlots] LU-SGS dq (write-once per sweep, by slot as the NS records)
     T *tdqf;        // [forward rows][kSweepSlots] forward-sweep dq

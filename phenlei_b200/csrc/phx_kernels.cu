@@ -880,8 +880,8 @@ __global__ void __launch_bounds__(kThreads) sweep_ghost_kernel(DevGrid g, NsCons
     ld8(w.dqfwd + (size_t)ld(g.lead + cell) * kD, dl);
     const int j1 = ld(g.c2f_off + cell + 1);
     for (int j = ld(g.c2f_off + cell); j < j1; ++j) {
-        const int f = ld(g.c2f + j);
-        if (f >= g.nBFace) break;
+        const int f = ld(&g.c2x[j].x);   // a boundary face's only cell is its left cell
+        if (f < 0 || f >= g.nBFace) break;
         const int kind = ld(g.bkind + f), ghost = g.nCell + f;
         double fr[4];
         ld4(g.frec + (size_t)f * kF, fr);
@@ -1268,9 +1268,7 @@ __global__ void __launch_bounds__(kFixThreads) solution_fix_kernel(DevGrid g, Ns
         const int oc = key[i];
         double acc[5] = {0, 0, 0, 0, 0}, wsum = 0.0;
         for (int j = g.c2f_off[cell]; j < g.c2f_off[cell + 1]; ++j) {
-            const int f = g.c2f[j];
-            const int2 lr = g.lr[f];
-            const int nb = (cell == lr.x) ? lr.y : lr.x;
+            const int nb = g.c2x[j].y;
             const double *src = (g.orig[nb] < oc) ? qn : qo;
             if (src[nb] < rlim || src[4 * nt + nb] < plim) continue;
             wsum += 1.0;
