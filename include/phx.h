@@ -165,7 +165,11 @@ void phx_default_params(phx_params *p);
  * level schedules, and initialises the state to the free stream.
  * Replaces: Simulation::RunCFD grid set-up (Main/src/Simulation.cpp:205-260),
  * UnstructGrid::ComputeMetrics (API/Geometry/src/Geo_UnstructGrid.cpp:5695),
- * NSSolverUnstruct::AllocateGlobalVar / InitFlow, GPUGeomInfoAllocCopy. */
+ * NSSolverUnstruct::AllocateGlobalVar / InitFlow, GPUGeomInfoAllocCopy.
+ * A context that would leave less than two thirds of the device's memory free
+ * keeps neither face geometry nor the sweeps' factors, and forms them where
+ * they are used: the same results, a smaller context, a slower step
+ * (PHX_LAYOUT=full or compact in the environment takes the one or the other). */
 int phx_ctx_create(const phx_grid_desc *grid, const phx_params *params, phx_ctx **out);
 int phx_ctx_destroy(phx_ctx *ctx);
 const char *phx_last_error(const phx_ctx *ctx);

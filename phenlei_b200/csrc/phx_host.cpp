@@ -84,7 +84,10 @@ struct phx_ctx {
     int step = 0;
     bool haveResidual = false;
     std::vector<int> rankOf;              // storage index of each reference cell
-    std::vector<int> sweepRows[2];        // schedule rows of the LU-SGS sweeps, until the row arrays hold them
+    // schedule rows of the LU-SGS sweeps, and the lanes of the faces' uses (DevGrid::use), until the row
+    // arrays hold them
+    std::vector<int> sweepRows[2], sweepRowOff[2];
+    std::vector<int2> sweepUse;
     // partitioned grids (interface faces): the topology and storage maps that
     // phx_swap_geometry needs to form the weights again, and the halo plan
     bool hasInterface = false;
@@ -693,9 +696,9 @@ int make_visc(phx_ctx *ctx, Work<T> &w)
 }
 
 // The rows of one LU-SGS sweep, `bytes` each: zeros (lanes without an entry and
-// the boundary part of cells without boundary faces stay so) and, at the end of
-// each, the schedule row.
-int make_rows(phx_ctx *ctx, unsigned char **rows, int which, size_t bytes)
+// the boundary part of cells without boundary faces stay so; compact: the lanes'
+// uses and cells) and, at the end of each, the schedule row.
+int make_rows(phx_ctx *ctx, unsigned char **rows, int which, size_t bytes, const std::vector<int> *uses = nullptr)
 {
     const std::vector<int> &src = ctx->sweepRows[which];
     const size_t n = src.size() / kSweepRow, part = kSweepRow * sizeof(int);
@@ -703,6 +706,10 @@ int make_rows(phx_ctx *ctx, unsigned char **rows, int which, size_t bytes)
     if (r) return r;
     PHX_CUDA(ctx, cudaMemset(*rows, 0, n * bytes));
     PHX_CUDA(ctx, cudaMemcpy2D(*rows + bytes - part, bytes, src.data(), part, part, n, cudaMemcpyHostToDevice));
+    if (uses) {
+        const size_t ub = bytes - part;
+        PHX_CUDA(ctx, cudaMemcpy2D(*rows, bytes, uses->data(), ub, ub, n, cudaMemcpyHostToDevice));
+    }
     return PHX_OK;
 }
 
@@ -719,8 +726,6 @@ int make_turb(phx_ctx *ctx, Work<T> &w, TurbWork<T> &t)
     r |= dalloc(ctx, &t.tgrad, nc * kTg);
     r |= dalloc(ctx, &t.tcrec, nc * kTc);
     t.tface = reinterpret_cast<T *>(ctx->scratch);
-    r |= make_rows(ctx, &t.trowf, 0, kRowSa<T>);
-    r |= make_rows(ctx, &t.trowb, 1, kRowSa<T>);
     r |= dalloc(ctx, &t.tdq, (size_t)ctx->g.bwd.nRows * kSweepSlots);
     r |= dalloc(ctx, &t.tdqf, (size_t)ctx->g.fwd.nRows * kSweepSlots);
     r |= dalloc(ctx, &t.tsrc, nc);
@@ -748,17 +753,12 @@ int make_turb(phx_ctx *ctx, Work<T> &w, TurbWork<T> &t)
 template <class T>
 int make_work(phx_ctx *ctx, Work<T> &w, const std::vector<double> &limInit)
 {
-    const size_t nt = ctx->nTotal, nc = ctx->nCell, nf = ctx->nFace;
+    const size_t nt = ctx->nTotal, nc = ctx->nCell;
     int r = 0;
     r |= dalloc(ctx, &w.qrec, nt * kQ);
     r |= dalloc(ctx, &w.grec, nt * kG);
-    r |= dalloc(ctx, &w.fnrm, nf * kNrm);
-    r |= dalloc(ctx, &w.fgeo, nf * (ctx->prm.viscousType ? kGeo<true> : kGeo<false>));
-    if (ctx->sa) r |= dalloc(ctx, &w.fsa, nf * kGeoSa);
     w.flux = reinterpret_cast<T *>(ctx->scratch);
     r |= dalloc(ctx, &w.coef, (size_t)ctx->nBFace * kUse);
-    r |= make_rows(ctx, &w.rowf, 0, kRowNs<T, true>);
-    r |= make_rows(ctx, &w.rowb, 1, kRowNs<T, false>);
     r |= dalloc(ctx, &w.crec, nc * kC);
     r |= dalloc(ctx, &w.dtraw, nc);
     const size_t nf8 = (size_t)ctx->g.fwd.nRows * kSweepSlots * kD, nb8 = (size_t)ctx->g.bwd.nRows * kSweepSlots * kD;
@@ -776,9 +776,91 @@ int make_work(phx_ctx *ctx, Work<T> &w, const std::vector<double> &limInit)
     PHX_CUDA(ctx, cudaMemset(w.dqghost, 0, sizeof(T) * (size_t)ctx->nBFace * kD));   // until the first exchange
     PHX_CUDA(ctx, cudaMemset(w.grec, 0, sizeof(T) * nt * kG));
     PHX_CUDA(ctx, cudaMemset(w.crec, 0, sizeof(T) * nc * kC));
-    launch_face_geometry<T>(ctx->g, ctx->nc, w, ctx->stream);
-    PHX_CUDA(ctx, cudaGetLastError());
     return PHX_OK;
+}
+
+// Face geometry and LU-SGS rows, the last of a context's arrays.  Both in full make
+// a context of an SA run on hexahedra 1.9 kB a cell in mixed precision and 3.2 kB in
+// FP64; in the compact layout it is 1.2 and 1.7 kB.  A step is slower so (16M-cell
+// bump, mixed: 18.1 ms instead of 13.2), so the layout is compact only where the full
+// one would leave less than two thirds of the device's memory free: beyond 33M cells
+// (mixed; 19M in FP64), or for the last of many contexts (the zones of a partition),
+// which would not all fit in full.  PHX_LAYOUT=full or compact in the environment
+// takes that layout.
+template <class T>
+int make_layout(phx_ctx *ctx, Work<T> &w, TurbWork<T> &t, const std::vector<int2> &lr)
+{
+    const size_t nc = ctx->nCell, nf = ctx->nFace, rf = ctx->g.fwd.nRows, rb = ctx->g.bwd.nRows;
+    const size_t perFace = ctx->prm.viscousType ? kGeo<true> : kGeo<false>;
+    const size_t bytes = sizeof(T) * nf * (kNrm + perFace + (ctx->sa ? kGeoSa : 0)) + sizeof(int2) * nf +
+                         rf * (kRowNs<T, true> + (ctx->sa ? kRowSa<T> : 0)) +
+                         rb * (kRowNs<T, false> + (ctx->sa ? kRowSa<T> : 0));
+    size_t avail = 0, total = 0;
+    PHX_CUDA(ctx, cudaMemGetInfo(&avail, &total));
+    ctx->g.compact = bytes + total / 3 * 2 > avail;
+    if (const char *e = getenv("PHX_LAYOUT")) {
+        if (std::strcmp(e, "full") == 0) ctx->g.compact = 0;
+        if (std::strcmp(e, "compact") == 0) ctx->g.compact = 1;
+    }
+    int r = 0;
+    if (!ctx->g.compact) {
+        r |= upload(ctx, &ctx->g.use, ctx->sweepUse);
+        r |= dalloc(ctx, &w.fnrm, nf * kNrm);
+        r |= dalloc(ctx, &w.fgeo, nf * perFace);
+        if (ctx->sa) r |= dalloc(ctx, &w.fsa, nf * kGeoSa);
+        r |= make_rows(ctx, &w.rowf, 0, kRowNs<T, true>);
+        r |= make_rows(ctx, &w.rowb, 1, kRowNs<T, false>);
+        if (ctx->sa) {
+            r |= make_rows(ctx, &t.trowf, 0, kRowSa<T>);
+            r |= make_rows(ctx, &t.trowb, 1, kRowSa<T>);
+        }
+        if (r) return r;
+        launch_face_geometry<T>(ctx->g, ctx->nc, w, ctx->stream);
+        PHX_CUDA(ctx, cudaGetLastError());
+        return PHX_OK;
+    }
+    for (int which = 0; which < 2; ++which) {
+        // uses and cells of every row, kLine words; row i of a warp holds those of its row i + 2
+        constexpr int kLine = 32 * 2 + kSweepSlots;
+        SweepDev &sw = which == 0 ? ctx->g.fwd : ctx->g.bwd;
+        const std::vector<int> &sched = ctx->sweepRows[which];
+        std::vector<int> all((size_t)sw.nRows * kLine, -1), ahead((size_t)sw.nRows * kLine, -1);
+        for (size_t f = ctx->nBFace; f < nf; ++f)
+            for (int side = 0; side < 2; ++side) {
+                int at = side == 0 ? ctx->sweepUse[f].x : ctx->sweepUse[f].y;
+                if ((at < 0) != (which == 1)) continue;
+                if (at < 0) at = ~at;
+                int *u = &all[(size_t)(at >> 5) * kLine + (at & 31) * 2];
+                u[0] = (int)((unsigned)f | (side == 0 ? 0u : 0x80000000u));
+                u[1] = side == 0 ? lr[f].y : lr[f].x;
+            }
+        for (size_t i = 0; i < (size_t)sw.nRows; ++i)
+            for (int k = 0; k < kSweepSlots; ++k) all[i * kLine + 64 + k] = sched[i * kSweepRow + 32 + k * 4];
+        std::vector<int2> fu((size_t)sw.nWarps * 64, make_int2(0, -1));
+        std::vector<int> fc((size_t)sw.nWarps * 16, -1);
+        for (int v = 0; v < sw.nWarps; ++v)
+            for (int i = ctx->sweepRowOff[which][v]; i < ctx->sweepRowOff[which][v + 1]; ++i) {
+                const int k = i - ctx->sweepRowOff[which][v];
+                const int *u = &all[(size_t)i * kLine];
+                if (k >= 2) {
+                    std::copy(u, u + kLine, &ahead[(size_t)(i - 2) * kLine]);
+                    continue;
+                }
+                for (int t2 = 0; t2 < 32; ++t2) fu[(size_t)v * 64 + k * 32 + t2] = make_int2(u[2 * t2], u[2 * t2 + 1]);
+                for (int q = 0; q < kSweepSlots; ++q) fc[(size_t)v * 16 + k * 8 + q] = u[64 + q];
+            }
+        r |= upload(ctx, &sw.first_use, fu);
+        r |= upload(ctx, &sw.first_cell, fc);
+        r |= make_rows(ctx, which == 0 ? &w.rowf : &w.rowb, which, kRowCompact, &ahead);
+        if (r) return r;
+    }
+    t.trowf = w.rowf;
+    t.trowb = w.rowb;
+    r |= dalloc(ctx, &w.frad, nf * 2);
+    r |= dalloc(ctx, &w.lead, nc * kLeadF);
+    r |= dalloc(ctx, &w.gsum, (size_t)ctx->g.nGhostCell * kLeadF);
+    if (ctx->sa) r |= dalloc(ctx, &t.tmat, nf * 2);
+    return r;
 }
 
 }  // namespace
@@ -1017,7 +1099,11 @@ int phx_ctx_create(const phx_grid_desc *gd, const phx_params *prm, phx_ctx **out
         std::vector<uint8_t> has(nc, 0);
         for (int f = 0; f < nb; ++f) has[h.left[f]] = 1;
         for (int i = 0; i < nc; ++i)
-            if (has[ord[i]]) ghostCell.push_back(make_int2(i, sweep[1].first[ord[i]]));
+            if (has[ord[i]]) {
+                const int at = sweep[1].first[ord[i]];
+                ghostCell.push_back(make_int2(i, at));
+                sweep[1].row[(size_t)(at / kSweepSlots) * kSweepRow + 32 + at % kSweepSlots * 4 + 3] = (int)ghostCell.size();
+            }
     }
 
     // boundary classification (storage face order)
@@ -1185,8 +1271,9 @@ int phx_ctx_create(const phx_grid_desc *gd, const phx_params *prm, phx_ctx **out
         rc |= upload(ctx, &d.row_off, sweep[i].rowOff);
         rc |= upload(ctx, &d.first, sweep[i].start);
         ctx->sweepRows[i] = std::move(sweep[i].row);
+        ctx->sweepRowOff[i] = std::move(sweep[i].rowOff);
     }
-    rc |= upload(ctx, &g.use, use);
+    ctx->sweepUse = std::move(use);
     rc |= upload(ctx, &g.lead, lead);
     rc |= upload(ctx, &g.last, last);
     rc |= upload(ctx, &g.ghost_cell, ghostCell);
@@ -1201,8 +1288,13 @@ int phx_ctx_create(const phx_grid_desc *gd, const phx_params *prm, phx_ctx **out
     if (!rc) rc = ctx->mixed ? make_work(ctx, ctx->w32, limInit) : make_work(ctx, ctx->w64, limInit);
     if (!rc && ctx->sa) rc = ctx->mixed ? make_turb(ctx, ctx->w32, ctx->t32) : make_turb(ctx, ctx->w64, ctx->t64);
     else if (!rc && prm->viscousType) rc = ctx->mixed ? make_visc(ctx, ctx->w32) : make_visc(ctx, ctx->w64);
-    for (auto &v : ctx->sweepRows) std::vector<int>().swap(v);
     if (!rc) rc = dalloc(ctx, &ctx->forces, 16);
+    if (!rc) rc = ctx->mixed ? make_layout(ctx, ctx->w32, ctx->t32, lr) : make_layout(ctx, ctx->w64, ctx->t64, lr);
+    for (int i = 0; i < 2; ++i) {
+        std::vector<int>().swap(ctx->sweepRows[i]);
+        std::vector<int>().swap(ctx->sweepRowOff[i]);
+    }
+    std::vector<int2>().swap(ctx->sweepUse);
     if (!rc && cudaMemset(ctx->red, 0, sizeof(Reduce)) != cudaSuccess) rc = PHX_ERR_CUDA;
     if (rc) {
         const int code = rc < 0 ? rc : PHX_ERR_CUDA;
@@ -1781,9 +1873,11 @@ int phx_swap_geometry(phx_ctx *ctx, int64_t n, const int32_t *bfaces, const doub
         PHX_CUDA(ctx, cudaMemcpy(const_cast<uint8_t *>(ctx->g.vflag), vflag.data(), nf, cudaMemcpyHostToDevice));
     }
     PHX_CUDA(ctx, cudaStreamSynchronize(nullptr));   // the copies above, before a kernel on the context's stream
-    if (ctx->mixed) launch_face_geometry<float>(ctx->g, ctx->nc, ctx->w32, ctx->stream);
-    else launch_face_geometry<double>(ctx->g, ctx->nc, ctx->w64, ctx->stream);
-    if (const int rc = check_launch(ctx)) return rc;
+    if (!ctx->g.compact) {
+        if (ctx->mixed) launch_face_geometry<float>(ctx->g, ctx->nc, ctx->w32, ctx->stream);
+        else launch_face_geometry<double>(ctx->g, ctx->nc, ctx->w64, ctx->stream);
+        if (const int rc = check_launch(ctx)) return rc;
+    }
     if (avg_vol > 0.0) {
         // the Venkatakrishnan threshold scales with the average cell volume of all zones
         const double K = prm->venkatCoeff;

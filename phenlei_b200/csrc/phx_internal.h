@@ -44,8 +44,8 @@ constexpr int kF = 8;      // frec (FP64): nx ny nz area xfc yfc zfc | least-squ
 constexpr int kX = 4;      // xrec (FP64): xcc ycc zcc vol
 constexpr int kFlux = 12;  // face flux record: inviscid F0..4 (times area) | inviscid and viscous spectral parts |
                            // viscous F1..4 (times area; F0 is zero) | pad
-// Face geometry in the working precision, formed once in FP64 from the metrics
-// (face_geometry_kernel).  fnrm: unit normal times area (least squares: vector
+// Face geometry in the working precision, formed in FP64 from the metrics
+// (phx_geometry.cuh).  fnrm: unit normal times area (least squares: vector
 // from the left to the right centre, weight).  fgeo: unit normal, area | face
 // centre less left centre, left weight of the face gradient | less right centre,
 // A | for viscous runs: left offset, B | right offset, centre distance along the
@@ -76,13 +76,17 @@ constexpr int kSweepFirst = 8, kSweepLast = 16;   // flags of the host schedule:
 // zeros); then per slot {storage cell (-1: idle, or not the cell's last row),
 // shared-memory slot of the result | kSweepMulti (the row holds a cell of several
 // rows) | kSweepCarry (not the cell's first), forward: slot of the cell's last
-// backward row, 0}.
+// backward row; backward, in the first row of a cell with boundary faces: its place
+// in ghost_cell + 1}.
 constexpr int kSweepRow = 64, kSweepZero = kSweepLocal * kSweepSlots;
 constexpr int kSweepMulti = 256, kSweepCarry = 512;
 // Bytes of a row as the sweeps copy it: factors of the lanes' face uses, right-
 // hand sides of the cells, schedule row; NS (both sweeps) and SA.
 template <class T, bool kForward>
 constexpr int kRowNs = (32 * kUse + kSweepSlots * (kForward ? kLeadF : kLeadB)) * (int)sizeof(T) + kSweepRow * 4;
+// Compact layout: of the warp's row after next, the lanes' uses {face, neighbour} and the slots' cells (-1: none, or
+// not the cell's last row); schedule row.
+constexpr int kRowCompact = 32 * 8 + kSweepSlots * 4 + kSweepRow * 4;
 template <class T>
 constexpr int kRowSa = (32 + kSweepSlots * kLeadT) * (int)sizeof(T) + kSweepRow * 4;
 constexpr long long kDefaultSpinLimit = 20000000LL;   // polls per dependency wait (~1-2 s)
@@ -90,10 +94,10 @@ constexpr int kMaxDevices = 64;                       // per-device launch cache
 // Spalart-Allmaras records
 constexpr int kTr = 4;     // trec: nu~ | eddy viscosity | laminar viscosity of the NS step | pad
 constexpr int kTg = 4;     // tgrad: d nu~ / dx, dy, dz | pad
-constexpr int kTc = 4;     // tcrec: res_turb | spec_turb | pad
+constexpr int kTc = 4;     // tcrec: res_turb | spec_turb | its reciprocal | pad (compact: backward right-hand side)
 constexpr int kTf = 4;     // tface: convection and first diffusion flux | second diffusion flux (times the side's own
                            // diffusivity) | spectral terms of the left and of the right cell
-// SA face geometry (working precision, formed once in FP64): unit normal, area |
+// SA face geometry (working precision, formed in FP64): unit normal, area |
 // factor of the difference right less left in the normal derivative | one over
 // the mean volume | pad.
 constexpr int kGeoSa = 8;
@@ -104,10 +108,17 @@ struct SweepDev {
     int nWarps, nRows;
     const int *row_off;
     const int *first;    // [nWarps][2][32] entries of the warp's first two rows
+    const int2 *first_use;    // compact layout: [nWarps][2][32] their uses
+    const int *first_cell;    // compact layout: [nWarps][2][8] and cells
 };
 
 // Read-only device grid (FP64 metrics, connectivity, schedules), storage order.
 struct DevGrid {
+    // 0, full layout: the face geometry is stored, and the LU-SGS rows hold all that the
+    // sweeps need, written by the passes.  1, compact layout (large meshes): the passes
+    // form the geometry, the rows hold the schedule alone and the sweeps gather their
+    // factors; the same values.
+    int compact;
     int nCell, nBFace, nFace, nTotal;
     const int2 *lr;              // [nFace] left, right (boundary face f: right = nCell + f)
     const double *frec;          // [nFace][kF]
@@ -130,7 +141,7 @@ struct DevGrid {
     const int32_t *btype;        // [nBFace] bcType
     const uint8_t *farfield_adj; // [nCell] 1 if the cell touches a limiter-zeroing boundary
     SweepDev fwd, bwd;           // LU-SGS schedules
-    const int2 *use;             // [nFace] lane (row * 32 + lane) of the left and of the right cell's use of the face;
+    const int2 *use;             // [nFace] (full layout) lane (row * 32 + lane) of the left and of the right cell's use of the face;
                                  // >= 0 in the forward sweep, ~ it in the backward sweep (interior faces)
     const int *lead;             // [nCell] slot (row * kSweepSlots + slot) of the cell's last forward row
     const int *last;             // [nCell] and of its last backward row
@@ -189,12 +200,23 @@ struct NsConst {
 template <class T>
 struct Work {
     T *qrec;        // [nTotal][kQ] working state, c2 = |gamma p / rho|, total enthalpy, limiter
-    T *fnrm, *fgeo; // [nFace][kNrm], [nFace][kGeo] face geometry
-    T *fsa;         // [nFace][kGeoSa] SA face geometry (SA runs; else null)
+    // full layout | compact layout
+    union {
+        T *fnrm;    // [nFace][kNrm] face geometry
+        T *frad;    // [nFace][2] Roe spectral radius, viscous spectral term
+    };
+    union {
+        T *fgeo;    // [nFace][kGeo] face geometry
+        T *lead;    // [nCell][kLeadF] right-hand side of the backward sweep
+    };
+    union {
+        T *fsa;     // [nFace][kGeoSa] SA face geometry (SA runs; else null)
+        T *gsum;    // [nGhostCell][kLeadF] boundary part of the backward right-hand side
+    };
     T *grec;        // [nTotal][kG] primitive gradients (ghost rows: interface ghosts only, from the halo exchange)
     T *flux;        // [nFace][kFlux] face flux times area and inviscid spectral radius term (in the scratch)
     T *coef;        // [nBFace][kUse] LU-SGS factors of the boundary faces' uses
-    unsigned char *rowf, *rowb;   // [rows][kRowNs] LU-SGS rows of the forward and the backward sweep
+    unsigned char *rowf, *rowb;   // [rows][kRowNs] (compact: [kRowCompact]) rows of the forward and the backward sweep
     T *crec;        // [nCell][kC] residual, diagonal, spectral radii
     T *dtraw;       // [nCell] CFL * vol / spectral radius, before the ktmax clamp
     // LU-SGS dq, write-once per sweep, by the slot of the cell's last row (a
@@ -213,7 +235,8 @@ struct TurbWork {
     T *tgrad;       // [nCell][kTg] gradient of nu~
     T *tcrec;       // [nCell][kTc] residual, spectral radius, its reciprocal, pad
     T *tface;       // [nFace][kTf] face terms (in the scratch)
-    unsigned char *trowf, *trowb;   // [rows][kRowSa] LU-SGS rows
+    unsigned char *trowf, *trowb;   // [rows][kRowSa] LU-SGS rows (compact: the NS sweeps' rows)
+    T *tmat;        // [nFace][2] compact layout: LU-SGS matrix of the left and the right cell's use
     T *tdq;         // [backward rows][kSweepSlots] LU-SGS dq (write-once per sweep, by slot as the NS records)
     T *tdqf;        // [forward rows][kSweepSlots] forward-sweep dq
     T *tsrc;        // [nCell] source computed by the learned-source kernel (sa_source != 0)
@@ -228,7 +251,7 @@ struct Reduce {
 };
 
 // Kernel launchers (phx_kernels.cu).
-// Face geometry in the working precision from the FP64 metrics.
+// The stored face geometry from the FP64 metrics.
 template <class T>
 void launch_face_geometry(const DevGrid &g, const NsConst &c, const Work<T> &w, cudaStream_t s);
 template <class T>

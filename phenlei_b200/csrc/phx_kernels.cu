@@ -13,6 +13,7 @@
 
 #include "phx_internal.h"
 #include "phx_device.cuh"
+#include "phx_geometry.cuh"
 #include "phx_physics.cuh"
 
 namespace phx {
@@ -125,12 +126,11 @@ void launch_sync_qrec(const DevGrid &g, const NsConst &c, const double *q64, con
 }
 
 // ---------------------------------------------------------------------------
-// Face geometry for the working precision (layout: kNrm, kGeo), in FP64 from the
-// metrics: FaceWeight (Geo_UnstructGrid.cpp:2420-2478) and the geometric part of
-// ComputeVisflux (NSSolverUnstruct.cpp:13147-13236).  Interface faces are
-// interior faces (FaceWeight, Geo_UnstructGrid.cpp:2475).  Formed in every pass
-// before, it took three square roots, five divisions and most conversions of the
-// mixed face pass, and 128 bytes of FP64 metrics a face.
+// Face geometry records of the full layout (phx_geometry.cuh).  Formed in the
+// passes instead, the 1M-cell bump's gradient takes 139 us (118), its face and cell
+// passes 300 (255) and its SA residual 241 (181), mixed: square roots, divisions and
+// conversions in FP64 beside single-precision work.  In FP64 it comes to about the
+// same (gradient 288 -> 250, face and cell passes 609 -> 628, SA residual 286 -> 319).
 // ---------------------------------------------------------------------------
 template <class T>
 __global__ void __launch_bounds__(kThreads) face_geometry_kernel(DevGrid g, NsConst c, Work<T> w)
@@ -138,63 +138,20 @@ __global__ void __launch_bounds__(kThreads) face_geometry_kernel(DevGrid g, NsCo
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= g.nFace) return;
     const int2 lr = ld(g.lr + f);
-    double fr[8], xl[4], xr[4];
-    ld8(g.frec + (size_t)f * kF, fr);
-    ld4(g.xrec + (size_t)lr.x * kX, xl);
-    ld4(g.xrec + (size_t)lr.y * kX, xr);
-    T *nrm = w.fnrm + (size_t)f * kNrm;
-    for (int k = 0; k < 3; ++k) nrm[k] = c.gradient == 1 ? (T)(xr[k] - xl[k]) : (T)(fr[k] * fr[3]);
-    nrm[3] = (T)fr[7];
-    T *o = w.fgeo + (size_t)f * (c.viscous ? kGeo<true> : kGeo<false>);
-    double dl[3], dr[3];
-    for (int k = 0; k < 3; ++k) {
-        dl[k] = fr[4 + k] - xl[k];
-        dr[k] = fr[4 + k] - xr[k];
-        o[k] = (T)fr[k];
-        o[4 + k] = (T)dl[k];
-        o[8 + k] = (T)dr[k];
-    }
-    o[3] = (T)fr[3];
-    o[7] = T(1);
-    o[11] = T(0);
-    if (!c.viscous) return;
-    const bool bnd = f < g.nBFace && g.bkind[f] != BK_INTERFACE;
-    const double d1 = sqrt(dl[0] * dl[0] + dl[1] * dl[1] + dl[2] * dl[2]);
-    const double d2 = sqrt(dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2]);
-    if (!bnd) o[7] = (T)(d2 / (d1 + d2 + kSmall));
-    const double dL = -(fr[0] * dl[0] + fr[1] * dl[1] + fr[2] * dl[2]);
-    const double dR = -(fr[0] * dr[0] + fr[1] * dr[1] + fr[2] * dr[2]);
-    const int vf = g.vflag[f];
-    double A = 0.0, B = 0.0;
-    if (vf & 2) {
-        const double wl = bnd ? 1.0 : dL * dL / (dL * dL + dR * dR);
-        A = wl / dL;
-        B = (1.0 - wl) / dR;
-    }
-    o[11] = (T)A;
-    for (int k = 0; k < 3; ++k) {
-        o[12 + k] = vf & 1 ? (T)(fr[k] * dL + dl[k]) : T(0);
-        o[16 + k] = vf & 1 ? (T)(fr[k] * dR + dr[k]) : T(0);
-    }
-    o[15] = (T)B;
+    T nr[4], r[5][4];
+    form_normal<T>(g, c.gradient == 1, f, lr.x, lr.y, nr);
+    st4(w.fnrm + (size_t)f * kNrm, nr);
+    const int n = (c.viscous ? kGeo<true> : kGeo<false>) / 4;
+    if (c.viscous) form_face<T, true>(g, f, lr.x, lr.y, r[0], r[1], r[2], r[3], r[4]);
+    else form_face<T, false>(g, f, lr.x, lr.y, r[0], r[1], r[2], r[3], r[4]);
+#pragma unroll
+    for (int k = 0; k < 5; ++k)
+        if (k < n) st4(w.fgeo + (size_t)f * n * 4 + k * 4, r[k]);
     if (w.fsa) {
-        // normal derivative of TurbSolverUnstr::ComputeVisflux (TurbSolverUnstr.cpp:
-        // 4438-4674): the weighted differences to the mean of both sides, or across
-        // the whole distance on boundary faces other than symmetry
-        double C = 0.0;
-        if (vf & 4) {
-            const double wl = dL * dL / (dL * dL + dR * dR);
-            C = 0.5 * ((1.0 - wl) / dR - wl / dL);
-            if (bnd && g.btype[f] != PHX_BC_SYMMETRY)
-                C = 1.0 / ((xr[0] - xl[0]) * fr[0] + (xr[1] - xl[1]) * fr[1] + (xr[2] - xl[2]) * fr[2]);
-        }
-        T *sa = w.fsa + (size_t)f * kGeoSa;
-        for (int k = 0; k < 4; ++k) sa[k] = (T)fr[k];
-        sa[4] = (T)C;
-        sa[5] = (T)(1.0 / (0.5 * (xl[3] + xr[3])));
-        sa[6] = sa[7] = T(0);
+        T sa[8];
+        form_sa<T>(g, f, lr.x, lr.y, sa);
+        st8(w.fsa + (size_t)f * kGeoSa, sa);
     }
-    o[19] = (T)fabs(fr[0] * (xr[0] - xl[0]) + fr[1] * (xr[1] - xl[1]) + fr[2] * (xr[2] - xl[2]));
 }
 
 template <class T>
@@ -274,8 +231,8 @@ __global__ void __launch_bounds__(kThreads) node_value_kernel(DevGrid g, NsConst
 template <class T>
 constexpr int kPassThreads = sizeof(T) == 4 ? 256 : 128;
 
-// kGrad: 0 GG-cell, 1 least squares, 2 GG-node.
-template <class T, bool kTemp, int kGrad>
+// kGrad: 0 GG-cell, 1 least squares, 2 GG-node.  kCompact: geometry formed here, not stored.
+template <class T, bool kTemp, int kGrad, bool kCompact>
 __global__ void __launch_bounds__(kPassThreads<T>) gradient_limiter_kernel(DevGrid g, NsConst c, Work<T> w)
 {
     constexpr bool kLsq = kGrad == 1;
@@ -301,7 +258,8 @@ __global__ void __launch_bounds__(kPassThreads<T>) gradient_limiter_kernel(DevGr
         const int f = isLeft ? e.x : ~e.x;
         T qn[8], nr[4];
         ld8(w.qrec + (size_t)e.y * kQ, qn);
-        ld4(w.fnrm + (size_t)f * kNrm, nr);
+        if (kCompact) form_normal<T>(g, kLsq, f, isLeft ? cell : e.y, isLeft ? e.y : cell, nr);
+        else ld4(w.fnrm + (size_t)f * kNrm, nr);
         T vn[NV];
 #pragma unroll
         for (int k = 0; k < 5; ++k) vn[k] = qn[k];
@@ -395,10 +353,15 @@ __global__ void __launch_bounds__(kPassThreads<T>) gradient_limiter_kernel(DevGr
         for (int j = j0; j < j1; ++j) {
             const int e = ld(&g.c2x[j].x);
             const bool isLeft = e >= 0;
-            const T *geo = w.fgeo + (size_t)(isLeft ? e : ~e) * kGeo<kTemp>;
+            const int f = isLeft ? e : ~e;
             T fn[4], dc[4];
-            ld4(geo, fn);
-            ld4(geo + (isLeft ? 4 : 8), dc);
+            if (kCompact) {
+                form_side<T>(g, f, cell, fn, dc);
+            } else {
+                const T *geo = w.fgeo + (size_t)f * kGeo<kTemp>;
+                ld4(geo, fn);
+                ld4(geo + (isLeft ? 4 : 8), dc);
+            }
             const T dx = dc[0], dy = dc[1], dz = dc[2];
             const T ds = sqrt(dx * dx + dy * dy + dz * dz);
             const T nd = fn[0] * dx + fn[1] * dy + fn[2] * dz;
@@ -422,7 +385,10 @@ __global__ void __launch_bounds__(kPassThreads<T>) gradient_limiter_kernel(DevGr
         for (int j = j0; j < j1; ++j) {
             const int e = ld(&g.c2x[j].x);
             T dc[4];
-            ld4(w.fgeo + (size_t)(e >= 0 ? e : ~e) * kGeo<kTemp> + (e >= 0 ? 4 : 8), dc);
+            if (kCompact) {
+                T fn[4];
+                form_side<T>(g, e >= 0 ? e : ~e, cell, fn, dc);
+            } else ld4(w.fgeo + (size_t)(e >= 0 ? e : ~e) * kGeo<kTemp> + (e >= 0 ? 4 : 8), dc);
             const T dx = dc[0], dy = dc[1], dz = dc[2];
             T d = gx[0] * dx + gy[0] * dy + gz[0] * dz;
             if (d > small) lim = tmin(lim, venfun(dmaxr, d, er));
@@ -436,22 +402,29 @@ __global__ void __launch_bounds__(kPassThreads<T>) gradient_limiter_kernel(DevGr
     w.qrec[(size_t)cell * kQ + 7] = lim;
 }
 
-template <class T>
-void launch_gradient_limiter(const DevGrid &g, const NsConst &c, const Work<T> &w, int nodePrev, cudaStream_t s)
+template <class T, bool kCompact>
+static void launch_gradient(const DevGrid &g, const NsConst &c, const Work<T> &w, cudaStream_t s)
 {
     constexpr int pt = kPassThreads<T>;
     const int blocks = (g.nCell + pt - 1) / pt;
+    if (c.viscous) {
+        if (c.gradient == 1) gradient_limiter_kernel<T, true, 1, kCompact><<<blocks, pt, 0, s>>>(g, c, w);
+        else if (c.gradient == 2) gradient_limiter_kernel<T, true, 2, kCompact><<<blocks, pt, 0, s>>>(g, c, w);
+        else gradient_limiter_kernel<T, true, 0, kCompact><<<blocks, pt, 0, s>>>(g, c, w);
+    } else {
+        if (c.gradient == 1) gradient_limiter_kernel<T, false, 1, kCompact><<<blocks, pt, 0, s>>>(g, c, w);
+        else if (c.gradient == 2) gradient_limiter_kernel<T, false, 2, kCompact><<<blocks, pt, 0, s>>>(g, c, w);
+        else gradient_limiter_kernel<T, false, 0, kCompact><<<blocks, pt, 0, s>>>(g, c, w);
+    }
+}
+
+template <class T>
+void launch_gradient_limiter(const DevGrid &g, const NsConst &c, const Work<T> &w, int nodePrev, cudaStream_t s)
+{
     if (c.gradient == 2)
         node_value_kernel<T><<<(g.nNode + kThreads - 1) / kThreads, kThreads, 0, s>>>(g, c, w, nodePrev);
-    if (c.viscous) {
-        if (c.gradient == 1) gradient_limiter_kernel<T, true, 1><<<blocks, pt, 0, s>>>(g, c, w);
-        else if (c.gradient == 2) gradient_limiter_kernel<T, true, 2><<<blocks, pt, 0, s>>>(g, c, w);
-        else gradient_limiter_kernel<T, true, 0><<<blocks, pt, 0, s>>>(g, c, w);
-    } else {
-        if (c.gradient == 1) gradient_limiter_kernel<T, false, 1><<<blocks, pt, 0, s>>>(g, c, w);
-        else if (c.gradient == 2) gradient_limiter_kernel<T, false, 2><<<blocks, pt, 0, s>>>(g, c, w);
-        else gradient_limiter_kernel<T, false, 0><<<blocks, pt, 0, s>>>(g, c, w);
-    }
+    if (g.compact) launch_gradient<T, true>(g, c, w, s);
+    else launch_gradient<T, false>(g, c, w, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -575,7 +548,7 @@ __device__ __forceinline__ void reset_reduce(Reduce *r)
 // after the other, so that little is held at a time.  With the cell pass, on the
 // 1M-cell bump: mixed 335 -> 255 us, FP64 918 -> 607 us against geometry formed
 // in the pass, gradients read twice and 256 threads at 166 registers.
-template <class T, bool kVisc, int kScheme>
+template <class T, bool kVisc, int kScheme, bool kCompact>
 __global__ void __launch_bounds__(kPassThreads<T>, 3) face_flux_kernel(DevGrid g, NsConst c, Work<T> w, Reduce *red)
 {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -583,12 +556,16 @@ __global__ void __launch_bounds__(kPassThreads<T>, 3) face_flux_kernel(DevGrid g
     if (f >= g.nFace) return;
     const int2 lr = ld(g.lr + f);
     const int le = lr.x, re = lr.y;
-    const T *geo = w.fgeo + (size_t)f * kGeo<kVisc>;
     T gn[4], gl[4], gr[4], xl[4], xr[4];
-    ld4(geo, gn);
-    ld4(geo + 4, gl);
-    ld4(geo + 8, gr);
-    if (kVisc) { ld4(geo + 12, xl); ld4(geo + 16, xr); }
+    if (kCompact) {
+        form_face<T, kVisc>(g, f, le, re, gn, gl, gr, xl, xr);
+    } else {
+        const T *geo = w.fgeo + (size_t)f * kGeo<kVisc>;
+        ld4(geo, gn);
+        ld4(geo + 4, gl);
+        ld4(geo + 8, gr);
+        if (kVisc) { ld4(geo + 12, xl); ld4(geo + 16, xr); }
+    }
     T qL[8], qR[8];
     ld8(w.qrec + (size_t)le * kQ, qL);
     ld8(w.qrec + (size_t)re * kQ, qR);
@@ -682,11 +659,15 @@ __global__ void __launch_bounds__(kPassThreads<T>, 3) face_flux_kernel(DevGrid g
     sweep_use<T>(qR, xn, yn, zn, area, rad, vspec, v);
     if (f < g.nBFace) {
         put_use(w.coef + (size_t)f * kUse, 0, v);
-    } else {
+    } else if (!kCompact) {
         const int2 at = ld(g.use + f);
         put_use(use_at<T>(w, at.x), (at.x < 0 ? ~at.x : at.x) & 31, v);
         sweep_use<T>(qL, -xn, -yn, -zn, area, rad, vspec, v);
         put_use(use_at<T>(w, at.y), (at.y < 0 ? ~at.y : at.y) & 31, v);
+    }
+    if (kCompact) {
+        w.frad[2 * (size_t)f] = rad;
+        w.frad[2 * (size_t)f + 1] = vspec;
     }
 }
 
@@ -755,7 +736,7 @@ __global__ void __launch_bounds__(kThreads) cell_residual_kernel(DevGrid g, NsCo
         st8(w.crec + (size_t)cell * kC, out);
         out[6] = dt;
         out[7] = T(0);
-        st8(lead_at<T, true>(w, ld(g.lead + cell)), out);
+        if (!g.compact) st8(lead_at<T, true>(w, ld(g.lead + cell)), out);
     }
     // block minimum, then one atomic per block, skipped when it cannot lower
     // the running minimum (positive doubles order like their bit patterns)
@@ -771,23 +752,31 @@ __global__ void __launch_bounds__(kThreads) cell_residual_kernel(DevGrid g, NsCo
     }
 }
 
+template <class T, bool kCompact>
+static void launch_face_flux(const DevGrid &g, const NsConst &c, const Work<T> &w, Reduce *red, cudaStream_t s)
+{
+    constexpr int ft = kPassThreads<T>;
+    const int fb = (g.nFace + ft - 1) / ft;
+    const int kind = c.scheme == PHX_SCHEME_ROE ? 0 : c.scheme == PHX_SCHEME_VANLEER_ROTATE ? 2 : 1;
+    if (c.viscous) {
+        if (kind == 0) face_flux_kernel<T, true, 0, kCompact><<<fb, ft, 0, s>>>(g, c, w, red);
+        else if (kind == 2) face_flux_kernel<T, true, 2, kCompact><<<fb, ft, 0, s>>>(g, c, w, red);
+        else face_flux_kernel<T, true, 1, kCompact><<<fb, ft, 0, s>>>(g, c, w, red);
+    } else {
+        if (kind == 0) face_flux_kernel<T, false, 0, kCompact><<<fb, ft, 0, s>>>(g, c, w, red);
+        else if (kind == 2) face_flux_kernel<T, false, 2, kCompact><<<fb, ft, 0, s>>>(g, c, w, red);
+        else face_flux_kernel<T, false, 1, kCompact><<<fb, ft, 0, s>>>(g, c, w, red);
+    }
+}
+
 template <class T>
 void launch_residual(const DevGrid &g, const NsConst &c, const Work<T> &w, Reduce *red, double cfl, cudaStream_t s)
 {
-    constexpr int ft = kPassThreads<T>;
-    const int fb = (g.nFace + ft - 1) / ft, cb = (g.nCell + kThreads - 1) / kThreads;
-    const int kind = c.scheme == PHX_SCHEME_ROE ? 0 : c.scheme == PHX_SCHEME_VANLEER_ROTATE ? 2 : 1;
-    if (c.viscous) {
-        if (kind == 0) face_flux_kernel<T, true, 0><<<fb, ft, 0, s>>>(g, c, w, red);
-        else if (kind == 2) face_flux_kernel<T, true, 2><<<fb, ft, 0, s>>>(g, c, w, red);
-        else face_flux_kernel<T, true, 1><<<fb, ft, 0, s>>>(g, c, w, red);
-        cell_residual_kernel<T, true><<<cb, kThreads, 0, s>>>(g, c, w, red, cfl);
-    } else {
-        if (kind == 0) face_flux_kernel<T, false, 0><<<fb, ft, 0, s>>>(g, c, w, red);
-        else if (kind == 2) face_flux_kernel<T, false, 2><<<fb, ft, 0, s>>>(g, c, w, red);
-        else face_flux_kernel<T, false, 1><<<fb, ft, 0, s>>>(g, c, w, red);
-        cell_residual_kernel<T, false><<<cb, kThreads, 0, s>>>(g, c, w, red, cfl);
-    }
+    if (g.compact) launch_face_flux<T, true>(g, c, w, red, s);
+    else launch_face_flux<T, false>(g, c, w, red, s);
+    const int cb = (g.nCell + kThreads - 1) / kThreads;
+    if (c.viscous) cell_residual_kernel<T, true><<<cb, kThreads, 0, s>>>(g, c, w, red, cfl);
+    else cell_residual_kernel<T, false><<<cb, kThreads, 0, s>>>(g, c, w, red, cfl);
 }
 
 // ---------------------------------------------------------------------------
@@ -894,7 +883,7 @@ __global__ void __launch_bounds__(kThreads) sweep_ghost_kernel(DevGrid g, NsCons
 #pragma unroll
         for (int m = 0; m < 5; ++m) sum[m] += df[m];
     }
-    st8(lead_at<T, false>(w, gc.y) + 8, sum);
+    st8(g.compact ? w.gsum + (size_t)i * kLeadF : lead_at<T, false>(w, gc.y) + 8, sum);
 }
 
 // One sweep: a warp per block, so that the few warps of a small mesh spread over
@@ -912,11 +901,59 @@ template <class T>
 constexpr int kSweepHead = (kSweepZero + 1) * 8 * (int)sizeof(T) + (sizeof(T) == 4 ? 96 : 64);
 static_assert(kSweepHead<float> % 128 == 0 && kSweepHead<double> % 128 == 0, "aligned stages");
 
-template <class T, bool kForward>
-__global__ void __launch_bounds__(32) lusgs_kernel(DevGrid g, NsConst c, Work<T> w, Reduce *red, int stages)
+// Compact layout: the rows hold the schedule alone.  A lane forms its factors from
+// the neighbour's state, the metrics and the face's two spectral terms, as the face
+// pass does for full rows; right-hand sides lie by cell.  A row
+// names the uses and cells of the warp's row after next, so that these loads are on
+// their way for two rows (16M-cell bump, mixed, both NS sweeps: 5.6 ms, 7.8 when they
+// begin with their row, 3.1 with full rows).
+template <class T>
+struct UseIn {
+    int2 e;          // face (sign bit: the normal points into the cell), neighbour (-1: none)
+    double n[4];
+    T q[4], hm, rad, vspec;
+};
+template <class T>
+__device__ __forceinline__ void fetch_use(const DevGrid &g, const Work<T> &w, int2 e, UseIn<T> &s)
 {
-    using Pipe = RowPipe<kRowNs<T, kForward>>;
-    constexpr int kLead = kForward ? kLeadF : kLeadB, kRow = kRowNs<T, kForward>;
+    s.e = e;
+    if (e.y < 0) return;
+    const int f = e.x & 0x7fffffff;
+    const T *q = w.qrec + (size_t)e.y * kQ;
+    ld4(g.frec + (size_t)f * kF, s.n);
+    ld4(q, s.q);
+    s.hm = ld(q + 6);
+    s.rad = ld(w.frad + 2 * (size_t)f);
+    s.vspec = ld(w.frad + 2 * (size_t)f + 1);
+}
+template <class T>
+__device__ __forceinline__ void form_use(const UseIn<T> &s, T *u)
+{
+    if (s.e.y < 0) {
+#pragma unroll
+        for (int k = 0; k < kUse; ++k) u[k] = T(0);
+        return;
+    }
+    const T sg = s.e.x < 0 ? T(-1) : T(1);
+    const T qn[8] = {s.q[0], s.q[1], s.q[2], s.q[3], T(0), T(0), s.hm, T(0)};
+    sweep_use<T>(qn, sg * (T)s.n[0], sg * (T)s.n[1], sg * (T)s.n[2], (T)s.n[3], s.rad, s.vspec, u);
+}
+// Right-hand side of a cell (lane 0 of its slot; -1: none): residual (5), reciprocal diagonal, forward: time step.
+template <class T, bool kForward>
+__device__ __forceinline__ void fetch_lead(const Work<T> &w, int cell, T *q)
+{
+    if (cell < 0) return;
+    ld8((kForward ? w.crec : w.lead) + (size_t)cell * kC, q);
+    if (kForward) q[6] = ld(w.dtraw + cell);
+}
+
+// kCompact: registers for as many warps an SM as the schedule may be made for (sweep_max_warps)
+template <class T, bool kForward, bool kCompact>
+__global__ void __launch_bounds__(32, kCompact ? (sizeof(T) == 4 ? 16 : 12) : 0)
+    lusgs_kernel(DevGrid g, NsConst c, Work<T> w, Reduce *red, int stages)
+{
+    constexpr int kLead = kForward ? kLeadF : kLeadB, kRow = kCompact ? kRowCompact : kRowNs<T, kForward>;
+    using Pipe = RowPipe<kRow>;
     constexpr int kLeadOff = 32 * kUse * (int)sizeof(T), kRowOff = kRow - kSweepRow * 4;
     extern __shared__ __align__(128) unsigned char sm[];
     T *loc = reinterpret_cast<T *>(sm);
@@ -940,22 +977,45 @@ __global__ void __launch_bounds__(32) lusgs_kernel(DevGrid g, NsConst c, Work<T>
         if (en >= 0) poll5_load(out + (size_t)en * kD, v);
     };
     T va[5], vb[5], rhs[5];
+    UseIn<T> ua, ub;
+    T qa[8], qb[8];
     int ea, eb;
+    if (kCompact) {
+        const int2 *fu = sw.first_use + blockIdx.x * 64;
+        const int *fc = sw.first_cell + blockIdx.x * 16;
+        fetch_use<T>(g, w, fu[t], ua);
+        fetch_use<T>(g, w, fu[32 + t], ub);
+        fetch_lead<T, kForward>(w, lane == 0 ? fc[slot] : -1, qa);
+        fetch_lead<T, kForward>(w, lane == 0 ? fc[8 + slot] : -1, qb);
+    }
     entry(sw.first + blockIdx.x * 64, ea, va);
     entry(sw.first + blockIdx.x * 64 + 32, eb, vb);
     bool ok = true;
-    auto step = [&](int i, int &en, T *v) -> bool {
+    auto step = [&](int i, int &en, T *v, UseIn<T> &in, T *qin) -> bool {
         const unsigned char *row = pipe.at(pipe.slot) + i * kRow;
         const int4 info = reinterpret_cast<const int4 *>(row + kRowOff + 128)[slot];
         const T *lead = reinterpret_cast<const T *>(row + kLeadOff) + slot * kLead;
-        T u[kUse];
-        get_use(reinterpret_cast<const T *>(row) + t * kUse, t, u);
+        T u[kUse], q[8], b[5] = {0, 0, 0, 0, 0};
+        if (kCompact) {
+            form_use<T>(in, u);
+            fetch_use<T>(g, w, reinterpret_cast<const int2 *>(row)[t], in);
+#pragma unroll
+            for (int m = 0; m < 8; ++m) q[m] = qin[m];
+            fetch_lead<T, kForward>(w, lane == 0 ? reinterpret_cast<const int *>(row + 256)[slot] : -1, qin);
+            if (!kForward && lane == 0 && info.w > 0) {
+                const T *gs = w.gsum + (size_t)(info.w - 1) * kLeadF;
+                ld4(gs, b);
+                b[4] = ld(gs + 4);
+            }
+        } else {
+            get_use(reinterpret_cast<const T *>(row) + t * kUse, t, u);
+        }
         if (en < 0) {
             const T *a = loc + ~en * 8;
-            T b[4];
-            get4(a, b);
+            T o[4];
+            get4(a, o);
 #pragma unroll
-            for (int m = 0; m < 4; ++m) v[m] = b[m];
+            for (int m = 0; m < 4; ++m) v[m] = o[m];
             v[4] = a[4];
         }
         // fault injection (phx_fault_hold_cell): the held cell waits on
@@ -985,11 +1045,12 @@ __global__ void __launch_bounds__(32) lusgs_kernel(DevGrid g, NsConst c, Work<T>
 #pragma unroll
             for (int m = 0; m < 5; ++m) sum[m] = df[m];
         } else {
-            T b[4];
-            get4(lead + (kForward ? 0 : 8), b);
+            if (!kCompact) {
+                get4(lead + (kForward ? 0 : 8), b);
+                b[4] = lead[kForward ? 0 : 12];
+            }
 #pragma unroll
-            for (int m = 0; m < 4; ++m) sum[m] = b[m] + df[m];
-            sum[4] = lead[kForward ? 0 : 12] + df[4];
+            for (int m = 0; m < 5; ++m) sum[m] = b[m] + df[m];
         }
         if ((info.y & kSweepMulti) && (info.y & kSweepCarry)) {
 #pragma unroll
@@ -1010,8 +1071,8 @@ __global__ void __launch_bounds__(32) lusgs_kernel(DevGrid g, NsConst c, Work<T>
             // 1 / (dt' / vol) + spectral radii, dt' = min(dt, ktmax min dt)
             // (ReduceMaxTimeStep, :5717-5745): formed by the residual pass for
             // the raw dt, by the forward sweep where the clamp applies
-            T q[8], o[5];
-            get8(lead, q);
+            T o[5];
+            if (!kCompact) get8(lead, q);
             if (kForward && q[6] > clamp) {
                 const T *cr = w.crec + (size_t)info.x * kC;
                 T d = idiv(T(1), idiv(clamp, (T)ld(g.xrec + (size_t)info.x * kX + 3)));
@@ -1027,7 +1088,7 @@ __global__ void __launch_bounds__(32) lusgs_kernel(DevGrid g, NsConst c, Work<T>
             st4(own, o);
             own[4] = o[4];
             publish5(mine, o);
-            if (kForward) st8(lead_at<T, false>(w, info.z), q);
+            if (kForward) st8(kCompact ? w.lead + (size_t)info.x * kLeadF : lead_at<T, false>(w, info.z), q);
         }
         mine += kSweepSlots * kD;
         __syncwarp();
@@ -1035,7 +1096,7 @@ __global__ void __launch_bounds__(32) lusgs_kernel(DevGrid g, NsConst c, Work<T>
     };
     int k = 0;
     while (ok && k < pipe.nstage) {
-        ok = pipe.wait() && step(0, ea, va) && (2 * k + 1 >= nrow || step(1, eb, vb));
+        ok = pipe.wait() && step(0, ea, va, ua, qa) && (2 * k + 1 >= nrow || step(1, eb, vb, ub, qb));
         if (!ok) break;
         pipe.advance(t);
         ++k;
@@ -1061,8 +1122,11 @@ __global__ void __launch_bounds__(kThreads) sweep_reset_kernel(int rowsF, int ro
 }
 
 // Shared memory of a sweep's warp with the given number of stages.
-template <class T, bool kForward>
-static int sweep_smem(int stages) { return kSweepHead<T> + stages * RowPipe<kRowNs<T, kForward>>::kStage; }
+template <class T, bool kForward, bool kCompact>
+static int sweep_smem(int stages)
+{
+    return kSweepHead<T> + stages * RowPipe<kCompact ? kRowCompact : kRowNs<T, kForward>>::kStage;
+}
 
 // Warps of the sweeps that are resident together with two stages each: the
 // schedule is made for at most this many.  PHX_LUSGS_MAX_BLOCKS caps them
@@ -1070,12 +1134,18 @@ static int sweep_smem(int stages) { return kSweepHead<T> + stages * RowPipe<kRow
 template <class T>
 int sweep_max_warps(int numSMs)
 {
-    cudaFuncSetAttribute(lusgs_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sweep_smem<T, true>(4));
-    cudaFuncSetAttribute(lusgs_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sweep_smem<T, false>(4));
-    int f = 0, b = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, lusgs_kernel<T, true>, 32, sweep_smem<T, true>(2));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, lusgs_kernel<T, false>, 32, sweep_smem<T, false>(2));
-    int n = std::max(1, std::min(std::min(f, b), 16)) * numSMs;
+    int n = 16;
+    auto resident = [&](auto kernel, int most, int two) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        int k = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kernel, 32, two);
+        n = std::min(n, k);
+    };
+    resident(lusgs_kernel<T, true, false>, sweep_smem<T, true, false>(4), sweep_smem<T, true, false>(2));
+    resident(lusgs_kernel<T, false, false>, sweep_smem<T, false, false>(4), sweep_smem<T, false, false>(2));
+    resident(lusgs_kernel<T, true, true>, sweep_smem<T, true, true>(4), sweep_smem<T, true, true>(2));
+    resident(lusgs_kernel<T, false, true>, sweep_smem<T, false, true>(4), sweep_smem<T, false, true>(2));
+    n = std::max(1, n) * numSMs;
     if (const char *cap = getenv("PHX_LUSGS_MAX_BLOCKS")) {
         const int v = atoi(cap);
         if (v > 0 && n > v) n = v;
@@ -1085,7 +1155,7 @@ int sweep_max_warps(int numSMs)
 template int sweep_max_warps<double>(int);
 template int sweep_max_warps<float>(int);
 
-template <class T, bool kForward>
+template <class T, bool kForward, bool kCompact>
 static cudaError_t launch_sweep(const DevGrid &g, const NsConst &c, const Work<T> &w, Reduce *red, int numSMs, cudaStream_t s)
 {
     const int warps = (kForward ? g.fwd : g.bwd).nWarps;
@@ -1093,14 +1163,14 @@ static cudaError_t launch_sweep(const DevGrid &g, const NsConst &c, const Work<T
     // 1 KB of each block the system's)
     int stages = 2;
     const int perSM = (warps + numSMs - 1) / numSMs;
-    while (stages < 4 && perSM * (sweep_smem<T, kForward>(stages + 1) + 1024) <= 224 * 1024) ++stages;
+    while (stages < 4 && perSM * (sweep_smem<T, kForward, kCompact>(stages + 1) + 1024) <= 224 * 1024) ++stages;
     DevGrid gg = g;
     NsConst cc = c;
     Work<T> ww = w;
     Reduce *rr = red;
     void *args[] = {&gg, &cc, &ww, &rr, &stages};
-    return cudaLaunchCooperativeKernel((void *)lusgs_kernel<T, kForward>, dim3(warps), dim3(32), args,
-                                       sweep_smem<T, kForward>(stages), s);
+    return cudaLaunchCooperativeKernel((void *)lusgs_kernel<T, kForward, kCompact>, dim3(warps), dim3(32), args,
+                                       sweep_smem<T, kForward, kCompact>(stages), s);
 }
 
 template <class T>
@@ -1112,12 +1182,14 @@ int launch_lusgs(const DevGrid &g, const NsConst &c, const Work<T> &w, Reduce *r
         const long long n = (long long)std::max(g.fwd.nRows, g.bwd.nRows) * kSweepSlots * kD / 4;
         const int rb = (int)std::min<long long>((n + kThreads - 1) / kThreads, (long long)numSMs * 16);
         sweep_reset_kernel<T><<<rb, kThreads, 0, s>>>(g.fwd.nRows, g.bwd.nRows, w.dqfwd, w.dqrec);
-        e = launch_sweep<T, true>(g, c, w, red, numSMs, s);
+        e = g.compact ? launch_sweep<T, true, true>(g, c, w, red, numSMs, s)
+                      : launch_sweep<T, true, false>(g, c, w, red, numSMs, s);
     }
     if (e == cudaSuccess && (sweeps & kSweepBackward)) {
         if (g.nGhostCell > 0)
             sweep_ghost_kernel<T><<<(g.nGhostCell + kThreads - 1) / kThreads, kThreads, 0, s>>>(g, c, w);
-        e = launch_sweep<T, false>(g, c, w, red, numSMs, s);
+        e = g.compact ? launch_sweep<T, false, true>(g, c, w, red, numSMs, s)
+                      : launch_sweep<T, false, false>(g, c, w, red, numSMs, s);
     }
     return e == cudaSuccess ? 0 : (int)e;
 }

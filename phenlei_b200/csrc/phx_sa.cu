@@ -14,6 +14,7 @@
 #include <algorithm>
 
 #include "phx_device.cuh"
+#include "phx_geometry.cuh"
 #include "phx_internal.h"
 #include "phx_physics.cuh"
 #include "phx_mlp.h"
@@ -114,8 +115,8 @@ void launch_turb_node_values(const DevGrid &g, const Work<T> &w, const TurbWork<
     turb_node_kernel<T><<<(g.nNode + kThreads - 1) / kThreads, kThreads, 0, s>>>(g, w, t);
 }
 
-// kGrad: 0 GG-cell, 1 least squares, 2 GG-node.
-template <class T, int kGrad>
+// kGrad: 0 GG-cell, 1 least squares, 2 GG-node.  kCompact: geometry formed here, not stored.
+template <class T, int kGrad, bool kCompact>
 __global__ void __launch_bounds__(kThreads) sa_visc_grad_kernel(DevGrid g, NsConst c, Work<T> w, TurbWork<T> t)
 {
     constexpr bool kLsq = kGrad == 1;
@@ -143,7 +144,8 @@ __global__ void __launch_bounds__(kThreads) sa_visc_grad_kernel(DevGrid g, NsCon
         const int f = isLeft ? e.x : ~e.x;
         const T vn = ldcg(w.trec + (size_t)e.y * kTr);   // slot 1 of the rows is written by this kernel
         T nr[4];
-        ld4(w.fnrm + (size_t)f * kNrm, nr);
+        if (kCompact) form_normal<T>(g, kLsq, f, isLeft ? cell : e.y, isLeft ? e.y : cell, nr);
+        else ld4(w.fnrm + (size_t)f * kNrm, nr);
         if (kLsq) {
             const T dq = nr[3] * (isLeft ? vn - nue : nue - vn);
             gx += dq * nr[0]; gy += dq * nr[1]; gz += dq * nr[2];
@@ -203,7 +205,7 @@ __device__ __forceinline__ T *sa_lead_at(unsigned char *rows, int slot)
 //    the diffusion spectral term and the face matrices mat_turbl / mat_turbr,
 //    stored per face use for the sweeps.
 // ---------------------------------------------------------------------------
-template <class T>
+template <class T, bool kCompact>
 __global__ void __launch_bounds__(kThreads) sa_face_kernel(DevGrid g, NsConst c, Work<T> w, TurbWork<T> t)
 {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -215,7 +217,8 @@ __global__ void __launch_bounds__(kThreads) sa_face_kernel(DevGrid g, NsConst c,
     const bool bnd = f < g.nBFace && g.bkind[f] != BK_INTERFACE;
     const int bt = bnd ? g.btype[f] : 0;
     T geo[8], qL[8], qR[8], tl[4], tr[4];
-    ld8(w.fsa + (size_t)f * kGeoSa, geo);
+    if (kCompact) form_sa<T>(g, f, le, re, geo);
+    else ld8(w.fsa + (size_t)f * kGeoSa, geo);
     ld8(w.qrec + (size_t)le * kQ, qL);
     ld8(w.qrec + (size_t)re * kQ, qR);
     ld4(w.trec + (size_t)le * kTr, tl);
@@ -289,7 +292,10 @@ __global__ void __launch_bounds__(kThreads) sa_face_kernel(DevGrid g, NsConst c,
         matR += oRe * ovol * ns2 * cr;
     }
     st4(t.tface + (size_t)f * kTf, out);
-    if (f >= g.nBFace) {
+    if (kCompact) {
+        t.tmat[2 * (size_t)f] = matR;
+        t.tmat[2 * (size_t)f + 1] = matL;
+    } else if (f >= g.nBFace) {
         const int2 at = ld(g.use + f);
         *sa_use_at<T>(t, at.x) = matR;
         *sa_use_at<T>(t, at.y) = matL;
@@ -359,9 +365,19 @@ __global__ void __launch_bounds__(kThreads) sa_cell_kernel(DevGrid g, NsConst c,
     res += own * (visl / rho + positive_sa(nue, visl, rho));
     T o[4] = {res, spec, idiv(T(1), spec), T(0)};   // the sweep multiplies by the reciprocal
     st4(t.tcrec + (size_t)cell * kTc, o);
+    if (g.compact) return;
     T *lead = sa_lead_at<T>(t.trowf, ld(g.lead + cell));
     lead[0] = o[0];
     lead[1] = o[2];
+}
+
+template <class T, bool kCompact>
+static void launch_sa_visc_grad(const DevGrid &g, const NsConst &c, const Work<T> &w, const TurbWork<T> &t, cudaStream_t s)
+{
+    const int cb = (g.nCell + kThreads - 1) / kThreads;
+    if (c.gradient == 1) sa_visc_grad_kernel<T, 1, kCompact><<<cb, kThreads, 0, s>>>(g, c, w, t);
+    else if (c.gradient == 2) sa_visc_grad_kernel<T, 2, kCompact><<<cb, kThreads, 0, s>>>(g, c, w, t);
+    else sa_visc_grad_kernel<T, 0, kCompact><<<cb, kThreads, 0, s>>>(g, c, w, t);
 }
 
 template <class T>
@@ -374,11 +390,11 @@ void launch_sa_residual(const DevGrid &g, const NsConst &c, const double *q64, c
     // TurbSolver::UpdateResiduals repeats the boundary (ghost eddy viscosity of
     // the new interior values)
     launch_sa_boundary<T>(g, c, q64, w, t, s);
-    if (c.gradient == 1) sa_visc_grad_kernel<T, 1><<<cb, kThreads, 0, s>>>(g, c, w, t);
-    else if (c.gradient == 2) sa_visc_grad_kernel<T, 2><<<cb, kThreads, 0, s>>>(g, c, w, t);
-    else sa_visc_grad_kernel<T, 0><<<cb, kThreads, 0, s>>>(g, c, w, t);
+    if (g.compact) launch_sa_visc_grad<T, true>(g, c, w, t, s);
+    else launch_sa_visc_grad<T, false>(g, c, w, t, s);
     launch_sa_boundary<T>(g, c, q64, w, t, s);
-    sa_face_kernel<T><<<fb, kThreads, 0, s>>>(g, c, w, t);
+    if (g.compact) sa_face_kernel<T, true><<<fb, kThreads, 0, s>>>(g, c, w, t);
+    else sa_face_kernel<T, false><<<fb, kThreads, 0, s>>>(g, c, w, t);
     if (c.saSource && mlp) launch_mlp_source<T>(g, c, w, t, *mlp, red, nmlp, numSMs, s);
     sa_cell_kernel<T><<<cb, kThreads, 0, s>>>(g, c, w, t, red);
 }
@@ -398,10 +414,13 @@ void launch_sa_residual(const DevGrid &g, const NsConst &c, const double *q64, c
 // all SMs: the 200k plate 400 -> 202 us, the 1M-cell bump 779 -> 400 us.
 static constexpr int kSaStages = 8;
 
-template <class T, bool kForward>
+// Compact layout: the rows are those of the NS sweeps (schedule alone), the matrix
+// of a use lies by face, and the right-hand sides in the cell's record, whose pad
+// carries the forward sweep's to the backward one.
+template <class T, bool kForward, bool kCompact>
 __global__ void __launch_bounds__(32) sa_lusgs_kernel(DevGrid g, TurbWork<T> t, Reduce *red, long long spinLimit)
 {
-    constexpr int kRow = kRowSa<T>, kRowOff = kRow - kSweepRow * 4;
+    constexpr int kRow = kCompact ? kRowCompact : kRowSa<T>, kRowOff = kRow - kSweepRow * 4;
     using Pipe = RowPipe<kRow>;
     __shared__ __align__(128) unsigned char buf[kSaStages * Pipe::kStage];
     __shared__ T loc[kSweepZero + 1];
@@ -421,16 +440,38 @@ __global__ void __launch_bounds__(32) sa_lusgs_kernel(DevGrid g, TurbWork<T> t, 
         if (en >= 0) v = ld_poll(out + en);
     };
     T va = T(0), vb = T(0), rhs = T(0);
+    T ina[3] = {0, 0, 0}, inb[3] = {0, 0, 0};   // compact: matrix, right-hand side, reciprocal spectral radius
     int ea, eb;
+    auto fetch = [&](int2 e, int cell, T *o) {
+        o[0] = e.y >= 0 ? ld(t.tmat + 2 * (size_t)(e.x & 0x7fffffff) + (e.x < 0)) : T(0);
+        if (lane == 0 && cell >= 0) {
+            const T *cr = t.tcrec + (size_t)cell * kTc;
+            o[1] = ldcg(cr + (kForward ? 0 : 3));
+            o[2] = ldcg(cr + 2);
+        }
+    };
+    if (kCompact) {
+        fetch(sw.first_use[blockIdx.x * 64 + th], sw.first_cell[blockIdx.x * 16 + slot], ina);
+        fetch(sw.first_use[blockIdx.x * 64 + 32 + th], sw.first_cell[blockIdx.x * 16 + 8 + slot], inb);
+    }
     entry(sw.first + blockIdx.x * 64, ea, va);
     entry(sw.first + blockIdx.x * 64 + 32, eb, vb);
     bool ok = true;
-    auto step = [&](int i, int &en, T &v) -> bool {
+    auto step = [&](int i, int &en, T &v, T *in) -> bool {
         const unsigned char *row = pipe.at(pipe.slot) + i * kRow;
         const int4 info = reinterpret_cast<const int4 *>(row + kRowOff + 128)[slot];
-        const T mat = reinterpret_cast<const T *>(row)[th];
-        const T *lead = reinterpret_cast<const T *>(row) + 32 + slot * kLeadT;
-        const T r0 = lead[0], rspec = lead[1];
+        T mat, r0, rspec;
+        if (kCompact) {
+            mat = in[0];
+            r0 = in[1];
+            rspec = in[2];
+            fetch(reinterpret_cast<const int2 *>(row)[th], reinterpret_cast<const int *>(row + 256)[slot], in);
+        } else {
+            const T *lead = reinterpret_cast<const T *>(row) + 32 + slot * kLeadT;
+            mat = reinterpret_cast<const T *>(row)[th];
+            r0 = lead[0];
+            rspec = lead[1];
+        }
         if (en < 0) v = loc[~en];
         bool ready = en < 0 || !is_sentinel(v);
         if (!__all_sync(0xffffffffu, ready)) {
@@ -458,7 +499,9 @@ __global__ void __launch_bounds__(32) sa_lusgs_kernel(DevGrid g, TurbWork<T> t, 
             const T q = r0 - sum, o = q * rspec;
             loc[info.y & 255] = o;
             st_relaxed(mine, unsentinel(o));
-            if (kForward) {
+            if (kForward && kCompact) {
+                t.tcrec[(size_t)info.x * kTc + 3] = q;
+            } else if (kForward) {
                 T *nxt = sa_lead_at<T>(t.trowb, info.z);
                 nxt[0] = q;
                 nxt[1] = rspec;
@@ -470,7 +513,7 @@ __global__ void __launch_bounds__(32) sa_lusgs_kernel(DevGrid g, TurbWork<T> t, 
     };
     int k = 0;
     while (ok && k < pipe.nstage) {
-        ok = pipe.wait() && step(0, ea, va) && (2 * k + 1 >= nrow || step(1, eb, vb));
+        ok = pipe.wait() && step(0, ea, va, ina) && (2 * k + 1 >= nrow || step(1, eb, vb, inb));
         if (!ok) break;
         pipe.advance(th);
         ++k;
@@ -496,10 +539,17 @@ __global__ void __launch_bounds__(kThreads) sa_sweep_reset_kernel(int nf, int nb
 template <class T>
 int sa_sweep_max_warps(int numSMs)
 {
-    int f = 0, b = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, sa_lusgs_kernel<T, true>, 32, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, sa_lusgs_kernel<T, false>, 32, 0);
-    return std::max(1, std::min(f, b)) * numSMs;
+    int n = 32;
+    auto resident = [&](auto kernel) {
+        int k = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kernel, 32, 0);
+        n = std::min(n, k);
+    };
+    resident(sa_lusgs_kernel<T, true, false>);
+    resident(sa_lusgs_kernel<T, false, false>);
+    resident(sa_lusgs_kernel<T, true, true>);
+    resident(sa_lusgs_kernel<T, false, true>);
+    return std::max(1, n) * numSMs;
 }
 template int sa_sweep_max_warps<double>(int);
 template int sa_sweep_max_warps<float>(int);
@@ -519,10 +569,12 @@ int launch_sa_lusgs(const DevGrid &g, const NsConst &c, const Work<T> &w, const 
         const int nf = g.fwd.nRows * kSweepSlots, nb = g.bwd.nRows * kSweepSlots;
         const int rb = std::min((std::max(nf, nb) + kThreads - 1) / kThreads, numSMs * 16);
         sa_sweep_reset_kernel<T><<<rb, kThreads, 0, s>>>(nf, nb, t.tdqf, t.tdq);
-        e = cudaLaunchCooperativeKernel((void *)sa_lusgs_kernel<T, true>, dim3(g.fwd.nWarps), dim3(32), args, 0, s);
+        e = cudaLaunchCooperativeKernel(g.compact ? (void *)sa_lusgs_kernel<T, true, true> : (void *)sa_lusgs_kernel<T, true, false>,
+                                        dim3(g.fwd.nWarps), dim3(32), args, 0, s);
     }
     if (e == cudaSuccess && (sweeps & kSweepBackward))
-        e = cudaLaunchCooperativeKernel((void *)sa_lusgs_kernel<T, false>, dim3(g.bwd.nWarps), dim3(32), args, 0, s);
+        e = cudaLaunchCooperativeKernel(g.compact ? (void *)sa_lusgs_kernel<T, false, true> : (void *)sa_lusgs_kernel<T, false, false>,
+                                        dim3(g.bwd.nWarps), dim3(32), args, 0, s);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
