@@ -451,8 +451,10 @@ struct MlpRows {
 // block, its activations in shared memory (as the tile products read them: rows
 // by columns and transposed) and its pre-activations in registers, and the
 // weight gradients of a block's tiles stay in registers until the end
-// (part[block][kNParam]).  256 threads, 4 x 4 outputs each, six 64 x 64 x 64
-// products a tile.  A batch of 8,192 is 128 blocks of one tile: 29 us, bound by
+// (part[block][kNParam]).  The sums over a tile's rows that no product forms (bias
+// gradients, loss) are taken as trees, and the loss runs on in double over tiles
+// and batches, so that no sum is longer than in column sums of the whole batch.
+// 256 threads, 4 x 4 outputs each, six 64 x 64 x 64 products a tile.  A batch of 8,192 is 128 blocks of one tile: 35 us, bound by
 // the FP32 pipe of one block per SM, and 6 us for the sum over the blocks with
 // Adam.  The products layer by layer that it replaces took 1.43 ms, four of them,
 // the weight gradients, on at most 16 blocks with a serial sum over the batch.
@@ -473,6 +475,16 @@ __device__ __forceinline__ void tile_mma(const float *a, const float *b, int ty,
             for (int j = 0; j < 4; ++j) acc[i][j] += ua[i] * va[j];
     }
 }
+// Sum of a column of a tile: four runs of 16 rows.
+__device__ __forceinline__ float tile_column(const float *col)
+{
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+    for (int r = 0; r < kTrRows / 4; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s[q] += col[(r + q * (kTrRows / 4)) * kTrS];
+    return (s[0] + s[1]) + (s[2] + s[3]);
+}
 __device__ __forceinline__ void tile_put(float *rows, float *cols, int ty, int tx, const float (*v)[4])
 {
 #pragma unroll
@@ -485,7 +497,7 @@ __device__ __forceinline__ void tile_put(float *rows, float *cols, int ty, int t
     }
 }
 
-__global__ void __launch_bounds__(kTrThreads) mlp_grad_kernel(const float *p, MlpRows in, int B, float *part, float *loss)
+__global__ void __launch_bounds__(kTrThreads) mlp_grad_kernel(const float *p, MlpRows in, int B, float *part, double *loss)
 {
     extern __shared__ __align__(16) float ts[];
     float *w2t = ts, *w3t = w2t + kTrTile, *w2 = w3t + kTrTile, *w3 = w2 + kTrTile;
@@ -506,7 +518,8 @@ __global__ void __launch_bounds__(kTrThreads) mlp_grad_kernel(const float *p, Ml
     const float b4 = p[kOffB4];
     float g3[4][4] = {}, g2[4][4] = {};             // dW3, dW2 of rows ty * 4.., columns tx * 4..
     float g1[2] = {0.0f, 0.0f};                     // dW1 of elements t, t + 256
-    float gb = 0.0f, gw4 = 0.0f, gb4 = 0.0f, sq = 0.0f;   // gb: b3, b2, b1 on threads 0-63, 64-127, 128-191
+    float gb = 0.0f, gw4 = 0.0f, gb4 = 0.0f;        // gb: b3, b2, b1 on threads 0-63, 64-127, 128-191
+    double sq = 0.0;                                // gb4, sq: on thread 64
     const int tiles = (B + kTrRows - 1) / kTrRows;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         __syncthreads();
@@ -593,13 +606,18 @@ __global__ void __launch_bounds__(kTrThreads) mlp_grad_kernel(const float *p, Ml
         tile_put(dz, dzt, ty, tx, v);
         if (t < 64) {
             for (int r = 0; r < kTrRows; ++r) gw4 += dy[r] * h3[r * kTrS + t];
-        } else if (t == 64) {
-            for (int r = 0; r < kTrRows; ++r) { gb4 += dy[r]; sq += err[r]; }
+        } else if (t < 96) {
+            float d = dy[t - 64] + dy[t - 32], e = err[t - 64] + err[t - 32];
+            for (int o = 16; o > 0; o >>= 1) {
+                d += __shfl_xor_sync(0xffffffffu, d, o);
+                e += __shfl_xor_sync(0xffffffffu, e, o);
+            }
+            gb4 += d;
+            sq += e;
         }
         __syncthreads();
         tile_mma(dz, h2, ty, tx, g3);
-        if (t < 64)
-            for (int r = 0; r < kTrRows; ++r) gb += dz[r * kTrS + t];
+        if (t < 64) gb += tile_column(dz + t);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -614,8 +632,7 @@ __global__ void __launch_bounds__(kTrThreads) mlp_grad_kernel(const float *p, Ml
         tile_put(dz, dzt, ty, tx, v);
         __syncthreads();
         tile_mma(dz, h1, ty, tx, g2);
-        if (t >= 64 && t < 128)
-            for (int r = 0; r < kTrRows; ++r) gb += dz[r * kTrS + t - 64];
+        if (t >= 64 && t < 128) gb += tile_column(dz + t - 64);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -629,8 +646,7 @@ __global__ void __launch_bounds__(kTrThreads) mlp_grad_kernel(const float *p, Ml
             for (int j = 0; j < 4; ++j) v[i][j] *= s1[i][j];
         tile_put(dz, nullptr, ty, tx, v);
         __syncthreads();
-        if (t >= 128 && t < 192)
-            for (int r = 0; r < kTrRows; ++r) gb += dz[r * kTrS + t - 128];
+        if (t >= 128 && t < 192) gb += tile_column(dz + t - 128);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const int e = t + q * kTrThreads;
@@ -658,22 +674,25 @@ __global__ void __launch_bounds__(kTrThreads) mlp_grad_kernel(const float *p, Ml
     }
 }
 
-// Sum of the blocks' gradients (in their order, four runs of them at a time),
-// then Adam (Kingma & Ba 2015) on the parameter; or, without m, the gradient.
+// Sum of the blocks' gradients (sixteen runs of them, then pairwise), then Adam (Kingma & Ba 2015) on the parameter; or, without m, the gradient.
 __global__ void __launch_bounds__(256) mlp_adam_kernel(int nblk, const float *part, float *p, float *m, float *v, float lr,
                                                        float b1, float b2, float eps, float c1, float c2)
 {
     __shared__ float run[4][64];
     const int i = blockIdx.x * 64 + threadIdx.x % 64, q = threadIdx.x / 64;
-    float g = 0.0f;
+    float g[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (i < kNParam) {
         const int k1 = (q + 1) * nblk / 4;
-        for (int k = q * nblk / 4; k < k1; ++k) g += part[(size_t)k * kNParam + i];
+        int k = q * nblk / 4;
+        for (; k + 3 < k1; k += 4)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) g[j] += part[(size_t)(k + j) * kNParam + i];
+        for (; k < k1; ++k) g[0] += part[(size_t)k * kNParam + i];
     }
-    run[q][threadIdx.x % 64] = g;
+    run[q][threadIdx.x % 64] = (g[0] + g[1]) + (g[2] + g[3]);
     __syncthreads();
     if (q != 0 || i >= kNParam) return;
-    const float gi = ((run[0][threadIdx.x] + run[1][threadIdx.x]) + run[2][threadIdx.x]) + run[3][threadIdx.x];
+    const float gi = (run[0][threadIdx.x] + run[1][threadIdx.x]) + (run[2][threadIdx.x] + run[3][threadIdx.x]);
     if (!m) { p[i] = gi; return; }
     const float mi = b1 * m[i] + (1.0f - b1) * gi;
     const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
@@ -770,11 +789,11 @@ int mlp_train(const float *X, const float *Y, long long n, int epochs, int batch
     DevBuf db;
     float *dX = db.get<float>((size_t)n * kMlpIn), *dY = db.get<float>(n);
     int *dperm = db.get<int>(n);
-    // parameters, Adam moments, normalisation, the blocks' losses and gradients
-    float *p = db.get<float>(3 * (size_t)kNParam + 2 * kMlpIn + nblk + (size_t)nblk * kNParam);
-    if (!dX || !dY || !dperm || !p) return (int)cudaErrorMemoryAllocation;
-    float *m1 = p + kNParam, *m2 = m1 + kNParam, *dmean = m2 + kNParam, *drstd = dmean + kMlpIn, *loss = drstd + kMlpIn,
-          *part = loss + nblk;
+    // parameters, Adam moments, normalisation, the blocks' gradients; and their losses
+    float *p = db.get<float>(3 * (size_t)kNParam + 2 * kMlpIn + (size_t)nblk * kNParam);
+    double *loss = db.get<double>(nblk);
+    if (!dX || !dY || !dperm || !p || !loss) return (int)cudaErrorMemoryAllocation;
+    float *m1 = p + kNParam, *m2 = m1 + kNParam, *dmean = m2 + kNParam, *drstd = dmean + kMlpIn, *part = drstd + kMlpIn;
     cudaMemcpyAsync(dX, X, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dY, Y, sizeof(float) * n, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(p, prm.data(), sizeof(float) * kNParam, cudaMemcpyHostToDevice, s);
@@ -790,7 +809,7 @@ int mlp_train(const float *X, const float *Y, long long n, int epochs, int batch
         // shuffled while the device still runs the epoch before
         for (long long i = n - 1; i > 0; --i) std::swap(perm[i], perm[splitmix(rs) % (uint64_t)(i + 1)]);
         cudaMemcpyAsync(dperm, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s);
-        cudaMemsetAsync(loss, 0, sizeof(float) * nblk, s);
+        cudaMemsetAsync(loss, 0, sizeof(double) * nblk, s);
         for (long long off = 0; off + B <= n; off += B) {
             const MlpRows rows{dX, dY, dperm + off, dmean, drstd, 1.0f / tscale};
             mlp_grad_kernel<<<nblk, kTrThreads, kTrSmemFloats * sizeof(float), s>>>(p, rows, B, part, loss);
@@ -799,8 +818,8 @@ int mlp_train(const float *X, const float *Y, long long n, int epochs, int batch
             mlp_adam_kernel<<<(kNParam + 63) / 64, 256, 0, s>>>(nblk, part, p, m1, m2, lr, b1, b2, eps, c1, c2);
         }
     }
-    std::vector<float> lossHost(nblk);
-    cudaMemcpyAsync(lossHost.data(), loss, sizeof(float) * nblk, cudaMemcpyDeviceToHost, s);
+    std::vector<double> lossHost(nblk);
+    cudaMemcpyAsync(lossHost.data(), loss, sizeof(double) * nblk, cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) return (int)cudaGetLastError();
     double lh = 0.0;
     for (int i = 0; i < nblk; ++i) lh += lossHost[i];
@@ -831,19 +850,20 @@ int mlp_loss_grad(const float *params, const float *x, const float *y, int B, fl
     if (nLoss < 1) return (int)cudaGetLastError();
     DevBuf db;
     float *p = db.get<float>(kNParam), *gp = db.get<float>(kNParam), *dx = db.get<float>((size_t)B * kMlpIn),
-          *dy = db.get<float>(B), *loss = db.get<float>(nLoss), *part = db.get<float>((size_t)nLoss * kNParam);
+          *dy = db.get<float>(B), *part = db.get<float>((size_t)nLoss * kNParam);
+    double *loss = db.get<double>(nLoss);
     if (!p || !gp || !dx || !dy || !loss || !part) return (int)cudaErrorMemoryAllocation;
     cudaMemcpyAsync(p, params, sizeof(float) * kNParam, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dx, x, sizeof(float) * B * kMlpIn, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dy, y, sizeof(float) * B, cudaMemcpyHostToDevice, s);
-    cudaMemsetAsync(loss, 0, sizeof(float) * nLoss, s);
+    cudaMemsetAsync(loss, 0, sizeof(double) * nLoss, s);
     mlp_grad_kernel<<<nLoss, kTrThreads, kTrSmemFloats * sizeof(float), s>>>(
         p, MlpRows{dx, dy, nullptr, nullptr, nullptr, 1.0f}, B, part, loss);
     mlp_adam_kernel<<<(kNParam + 63) / 64, 256, 0, s>>>(nLoss, part, gp, nullptr, nullptr, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f,
                                                         1.0f);
-    std::vector<float> lh(nLoss);
+    std::vector<double> lh(nLoss);
     cudaMemcpyAsync(grad, gp, sizeof(float) * kNParam, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(lh.data(), loss, sizeof(float) * nLoss, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(lh.data(), loss, sizeof(double) * nLoss, cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) return (int)cudaGetLastError();
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e;

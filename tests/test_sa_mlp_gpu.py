@@ -265,22 +265,45 @@ def numpy_loss_grad(params, x, y):
 
 
 def test_training_gradients_match_numpy_float64():
-    """The hand-written training kernels (strided GEMMs, SiLU and its
-    derivative, column sums) against a float64 NumPy backward pass: dW and db
-    of all four layers for a fixed seeded model and batch, 1e-4 relative
-    (norm-wise per array; the kernels run in FP32)."""
+    """The training kernel (forward and backward pass in tiles of 64 rows)
+    against a float64 NumPy backward pass: dW and db of all four layers for a
+    fixed seeded model and batch, 1e-4 relative (norm-wise per array; the kernel
+    runs in FP32)."""
     rng = np.random.default_rng(7)
     n_par = int(S.lib().phx_mlp_param_count())
     shapes = [("w1", H * 6), ("b1", H), ("w2", H * H), ("b2", H), ("w3", H * H), ("b3", H), ("w4", H), ("b4", 1)]
     assert sum(n for _, n in shapes) == n_par
     fan = {"w1": 6, "w2": H, "w3": H, "w4": H}
     params = np.concatenate([rng.standard_normal(n) / np.sqrt(fan.get(k, 10.0)) for k, n in shapes]).astype(np.float32)
-    B = 1000   # not a multiple of the 16-row tiles or the 256-thread blocks
+    B = 1000   # not a multiple of the 64-row tiles
     x = rng.standard_normal((B, 6)).astype(np.float32)
     y = rng.standard_normal(B).astype(np.float32)
     loss, grad = S.mlp_loss_grad(params, x, y)
     lref, gref = numpy_loss_grad(params, x, y)
     assert abs(loss - lref) <= 1e-5 * lref
+    off = 0
+    for k, n in shapes:
+        assert rel_err(grad[off:off + n], gref[k].ravel()) <= 1e-4, k
+        off += n
+
+
+@pytest.mark.parametrize("B", [1, 63, 64, 65, 20001])
+def test_training_gradients_of_any_batch(B):
+    """One row, the edges of a 64-row tile, and 313 tiles, which no count of
+    blocks up to one per SM (148) shares evenly: gradients are carried from tile
+    to tile.  A value passes at most 64 FP32 additions within a tile, one a tile
+    of its block, and 14 over the blocks, and the layers' products 64 each: 1e-4
+    of an array's norm is a hundred times their rounding, and the loss, summed
+    as trees and then in double, is good to 1e-5."""
+    rng = np.random.default_rng(11)
+    shapes = [("w1", H * 6), ("b1", H), ("w2", H * H), ("b2", H), ("w3", H * H), ("b3", H), ("w4", H), ("b4", 1)]
+    fan = {"w1": 6, "w2": H, "w3": H, "w4": H}
+    params = np.concatenate([rng.standard_normal(n) / np.sqrt(fan.get(k, 10.0)) for k, n in shapes]).astype(np.float32)
+    x = rng.standard_normal((B, 6)).astype(np.float32)
+    y = rng.standard_normal(B).astype(np.float32)
+    loss, grad = S.mlp_loss_grad(params, x, y)
+    lref, gref = numpy_loss_grad(params, x, y)
+    assert abs(loss - lref) <= 1e-5 * max(lref, 1.0)   # outputs and targets of order one
     off = 0
     for k, n in shapes:
         assert rel_err(grad[off:off + n], gref[k].ravel()) <= 1e-4, k
