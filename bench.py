@@ -24,8 +24,9 @@ instead (strong scaling).
 `--impl reference` times the reference's own solver, built from its sources
 with its OpenMP loops over zones (oracle/_ref/ref_harness_omp), on a bounded
 sample of the same workload split into one zone per host thread; without that
-build, one zone on one core (oracle/_ref/ref_harness), and without any build
-of the reference, the oracle's single-threaded C restatement of the path.
+build, one zone on one core (oracle/_ref/ref_harness).  Without any build of the
+reference it prints an `unavailable` line: the oracle's C restatement of the path,
+which then stands in as the CPU baseline of a GPU line, is not the reference.
 """
 from __future__ import annotations
 
@@ -818,6 +819,12 @@ def main():
 
     if args.impl == "reference":
         if rank != 0:
+            return
+        from oracle import refrun
+
+        if not refrun.available():
+            print(json.dumps({"impl": "reference", "unavailable": "the reference's solver is not built here "
+                              "(oracle/_ref), and its sources are not on this machine"}))
             return
         cb = cpu_baseline(args, args.workload)
         line = {"impl": "reference", "metric": METRIC, "value": cb["value"], "unit": "Mcell-iters/s",

@@ -4,6 +4,7 @@
   contract names (metric, value, unit, steps, warmup, ms_per_step,
   higher_is_better, config, cpu_baseline, e2e with zero copy bytes), its
   throughput agreeing with its own step time.
+* Without a build of the reference the arm prints its `unavailable` line.
 * Under a launcher (RANK > 0) the reference arm exits without work or output.
 * When the threaded reference run fails twice, the arm times one zone on one
   core instead of failing.
@@ -46,6 +47,21 @@ def test_reference_arm_prints_one_contract_line():
     assert d["e2e"]["h2d_bytes_per_step"] == 0 and d["e2e"]["d2h_bytes_per_step"] == 0
     # value (Mcell-iterations/s) and the step time describe the same run
     assert abs(cb["cells"] / (d["ms_per_step"] / 1e3) / 1e6 - d["value"]) <= 0.02 * d["value"]
+
+
+def test_reference_arm_without_the_reference_says_so(monkeypatch, capsys):
+    """The oracle is this repository's own code: it never stands in for the reference."""
+    sys.path.insert(0, ROOT)
+    import bench
+
+    monkeypatch.setattr(refrun, "available", lambda: False)
+    monkeypatch.delenv("RANK", raising=False)
+    monkeypatch.setattr(sys, "argv", ["bench.py", "--impl", "reference", "--workload", "euler_bump_8k"])
+    bench.main()
+    lines = [ln for ln in capsys.readouterr().out.splitlines() if ln.strip()]
+    assert len(lines) == 1
+    d = json.loads(lines[0])
+    assert set(d) == {"impl", "unavailable"} and d["impl"] == "reference" and d["unavailable"]
 
 
 def test_reference_arm_is_rank_zero_only():
