@@ -132,6 +132,7 @@ class ClockSampler:
         self.device = device
         self.proc = None
         self.lines = []
+        self.first = 0
 
     def start(self):
         try:
@@ -140,6 +141,12 @@ class ClockSampler:
                  "-lms", "200"], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self.thread = threading.Thread(target=self._read, daemon=True)
             self.thread.start()
+            # while nvidia-smi attaches to the driver, launches wait (up to 0.6 s of a 0.3 s timed region):
+            # the region begins after its first line, and its lines are those that count
+            t0 = time.time()
+            while not self.lines and self.proc.poll() is None and time.time() - t0 < 20.0:
+                time.sleep(0.01)
+            self.first = len(self.lines)
         except FileNotFoundError:
             self.proc = None
 
@@ -157,7 +164,7 @@ class ClockSampler:
             self.proc.kill()
         sm, smax, reasons = [], [], set()
         names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
-        for ln in self.lines:
+        for ln in self.lines[self.first:] or self.lines[-1:]:
             parts = [p.strip() for p in ln.split(",")]
             if len(parts) < 7:
                 continue
