@@ -33,7 +33,7 @@ extern "C" {
 #define PHX_OK 0
 #define PHX_ERR_ARG -1       /* invalid argument (null pointer, bad size, unsupported option) */
 #define PHX_ERR_CUDA -2      /* a CUDA runtime call failed */
-#define PHX_ERR_TIMEOUT -3   /* a bounded device-side wait gave up (level barrier) */
+#define PHX_ERR_TIMEOUT -3   /* a bounded device-side wait gave up */
 #define PHX_ERR_NUMERIC -4   /* NaN / divergence detected in a reduction */
 #define PHX_ERR_STATE -5     /* call out of order (e.g. no state uploaded) */
 
@@ -162,14 +162,16 @@ void phx_default_params(phx_params *p);
 /* Creates a context: uploads the grid, computes the FP64 metrics on the
  * device side of the context (face normals/areas/centres, cell centres and
  * volumes, skewness, wall distance), the cell-to-face lists and the LU-SGS
- * level schedules, and initialises the state to the free stream.
+ * schedules, and initialises the state to the free stream.
  * Replaces: Simulation::RunCFD grid set-up (Main/src/Simulation.cpp:205-260),
  * UnstructGrid::ComputeMetrics (API/Geometry/src/Geo_UnstructGrid.cpp:5695),
  * NSSolverUnstruct::AllocateGlobalVar / InitFlow, GPUGeomInfoAllocCopy.
  * A context that would leave less than two thirds of the device's memory free
  * keeps neither face geometry nor the sweeps' factors, and forms them where
  * they are used: the same results, a smaller context, a slower step
- * (PHX_LAYOUT=full or compact in the environment takes the one or the other). */
+ * (PHX_LAYOUT=full or compact in the environment takes the one or the other).
+ * PHX_LUSGS_MAX_BLOCKS in the environment caps the sweeps' warps, a block of 32
+ * threads each, for the context being created (tuning and tests). */
 int phx_ctx_create(const phx_grid_desc *grid, const phx_params *params, phx_ctx **out);
 int phx_ctx_destroy(phx_ctx *ctx);
 const char *phx_last_error(const phx_ctx *ctx);
@@ -313,7 +315,8 @@ int phx_set_wait_limit(phx_ctx *ctx, int64_t polls);
 /* Failure-detection hook for tests: the forward LU-SGS result of reference
  * cell `cell` never comes (-1: off), so the wait on it runs out and the step
  * returns PHX_ERR_TIMEOUT instead of hanging.  Nothing faults: the sweep
- * stops at its next level boundary.  No counterpart in the reference. */
+ * stops where its warps next look at the status.  No counterpart in the
+ * reference. */
 int phx_fault_hold_cell(phx_ctx *ctx, int32_t cell);
 
 /* --- partitioned grids (zones joined by PHX_BC_INTERFACE faces) ------------

@@ -27,19 +27,6 @@ __device__ __forceinline__ void ld4(const float *p, float *o)
 }
 template <class T>
 __device__ __forceinline__ void ld8(const T *p, T *o) { ld4(p, o); ld4(p + 4, o + 4); }
-__device__ __forceinline__ void ld4cg(const double *p, double *o)
-{
-    const double2 a = __ldcg(reinterpret_cast<const double2 *>(p));
-    const double2 b = __ldcg(reinterpret_cast<const double2 *>(p) + 1);
-    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
-}
-__device__ __forceinline__ void ld4cg(const float *p, float *o)
-{
-    const float4 a = __ldcg(reinterpret_cast<const float4 *>(p));
-    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
-}
-template <class T>
-__device__ __forceinline__ void ld8cg(const T *p, T *o) { ld4cg(p, o); ld4cg(p + 4, o + 4); }
 __device__ __forceinline__ void st4(double *p, const double *v)
 {
     reinterpret_cast<double2 *>(p)[0] = make_double2(v[0], v[1]);
@@ -245,8 +232,9 @@ __device__ __forceinline__ void get8(const T *p, T *o) { get4(p, o); get4(p + 4,
 
 // Write-once sweep records.  Before a sweep every element of its output
 // records holds the sentinel, a NaN whose sign and payload no arithmetic
-// result carries (the GPU's NaN results are the positive canonical NaN, and
-// producers map the sentinel pattern itself to that NaN).  During the sweep
+// result carries: single-precision arithmetic gives no NaN but the positive
+// canonical one, and in double precision, which may hand a NaN operand on,
+// producers map the sentinel pattern to another NaN.  During the sweep
 // each element is stored once, so a reader that sees anything but the
 // sentinel sees the final value: the data is its own completion flag, and
 // neither a fence between the producer's stores nor a second load after the
@@ -266,8 +254,7 @@ __device__ __forceinline__ bool is_sentinel(double v)
 {
     return (unsigned long long)__double_as_longlong(v) == kSentinelD;
 }
-// a computed value as stored: the sentinel pattern becomes the canonical NaN
-// (single-precision arithmetic gives no other NaN)
+// a computed value as stored
 __device__ __forceinline__ float unsentinel(float v) { return v; }
 __device__ __forceinline__ double unsentinel(double v)
 {

@@ -8,7 +8,7 @@
 // per-cell and per-face data are array-of-structs records read with vector
 // loads.  The reference's numbering is kept wherever it decides an order:
 // every cell's face list is sorted by the reference face number (the order
-// LoadFlux and the Green-Gauss loop accumulate in), and the LU-SGS level
+// LoadFlux and the Green-Gauss loop accumulate in), and the LU-SGS
 // schedules come from the reference cell numbers.
 #pragma once
 #include <cuda_runtime.h>
@@ -90,7 +90,6 @@ constexpr int kRowCompact = 32 * 8 + kSweepSlots * 4 + kSweepRow * 4;
 template <class T>
 constexpr int kRowSa = (32 + kSweepSlots * kLeadT) * (int)sizeof(T) + kSweepRow * 4;
 constexpr long long kDefaultSpinLimit = 20000000LL;   // polls per dependency wait (~1-2 s)
-constexpr int kMaxDevices = 64;                       // per-device launch caches
 // Spalart-Allmaras records
 constexpr int kTr = 4;     // trec: nu~ | eddy viscosity | laminar viscosity of the NS step | pad
 constexpr int kTg = 4;     // tgrad: d nu~ / dx, dy, dz | pad

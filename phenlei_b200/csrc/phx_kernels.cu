@@ -2,9 +2,10 @@
 // phx_internal.h).
 //
 // Per-cell sums are owner-computes gathers over the cell's faces in the
-// reference's face order, so no atomics touch the state and the FP64 path
-// keeps the reference's accumulation order.  Face metrics stay FP64; the
-// working state T is double (FP64 path) or float (mixed path).
+// reference's face order, so no atomics touch the state (the SA cell pass sums
+// convection and diffusion side by side).  Metrics are formed and kept in FP64;
+// the passes read face geometry derived from them in the working precision T,
+// double (FP64 path) or float (mixed path).
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdlib.h>
@@ -539,9 +540,9 @@ __device__ __forceinline__ void reset_reduce(Reduce *r)
 // spectral-radius term, which is also the LU-SGS viscous factor of both face uses
 // (SpectrumRadiusViscous method 2, NSSolverUnstruct.cpp:5930-5960;
 // SolveLUSGSForward :15339-15357): GetVisFaceValue (:7126-7375, static adiabatic
-// walls) and ComputeVisflux (:12977-13378, perfect gas).  The face gradient F of u, v, w has its normal part
-// replaced by the normal derivative; what ComputeVisflux takes along two tangents
-// is F less its normal part.
+// walls) and ComputeVisflux (:12977-13378, perfect gas).  The face gradient F of u,
+// v, w has its normal part replaced by the normal derivative; what ComputeVisflux
+// takes along two tangents is F less its normal part.
 //
 // The pass is bound by memory latency: three blocks per SM, of 256 threads on the
 // mixed path and of 128 in double precision (at most 168 registers), and one side

@@ -60,7 +60,6 @@ SweepRows build_sweep(const SweepGraph &g, bool forward, int maxWarps)
         lev[c] = l;
         nlev = std::max(nlev, l + 1);
     }
-    out.nLevels = nlev;
     std::vector<int> loff(nlev + 1, 0), cells(nc);
     for (int c = 0; c < nc; ++c) loff[lev[c] + 1]++;
     for (int l = 0; l < nlev; ++l) loff[l + 1] += loff[l];

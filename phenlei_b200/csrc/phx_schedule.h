@@ -23,7 +23,7 @@ struct SweepGraph {
 // that holds the neighbour's result (-1: its record in memory is polled).  The
 // row's own results go to shared-memory slots store[r] * kSweepSlots + s.
 struct SweepRows {
-    int nWarps = 0, nLevels = 0;
+    int nWarps = 0;
     std::vector<int> rowOff, store;
     std::vector<int> cell, flags, ent, loc;
 };

@@ -154,9 +154,9 @@ def test_positivity_repair_matches_oracle():
 
 @pytest.mark.parametrize("blocks", ["1", "2"])
 def test_levels_wider_than_grid(monkeypatch, blocks):
-    """Sweep levels wider than the cooperative grid (several rounds per level)."""
+    """Sweep levels wider than the cooperative grid (several rows a level on a warp)."""
     monkeypatch.setenv("PHX_LUSGS_MAX_BLOCKS", blocks)
-    m = M.channel_bump(64, 32, 8)      # widest level > 64 groups of one 512-thread block
+    m = M.channel_bump(64, 32, 8)      # the widest level has far more cells than a warp's eight
     params = cases.EULER_BUMP
     o, q0 = _oracle_case(m, params, seed=6)
     o.iterate(2)
