@@ -141,8 +141,8 @@ class ClockSampler:
                  "-lms", "200"], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self.thread = threading.Thread(target=self._read, daemon=True)
             self.thread.start()
-            # while nvidia-smi attaches to the driver, launches wait (up to 0.6 s of a 0.3 s timed region):
-            # the region begins after its first line, and its lines are those that count
+            # the timed region begins after the first line, so that nvidia-smi does not attach to the driver
+            # in it, and the lines that count are its own
             t0 = time.time()
             while not self.lines and self.proc.poll() is None and time.time() - t0 < 20.0:
                 time.sleep(0.01)

